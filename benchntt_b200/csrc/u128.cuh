@@ -14,9 +14,9 @@
 //     reference's Barrett quotient is within one of the true quotient, so its
 //     single conditional subtraction always lands in [0, q): the reference
 //     returns exactly a*b mod q.  ArithFast computes that value with a
-//     pseudo-Mersenne fold (2^128 == 16k, 2^124 == k mod q): four 64-bit
-//     products for a*b, 4 limb products for the first fold, 1 for the second,
-//     one conditional subtraction.  Its operands must be below 2^124.
+//     pseudo-Mersenne fold (2^128 == 16k, 2^124 == k mod q): 16 limb products
+//     for a*b, 4 for the first fold, 1 for the second, one conditional
+//     subtraction.  Its first operand must be below 2^124.
 //   ArithRef  -- every other (q, mu): a replica of the reference's 64-bit word
 //     data flow, including the points where it drops carries, so it matches
 //     for arbitrary 128-bit inputs.
@@ -171,74 +171,145 @@ __device__ __forceinline__ U128 submod_pm(const U128& a, const U128& b, uint32_t
 
 // ------------------------------------------------------------------ ArithFast
 
-// p = a * b for a, b < 2^124 (every residue of an ArithFast modulus), as
-// four 64 x 64 -> 128-bit products of the 64-bit halves: the middle sum
-// a0*b1 + a1*b0 stays below 2^125 because the high halves are below 2^60.
-// Written on 64-bit halves so that the compiler picks the instructions for
-// the 32-bit partial products and their carries: the register-only butterfly
-// probe runs at 233 G butterflies/s this way, against 209 G/s with a
-// hand-written PTX carry chain per row of 32-bit limbs (mad.lo.cc/madc.hi.cc)
-// and 212 G/s when the middle sum's carry is kept for full 128-bit operands.
-__device__ __forceinline__ void mul_128x128(const U128& a, const U128& b, uint32_t p[8]) {
-  typedef unsigned __int128 u128x;
-  typedef unsigned long long u64x;
-  const u64x a0 = ((u64x)a.w[1] << 32) | a.w[0], a1 = ((u64x)a.w[3] << 32) | a.w[2];
-  const u64x b0 = ((u64x)b.w[1] << 32) | b.w[0], b1 = ((u64x)b.w[3] << 32) | b.w[2];
-  const u128x p00 = (u128x)a0 * b0, p11 = (u128x)a1 * b1;
-  const u128x mid = (u128x)a0 * b1 + (u128x)a1 * b0;
-  const u128x lo = p00 + (mid << 64);
-  const u128x hi = p11 + (mid >> 64) + (lo < p00 ? 1u : 0u);
-  p[0] = (uint32_t)lo;
-  p[1] = (uint32_t)(lo >> 32);
-  p[2] = (uint32_t)(lo >> 64);
-  p[3] = (uint32_t)(lo >> 96);
-  p[4] = (uint32_t)hi;
-  p[5] = (uint32_t)(hi >> 32);
-  p[6] = (uint32_t)(hi >> 64);
-  p[7] = (uint32_t)(hi >> 96);
-}
-
-// r = P mod q for q = 2^124 - k, P < 2^248, k < 2^28, folding first at the
-// limb boundary 2^128 (2^128 = 16 * 2^124 == 16k mod q), which needs no
-// shifts of P:
-//   P = H*2^128 + L      ->  t = L + H*16k          (< 2^128 + 2^152: 5 limbs)
-//   t = h*2^124 + l      ->  r = l + h*k            (h < 2^29; r < 2^124 + 2^57 < 2q)
-//   r >= q ? r - q : r, tested as bit 124 of r + k; r >= q needs r's top
-//   limb at least 0x0FFFFFFF, about one case in 2^28 for spread residues, so
-//   the exact test and the subtraction sit behind a branch.
-// Folding at 2^124 twice instead costs six more ALU instructions (funnel
-// shifts of P, the second fold's product added outside the multiply-add
-// chain): 204 against 209 G butterflies/s in the register-only probe.  Both reference
-// moduli and every prime bntt_ntt_prime returns have k < 2^28.
-__device__ __forceinline__ U128 reduce_pm124(const uint32_t p[8], uint32_t k) {
+// a * b mod q up to a multiple of q, for q = 2^124 - k, k < 2^28: the result r
+// is congruent to a * b and 0 <= r < 2^124 + 2^60.  a < 2^124; b is any value
+// below 2^128 - 2^101 (a partly reduced one included).
+//
+// The product's 16 partial products are summed in two columns of 64-bit
+// accumulators, E at the even limbs and O at the odd ones, so that every
+// partial product is one 32 x 32 + 64-bit multiply-add whose carry runs into
+// the next one of its column (each mad.lo.cc / madc.hi.cc pair on one pair of
+// limbs).  P = E + O*2^32 is never put together: the upper parts are added,
+// H = E / 2^128 + O / 2^96, and the two lower parts take the first fold
+// separately, 2^128 = 16 * 2^124 == 16k (mod q):
+//   t = E mod 2^128 + (O mod 2^96)*2^32 + H*16k      (< 2^156: 5 limbs)
+//   r = t mod 2^124 + (t >> 124)*k
+// What bounds it: the multiply-add pipe, on which a 32 x 32 + 64-bit
+// multiply-add takes 4 cycles per warp and scheduler and other integer
+// instructions there 2 (measured: 31 wide products per clock and SM against
+// 64 mad.lo).  This form has 21 wide multiply-adds (16 + 4 + 1) and about 20
+// other instructions; the product on 64-bit halves in C++ with the folds as
+// separate lo and hi rows had 22 and about 50.  In the register-only
+// butterfly probe with the exact add and sub: 233 -> 287 G butterflies/s.
+// Carries out of a column (c5, c6, c7) are added to H at the end; as
+// zero-extended accumulators of the next row they cost moves on the same pipe
+// (349 against 354 G/s in the probe without exact add and sub).
+__device__ __forceinline__ U128 mul_lazy(const U128& a, const U128& b, uint32_t k) {
+  uint32_t e0, e1, e2, e3, e4, e5, e6, e7, o1, o2, o3, o4, o5, o6, c5, c6, c7;
+  // limb 0 of a: E at 0 and 2, O at 1 and 3
+  asm("mul.lo.u32 %0, %4, %5;\n\t"
+      "mul.hi.u32 %1, %4, %5;\n\t"
+      "mul.lo.u32 %2, %4, %6;\n\t"
+      "mul.hi.u32 %3, %4, %6;\n\t"
+      : "=&r"(e0), "=&r"(e1), "=&r"(e2), "=&r"(e3)
+      : "r"(a.w[0]), "r"(b.w[0]), "r"(b.w[2]));
+  asm("mul.lo.u32 %0, %4, %5;\n\t"
+      "mul.hi.u32 %1, %4, %5;\n\t"
+      "mul.lo.u32 %2, %4, %6;\n\t"
+      "mul.hi.u32 %3, %4, %6;\n\t"
+      : "=&r"(o1), "=&r"(o2), "=&r"(o3), "=&r"(o4)
+      : "r"(a.w[0]), "r"(b.w[1]), "r"(b.w[3]));
+  // limb 1: O at 1 and 3, E at 2 and 4
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;\n\t"
+      : "+r"(o1), "+r"(o2), "+r"(o3), "+r"(o4), "=r"(c5)
+      : "r"(a.w[1]), "r"(b.w[0]), "r"(b.w[2]));
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, 0;\n\t"
+      "madc.hi.u32    %3, %4, %6, 0;\n\t"
+      : "+r"(e2), "+r"(e3), "=&r"(e4), "=&r"(e5)
+      : "r"(a.w[1]), "r"(b.w[1]), "r"(b.w[3]));
+  // limb 2: E at 2 and 4, O at 3 and 5
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;\n\t"
+      : "+r"(e2), "+r"(e3), "+r"(e4), "+r"(e5), "=r"(c6)
+      : "r"(a.w[2]), "r"(b.w[0]), "r"(b.w[2]));
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, 0;\n\t"
+      "madc.hi.u32    %3, %4, %6, 0;\n\t"
+      : "+r"(o3), "+r"(o4), "=&r"(o5), "=&r"(o6)
+      : "r"(a.w[2]), "r"(b.w[1]), "r"(b.w[3]));
+  // limb 3: O at 3 and 5, E at 4 and 6
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;\n\t"
+      : "+r"(o3), "+r"(o4), "+r"(o5), "+r"(o6), "=r"(c7)
+      : "r"(a.w[3]), "r"(b.w[0]), "r"(b.w[2]));
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, 0;\n\t"
+      "madc.hi.u32    %3, %4, %6, 0;\n\t"
+      : "+r"(e4), "+r"(e5), "=&r"(e6), "=&r"(e7)
+      : "r"(a.w[3]), "r"(b.w[1]), "r"(b.w[3]));
+  // H = upper parts and the carries at limbs 5, 6 and 7 (H <= P / 2^128)
+  uint32_t h0, h1, h2, h3;
+  asm("add.cc.u32  %0, %4, %8;\n\t"
+      "addc.cc.u32 %1, %5, %9;\n\t"
+      "addc.cc.u32 %2, %6, %10;\n\t"
+      "addc.u32    %3, %7, %11;\n\t"
+      : "=&r"(h0), "=&r"(h1), "=&r"(h2), "=&r"(h3)
+      : "r"(e4), "r"(e5), "r"(e6), "r"(e7), "r"(o4), "r"(o5), "r"(o6), "r"(c7));
+  asm("add.cc.u32  %0, %0, %3;\n\t"
+      "addc.cc.u32 %1, %1, %4;\n\t"
+      "addc.u32    %2, %2, 0;\n\t"
+      : "+r"(h1), "+r"(h2), "+r"(h3)
+      : "r"(c5), "r"(c6));
+  // first fold, by column, then the columns together
   const uint32_t c = k << 4;
-  uint32_t t0, t1, t2, t3, t4;
-  asm("mad.lo.cc.u32  %0, %5, %9, %10;\n\t"
-      "madc.lo.cc.u32 %1, %6, %9, %11;\n\t"
-      "madc.lo.cc.u32 %2, %7, %9, %12;\n\t"
-      "madc.lo.cc.u32 %3, %8, %9, %13;\n\t"
-      "madc.hi.u32    %4, %8, %9, 0;\n\t"
-      "mad.hi.cc.u32  %1, %5, %9, %1;\n\t"
-      "madc.hi.cc.u32 %2, %6, %9, %2;\n\t"
-      "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
-      "addc.u32       %4, %4, 0;\n\t"
-      : "=&r"(t0), "=&r"(t1), "=&r"(t2), "=&r"(t3), "=&r"(t4)
-      : "r"(p[4]), "r"(p[5]), "r"(p[6]), "r"(p[7]), "r"(c), "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]));
+  uint32_t t1, t2, t3, t4, u4;
+  asm("mad.lo.cc.u32  %0, %5, %7, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+      "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;\n\t"
+      : "+r"(e0), "+r"(e1), "+r"(e2), "+r"(e3), "=r"(t4)
+      : "r"(h0), "r"(h2), "r"(c));
+  asm("mad.lo.cc.u32  %0, %4, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %6, %2;\n\t"
+      "madc.hi.u32    %3, %5, %6, 0;\n\t"
+      : "+r"(o1), "+r"(o2), "+r"(o3), "=&r"(u4)
+      : "r"(h1), "r"(h3), "r"(c));
+  asm("add.cc.u32  %0, %4, %7;\n\t"
+      "addc.cc.u32 %1, %5, %8;\n\t"
+      "addc.cc.u32 %2, %6, %9;\n\t"
+      "addc.u32    %3, %10, %11;\n\t"
+      : "=&r"(t1), "=&r"(t2), "=&r"(t3), "=&r"(t4)
+      : "r"(e1), "r"(e2), "r"(e3), "r"(o1), "r"(o2), "r"(o3), "r"(t4), "r"(u4));
+  // second fold
   const uint32_t h = __funnelshift_r(t3, t4, 28);  // t >> 124
   U128 r;
   asm("mad.lo.cc.u32  %0, %4, %5, %6;\n\t"
       "madc.hi.cc.u32 %1, %4, %5, %7;\n\t"
       "addc.cc.u32    %2, %8, 0;\n\t"
       "addc.u32       %3, %9, 0;\n\t"
-      : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3])
-      : "r"(h), "r"(k), "r"(t0), "r"(t1), "r"(t2), "r"(t3 & 0x0FFFFFFFu));
+      : "=&r"(r.w[0]), "=&r"(r.w[1]), "=&r"(r.w[2]), "=&r"(r.w[3])
+      : "r"(h), "r"(k), "r"(e0), "r"(t1), "r"(t2), "r"(t3 & 0x0FFFFFFFu));
+  return r;
+}
+
+// r < 2^124 + 2^60 -> [0, q): r less q when r >= q, tested as bit 124 of
+// r + k.  r >= q needs r's top limb at least 0x0FFFFFFF, about one case in
+// 2^28 for spread residues, so the exact test and the subtraction sit behind
+// a branch.
+__device__ __forceinline__ U128 reduce_once(U128 r, uint32_t k) {
   if (__builtin_expect(r.w[3] >= 0x0FFFFFFFu, 0)) {  // r >= q is possible only here
     uint32_t s0, s1, s2, s3;
     asm("add.cc.u32  %0, %4, %8;\n\t"
         "addc.cc.u32 %1, %5, 0;\n\t"
         "addc.cc.u32 %2, %6, 0;\n\t"
         "addc.u32    %3, %7, 0;\n\t"
-        : "=r"(s0), "=r"(s1), "=r"(s2), "=r"(s3)
+        : "=&r"(s0), "=&r"(s1), "=&r"(s2), "=&r"(s3)
         : "r"(r.w[0]), "r"(r.w[1]), "r"(r.w[2]), "r"(r.w[3]), "r"(k));
     if (s3 >> 28) {  // r + k >= 2^124, i.e. r >= q
       r.w[0] = s0; r.w[1] = s1; r.w[2] = s2; r.w[3] = s3 & 0x0FFFFFFFu;
@@ -250,9 +321,7 @@ __device__ __forceinline__ U128 reduce_pm124(const uint32_t p[8], uint32_t k) {
 struct ArithFast {
   static constexpr bool kFast = true;
   __device__ __forceinline__ static U128 mul(const U128& a, const U128& b, const ModParams& m) {
-    uint32_t p[8];
-    mul_128x128(a, b, p);
-    return reduce_pm124(p, m.k);
+    return reduce_once(mul_lazy(a, b, m.k), m.k);
   }
 };
 
