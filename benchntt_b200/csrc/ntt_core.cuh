@@ -177,10 +177,133 @@ struct NttTile {
                                              const ModParams& mp, int layout,
                                              const MulB& mb = MulB{}) {
     U128 v[R];
-    pass<0, LDP, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
+    if constexpr (Arith::kFast) pass_lazy<0, LDP, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
+    else pass<0, LDP>(v, sr, sub, lane, smem, mp, layout, mb);
   }
 
-  template <int P, int LDP, int SRC = SRC_GLOBAL>
+  // Stages run on partly reduced values (u128.cuh) before pass p since they
+  // were last brought back to 8q + [0, 2^124 + 2^32): by the first pass's
+  // gather, or where one more pass would exceed kLazyStages.
+  __host__ __device__ static constexpr int lazy_before(int p) {
+    int a = 0;
+    for (int i = 0; i < p; ++i) a = (a + bits(i) > kLazyStages ? 0 : a) + bits(i);
+    return a;
+  }
+  __host__ __device__ static constexpr bool rebase(int p) { return lazy_before(p) + bits(p) > kLazyStages; }
+
+  // One pass on partly reduced values (fast moduli).  Only the elements that
+  // the first stage adds to need a base of 8q; the ones it multiplies are
+  // taken as they are.
+  template <int P, int LDP, int SRC>
+  __device__ __forceinline__ static void pass_lazy(U128 (&v)[R], const SubRef& sr, int sub, int lane,
+                                                   uint4* smem, const ModParams& mp, int layout,
+                                                   const MulB& mb) {
+    constexpr int r = bits(P);
+    constexpr int s0 = start(P);
+    constexpr int lo = M - s0 - r;        // lowest local bit this pass touches
+    constexpr int G = 1 << r;             // elements per group
+    constexpr int GPT = R / G;            // groups per thread
+    constexpr bool last = P == NPASS - 1;
+    static_assert(GPT >= 1, "pass wider than the register tile");
+    static_assert(r <= kLazyStages, "pass wider than the partly reduced range");
+    // element j of a group in HBM: the group's first element plus j * gstep
+    const size_t gstep = (size_t)1 << (lo + sr.lshift);
+    const uint32_t k = mp.k;
+
+    // element j of the group at local index base, slot sb
+    auto gather = [&](int base, int sb, int j) -> U128 {
+      if constexpr (P == 0 && (SRC & SRC_STAGED) != 0) {
+        return from_mem(smem[slot_at(sb, j << lo)], layout);  // staged in memory order
+      } else if constexpr (P == 0) {
+        if (!sr.valid) return U128{{0u, 0u, 0u, 0u}};
+        return from_mem(ld_data<LDP>(sr.x + ((size_t)base << sr.lshift) + (size_t)j * gstep), layout);
+      } else {
+        const uint4 t = smem[slot_at(sb, j << lo)];
+        return U128{{t.x, t.y, t.z, t.w}};
+      }
+    };
+    auto base_of = [&](int i) {
+      const int g = lane + i * TPT;
+      return (g & ((1 << lo) - 1)) | ((g >> lo) << (lo + r));
+    };
+    auto gt_of = [&](int i) { return (sr.trow << s0) + (uint32_t)((lane + i * TPT) >> lo); };
+
+#pragma unroll
+    for (int i = 0; i < GPT; ++i) {
+      const int base = base_of(i), sb = slot(sub, base);
+#pragma unroll
+      for (int j = 0; j < G; ++j) v[i * G + j] = gather(base, sb, j);
+    }
+    bool rerun = false;
+#pragma unroll
+    for (int i = 0; i < GPT; ++i) {
+#pragma unroll
+      for (int j = 0; j < G / 2; ++j) {
+        U128& x = v[i * G + j];
+        if constexpr (P == 0) x = add_8q(x, k);
+        else if constexpr (rebase(P)) x = add_8q(fold_top(x, k), k);
+      }
+      const uint32_t gt = gt_of(i);
+      lazy_stages<r>(v, i * G, [&](int t, int u) {
+        // tables are stored in limb order (LAYOUT_U128) by the plan
+        const uint4* twt = sr.tw + (gt << t);  // u as an immediate offset
+        const uint4 tv = (SRC & TW_SHARED) != 0 ? lds128(twt + u) : __ldg(twt + u);
+        return U128{{tv.x, tv.y, tv.z, tv.w}};
+      }, k, rerun);
+    }
+    // the transform's outputs: below q unless the top limb says otherwise
+    if constexpr (last) {
+      if (!mb.b) {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          v[j] = fold_top(v[j], k);
+          rerun |= v[j].w[3] >= 0x0FFFFFFFu;
+        }
+      }
+    }
+    if (__builtin_expect(rerun && sr.valid, 0)) {
+      // the pass's inputs are still where they were gathered from
+#pragma unroll
+      for (int i = 0; i < GPT; ++i) {
+        const int base = base_of(i), sb = slot(sub, base);
+        U128 t[G];
+#pragma unroll
+        for (int j = 0; j < G; ++j) t[j] = gather(base, sb, j);
+        exact_stages<r>(t, sr.tw, gt_of(i), mp, P > 0);
+#pragma unroll
+        for (int j = 0; j < G; ++j) v[i * G + j] = last ? t[j] : add_8q(t[j], k);
+      }
+    }
+
+#pragma unroll
+    for (int i = 0; i < GPT; ++i) {
+      const int base = base_of(i), sb = slot(sub, base);
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        if constexpr (last) {
+          if (sr.valid) {
+            uint4* yp = sr.y + ((size_t)base << sr.lshift) + (size_t)j * gstep;
+            U128 o = v[i * G + j];
+            if (mb.b) {
+              const uint4 bv = __ldg(mb.b + ((uint64_t)(yp - mb.ybase) & mb.bmask));
+              o = reduce_once(mul_lazy(from_mem(bv, layout), o, k), k);
+            }
+            *yp = to_mem(o, layout);
+          }
+        } else {
+          const U128& e = v[i * G + j];
+          smem[slot_at(sb, j << lo)] = make_uint4(e.w[0], e.w[1], e.w[2], e.w[3]);
+        }
+      }
+    }
+    if constexpr (P + 1 < NPASS) {
+      sync_between<P, P + 1>();
+      pass_lazy<P + 1, LDP, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
+    }
+  }
+
+  // One pass in the replica arithmetic (ArithRef).
+  template <int P, int LDP>
   __device__ __forceinline__ static void pass(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                               uint4* smem, const ModParams& mp, int layout,
                                               const MulB& mb) {
@@ -201,9 +324,7 @@ struct NttTile {
       const int sb = slot(sub, base);
 #pragma unroll
       for (int j = 0; j < G; ++j) {
-        if constexpr (P == 0 && (SRC & SRC_STAGED) != 0) {
-          v[i * G + j] = from_mem(smem[slot_at(sb, j << lo)], layout);  // staged in memory order
-        } else if constexpr (P == 0) {
+        if constexpr (P == 0) {
           if (sr.valid) {
             v[i * G + j] = from_mem(ld_data<LDP>(sr.x + ((size_t)base << sr.lshift) + (size_t)j * gstep), layout);
           } else {
@@ -229,7 +350,7 @@ struct NttTile {
         for (int u = 0; u < (1 << t); ++u) {
           // tables are stored in limb order (LAYOUT_U128) by the plan
           const uint4* twt = sr.tw + (gt << t);  // u as an immediate offset
-          const uint4 tv = (SRC & TW_SHARED) != 0 ? lds128(twt + u) : __ldg(twt + u);
+          const uint4 tv = __ldg(twt + u);
           const U128 w = U128{{tv.x, tv.y, tv.z, tv.w}};
 #pragma unroll
           for (int k = 0; k < half; ++k) {
@@ -266,7 +387,7 @@ struct NttTile {
     }
     if constexpr (P + 1 < NPASS) {
       sync_between<P, P + 1>();
-      pass<P + 1, LDP, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
+      pass<P + 1, LDP>(v, sr, sub, lane, smem, mp, layout, mb);
     }
   }
 

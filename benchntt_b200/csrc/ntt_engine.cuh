@@ -100,10 +100,11 @@ struct NttEngine {
   // scalar at ep->scale_at, bit EPI_MUL its pointwise product.
   template <int r, int LDP, bool INV = false, int EPI = 0>
   __device__ __forceinline__ static void pass(U128 (&v)[R], const SubRef& sr, int s0, int lo,
-                                              int lane, int tpt, bool first, bool last,
+                                              int lane, int tpt, bool first, bool last, bool rebase,
                                               const Layout& lay, uint4* smem, const ModParams& mp,
                                               int layout, const Epilogue* ep = nullptr) {
     constexpr int G = 1 << r, GPT = R / G;
+    constexpr bool lazy = Arith::kFast && !INV;  // partly reduced values (u128.cuh)
     const int hi_mask = ~((1 << lo) - 1);
     const int step = lay.lmul << lo;  // linear-index distance of j and j + 1
     // Slot of element j of a group: pad(lb + j*step).  With 4 elements per
@@ -127,18 +128,17 @@ struct NttEngine {
       const int g = lane + i * tpt;
       return g + (g & hi_mask) * (G - 1);
     };
-    // gather
-#pragma unroll
-    for (int i = 0; i < GPT; ++i) {
+    // gather group i into e[0..G)
+    auto gather = [&](U128* e, int i) {
       if (first) {
         const uint4* gp = sr.x + ((size_t)base(i) << sr.lshift);
 #pragma unroll
         for (int j = 0; j < G; ++j) {
           if (sr.valid) {
-            v[i * G + j] = from_mem(ld_data<LDP>(gp + (size_t)(j * gstep)), layout);
+            e[j] = from_mem(ld_data<LDP>(gp + (size_t)(j * gstep)), layout);
           } else {
 #pragma unroll
-            for (int w = 0; w < 4; ++w) v[i * G + j].w[w] = 0u;
+            for (int w = 0; w < 4; ++w) e[j].w[w] = 0u;
           }
         }
       } else {
@@ -146,8 +146,22 @@ struct NttEngine {
 #pragma unroll
         for (int j = 0; j < G; ++j) {
           const uint4 t = smem[slot_of(lb, j)];
-          v[i * G + j] = U128{{t.x, t.y, t.z, t.w}};
+          e[j] = U128{{t.x, t.y, t.z, t.w}};
         }
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < GPT; ++i) gather(&v[i * G], i);
+    bool rerun = false;
+    if constexpr (lazy) {  // the first stage adds to the lower half of each group
+      if (first || rebase) {
+#pragma unroll
+        for (int i = 0; i < GPT; ++i)
+#pragma unroll
+          for (int j = 0; j < G / 2; ++j) {
+            if (rebase) v[i * G + j] = fold_top(v[i * G + j], mp.k);
+            v[i * G + j] = add_8q(v[i * G + j], mp.k);
+          }
       }
     }
     // r stages per group; stage t of the group reads T[(gt << t) + u],
@@ -158,7 +172,12 @@ struct NttEngine {
     for (int i = 0; i < GPT; ++i) {
       const int g = lane + i * tpt;
       const uint32_t gt = (sr.trow << s0) + (uint32_t)(g >> lo);
-      if constexpr (INV && r > 2) {
+      if constexpr (lazy) {
+        lazy_stages<r>(v, i * G, [&](int t, int u) {
+          const uint4 tv = __ldg(sr.tw + (gt << t) + u);
+          return U128{{tv.x, tv.y, tv.z, tv.w}};
+        }, mp.k, rerun);
+      } else if constexpr (INV && r > 2) {
         if constexpr (r > 3) stage<r, 3, true>(v, i * G, gt, sr.tw, mp);
         stage<r, 2, true>(v, i * G, gt, sr.tw, mp);
         stage<r, 1, true>(v, i * G, gt, sr.tw, mp);
@@ -179,6 +198,25 @@ struct NttEngine {
               else butterfly<Arith>(v[i * G + j], v[i * G + j + half], w, mp);
             }
           }
+        }
+      }
+    }
+    if constexpr (lazy) {  // as NttTile::pass_lazy
+      if (last) {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          v[j] = fold_top(v[j], mp.k);
+          rerun |= v[j].w[3] >= 0x0FFFFFFFu;
+        }
+      }
+      if (__builtin_expect(rerun && sr.valid, 0)) {
+#pragma unroll
+        for (int i = 0; i < GPT; ++i) {
+          U128 e[G];
+          gather(e, i);
+          exact_stages<r>(e, sr.tw, (sr.trow << s0) + (uint32_t)((lane + i * tpt) >> lo), mp, !first);
+#pragma unroll
+          for (int j = 0; j < G; ++j) v[i * G + j] = last ? e[j] : add_8q(e[j], mp.k);
         }
       }
     }
@@ -251,24 +289,27 @@ struct NttEngine {
     lay.lbase = contig ? sub << M : sub;
     lay.lmul = contig ? 1 : threads >> (M - LOGR);
     U128 v[R];
+    int run_stages = 0;  // stages since the values were last brought back to 8q + [0, 2^124 + 2^32)
     for (int pp = 0; pp < ps.n; ++pp) {
       const int p = INV ? ps.n - 1 - pp : pp;
       const int r = ps.bits(p), s0 = ps.start(p), lo = M - s0 - r;
       const bool first = pp == 0, last = pp == ps.n - 1;
+      const bool rebase = run_stages + r > kLazyStages;
+      run_stages = (rebase ? 0 : run_stages) + r;
       if constexpr (LOGR >= 4) {
         if (r == 4)
-          pass<(LOGR >= 4 ? 4 : 1), LDP, INV, EPI>(v, sr, s0, lo, lane, tpt, first, last, lay, smem, mp,
-                                              layout, ep);
+          pass<(LOGR >= 4 ? 4 : 1), LDP, INV, EPI>(v, sr, s0, lo, lane, tpt, first, last, rebase, lay, smem,
+                                                   mp, layout, ep);
       }
       // with LOGR = 3 the balanced passes of 2^3..2^10 points have 2 or 3
       // stages, so width 1 needs no code there
       if (LOGR >= 3 && r == 3)
-        pass<(LOGR >= 3 ? 3 : 1), LDP, INV, EPI>(v, sr, s0, lo, lane, tpt, first, last, lay, smem, mp,
-                                                 layout, ep);
+        pass<(LOGR >= 3 ? 3 : 1), LDP, INV, EPI>(v, sr, s0, lo, lane, tpt, first, last, rebase, lay, smem,
+                                                 mp, layout, ep);
       else if (r == 2)
-        pass<2, LDP, INV, EPI>(v, sr, s0, lo, lane, tpt, first, last, lay, smem, mp, layout, ep);
+        pass<2, LDP, INV, EPI>(v, sr, s0, lo, lane, tpt, first, last, rebase, lay, smem, mp, layout, ep);
       else if (LOGR != 3)
-        pass<1, LDP, INV, EPI>(v, sr, s0, lo, lane, tpt, first, last, lay, smem, mp, layout, ep);
+        pass<1, LDP, INV, EPI>(v, sr, s0, lo, lane, tpt, first, last, rebase, lay, smem, mp, layout, ep);
       if (!last) {
         // the next pass exchanges within each warp when both hold one group
         // per thread of a contiguous tile and start at local bit 5 or below

@@ -62,8 +62,8 @@ extern "C" int bntt_probe_imad_peak(bntt_ctx* c, double* ops_per_second) {
   return BNTT_OK;
 }
 
-// Butterfly ceiling: the kernels' own butterfly (pseudo-Mersenne multiply,
-// the reference's addmod / submod) on register-resident data, in radix-4
+// Butterfly ceiling: the kernels' own butterfly (lazy_stages: pseudo-Mersenne
+// multiply, sums on partly reduced values) on register-resident data, in radix-4
 // groups of 4 butterflies (the persistent kernel's 4 elements per thread), at
 // the persistent kernel's occupancy (4 CTAs of 256 threads per SM).  No
 // memory traffic, no index arithmetic: the rate any NTT kernel of this
@@ -89,13 +89,10 @@ __global__ void __launch_bounds__(256, kProbeCtasPerSm) k_butterfly_probe(uint4*
     if (e < 4) v[e] = t;
     else w[e - 4] = t;
   }
-  for (uint32_t it = 0; it < iters; ++it) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) butterfly<ArithFast>(v[k], v[k + 2], w[0], mp);
-    butterfly<ArithFast>(v[0], v[1], w[1], mp);
-    butterfly<ArithFast>(v[2], v[3], w[2], mp);
-  }
-  uint32_t s = 0;
+  bool rerun = false;  // as the kernels: noted, and acted on outside the stages
+  for (uint32_t it = 0; it < iters; ++it)
+    lazy_stages<2>(v, 0, [&](int t, int u) { return w[t + u]; }, mp.k, rerun);
+  uint32_t s = rerun ? 1u : 0u;
 #pragma unroll
   for (int e = 0; e < 4; ++e) s ^= v[e].w[0] ^ v[e].w[1] ^ v[e].w[2] ^ v[e].w[3];
   if (s == 0x9E3779B9u) out[0] = make_uint4(s, 0u, 0u, 0u);  // keeps the results live
