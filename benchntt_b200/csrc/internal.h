@@ -73,7 +73,7 @@ const std::vector<SubKernel>& sub_kernels();
 const SubKernel* pick_sub_kernel(int m, int map, int fast, int logr_pref = 0, int tpc_pref = 0);
 // Launch over a geometry; returns BNTT status.
 int launch_sub(bntt_ctx* ctx, const SubKernel* k, const void* geom, const ModParams& mp,
-               int layout, cudaStream_t stream, int grid_cap = 0);
+               int layout, cudaStream_t stream);
 int blocks_per_sm(const SubKernel* k);
 
 // Autotuner choices (nullptr / -1 when not tuned).

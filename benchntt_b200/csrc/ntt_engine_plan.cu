@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256)
 
 // One HBM pass of the inverse on the compile-time tile (NttTile::run_inv, 4
 // elements per thread, 256-thread CTAs of 256 / 2^(M-2) sub-transforms, 4
-// resident per SM), persistent over the tiles like the forward k_ntt_sub:
+// resident per SM), one CTA per tile like the forward k_ntt_sub:
 // whole transforms of 2^3..2^10 points (contiguous), or one pass of a larger
 // transform (interleaved for the strided passes).  `finishing` marks the
 // pass that ends the transform (stage 0 inside it), which applies N^-1 from
@@ -97,14 +97,10 @@ __global__ void __launch_bounds__(256, 4)
   static_assert(T::THREADS == 256, "tile shape");
   extern __shared__ uint4 smem[];
   const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
-  const uint64_t ntiles = (g.nsub + TPC - 1) / TPC;
   const uint4* scale_at = finishing ? g.tw : nullptr;
-  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const SubRef sr = make_subref(g, tile * TPC + (uint64_t)sub);
-    if (layout == LAYOUT_HILO) T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_HILO, scale_at);
-    else T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
-    T::sync();  // smem is reused by the next tile
-  }
+  const SubRef sr = make_subref(g, (uint64_t)blockIdx.x * TPC + (uint64_t)sub);
+  if (layout == LAYOUT_HILO) T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_HILO, scale_at);
+  else T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
 }
 
 template <int M, int MAP>
@@ -112,16 +108,9 @@ int launch_tile_inv(bntt_plan* p, const SubGeom& g, int finishing, cudaStream_t 
   constexpr int TPC = 256 >> (M - 2);
   using T = NttTile<M, 2, TPC, MAP, ArithFast>;
   constexpr size_t smem = (size_t)T::SMEM_SLOTS * 16;
-  static std::atomic<int> cached{0};  // resident CTAs per SM; relaxed: same value from any thread
-  int bps = cached.load(std::memory_order_relaxed);
-  if (!bps) {
-    BNTT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, (const void*)k_ntt_tile_inv<M, MAP>, 256, smem));
-    bps = std::max(1, bps);
-    cached.store(bps, std::memory_order_relaxed);
-  }
   const uint64_t ntiles = (g.nsub + TPC - 1) / TPC;
-  const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)bps * p->ctx->sms);
-  k_ntt_tile_inv<M, MAP><<<grid, 256, smem, s>>>(g, p->mp, p->layout, finishing);
+  BNTT_REQUIRE(ntiles <= 0x7fffffffu, "%llu tiles are more than one launch takes", (unsigned long long)ntiles);
+  k_ntt_tile_inv<M, MAP><<<(unsigned)ntiles, 256, smem, s>>>(g, p->mp, p->layout, finishing);
   BNTT_CK(cudaGetLastError());
   p->ctx->launches++;
   return BNTT_OK;

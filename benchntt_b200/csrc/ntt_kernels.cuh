@@ -5,8 +5,15 @@
 
 namespace bntt {
 
-// Persistent launch over the tiles of a geometry: tile t holds sub-transforms
-// [t*TPC, t*TPC + TPC); each CTA walks tiles blockIdx.x, +gridDim.x, ...
+// One CTA per tile of a geometry: CTA t transforms sub-transforms
+// [t*TPC, t*TPC + TPC).  The hardware hands a CTA to an SM as soon as one of
+// its resident CTAs ends, which balances what the warp schedulers do not:
+// among the CTAs of an SM the oldest gets most of the issue slots, so with a
+// fixed share of the tiles per CTA (a grid of the resident CTAs walking the
+// tiles) the CTAs drifted apart and the SM ran its last third with fewer of
+// them (39 % of the warp slots active on average, of the 50 % the registers
+// allow).  65,536 x 1024: 1331 -> 1219 us; a grid of 2, 4 and 8 times the
+// resident CTAs lies between (1282, 1247, 1229).
 // MINB > 0 asks for at least MINB resident CTAs per SM (fewer registers per
 // thread, more warps to hide the latency of the carry chains).
 template <int M, int LOGR, int TPC, int MAP, class Arith, int MINB>
@@ -16,20 +23,17 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, Arith>::THREADS, MI
   extern __shared__ uint4 smem[];
   const int tid = threadIdx.x;
   const int sub = T::sub_of(tid), lane = T::lane_of(tid);
-  const uint64_t ntiles = (g.nsub + TPC - 1) / TPC;
-  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const SubRef sr = make_subref(g, tile * TPC + (uint64_t)sub);
-    // the element layout as a constant in each branch: no word select per
-    // HBM load and store
-    if (layout == LAYOUT_HILO) T::template run<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_HILO, MulB{g.b, g.y, g.bmask});
-    else T::template run<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_U128, MulB{g.b, g.y, g.bmask});
-    if constexpr (T::NPASS > 1) T::sync();  // smem is reused by the next tile
-  }
+  const SubRef sr = make_subref(g, (uint64_t)blockIdx.x * TPC + (uint64_t)sub);
+  // the element layout as a constant in each branch: no word select per
+  // HBM load and store
+  if (layout == LAYOUT_HILO) T::template run<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_HILO, MulB{g.b, g.y, g.bmask});
+  else T::template run<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_U128, MulB{g.b, g.y, g.bmask});
 }
 
-// The same over contiguous sub-transforms (L = 0: tile t is the 16-byte
-// elements [t*TPC*2^M, (t+1)*TPC*2^M) of g.x), with every tile's input copied
-// into shared memory by cp.async one tile ahead: while a CTA transforms tile
+// Contiguous sub-transforms (L = 0: tile t is the 16-byte elements
+// [t*TPC*2^M, (t+1)*TPC*2^M) of g.x), each CTA walking tiles blockIdx.x,
+// +gridDim.x, ..., with every tile's input copied into shared memory by
+// cp.async one tile ahead: while a CTA transforms tile
 // t, the copy of its next tile is in flight, so the load latency that bounds
 // small transforms (little work per element, a few tiles per CTA) overlaps
 // the arithmetic.  The copy lands in the tile's exchange slots, the first pass

@@ -65,14 +65,17 @@ int blocks_per_sm(const SubKernel* k) {
 }
 
 int launch_sub(bntt_ctx* ctx, const SubKernel* k, const void* geom, const ModParams& mp,
-               int layout, cudaStream_t stream, int grid_cap) {
+               int layout, cudaStream_t stream) {
   const SubGeom& g = *static_cast<const SubGeom*>(geom);
   const uint64_t ntiles = (g.nsub + (uint64_t)k->tpc - 1) / (uint64_t)k->tpc;
   if (ntiles == 0) return BNTT_OK;
-  const int bps = blocks_per_sm(k);
-  if (bps < 0) return -bps;
-  uint64_t grid = std::min<uint64_t>(ntiles, (uint64_t)bps * (uint64_t)ctx->sms);
-  if (grid_cap > 0) grid = std::min<uint64_t>(grid, (uint64_t)grid_cap);
+  BNTT_REQUIRE(ntiles <= 0x7fffffffu, "%llu tiles are more than one launch takes", (unsigned long long)ntiles);
+  uint64_t grid = ntiles;  // one CTA per tile; the staged kernels are persistent
+  if (k->smem > 48 * 1024 || k->src != 0) {
+    const int bps = blocks_per_sm(k);
+    if (bps < 0) return -bps;
+    if (k->src != 0) grid = std::min<uint64_t>(grid, (uint64_t)bps * (uint64_t)ctx->sms);
+  }
   SubGeom gg = g;
   ModParams mm = mp;
   int lay = layout;
