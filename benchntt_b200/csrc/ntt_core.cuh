@@ -393,7 +393,7 @@ struct NttTile {
 
   // The inverse network of the same passes: the last pass first, each pass's
   // stages in reverse order as Gentleman-Sande butterflies on the inverse
-  // table (gs_butterfly).  The store that finishes the transform (pass 0)
+  // table, on partly reduced values (inverse_stages).  The store that finishes the transform (pass 0)
   // multiplies the lower half of each group -- the x outputs of stage 0 --
   // by *scale_at (N^-1) when scale_at is not null; the upper half gets N^-1
   // through the inverse table's entry 1.  Fast moduli only.
@@ -403,23 +403,6 @@ struct NttTile {
                                                  const uint4* scale_at) {
     U128 v[R];
     pass_inv<NPASS - 1, LDP>(v, sr, sub, lane, smem, mp, layout, scale_at);
-  }
-
-  // stage t of a group of 2^r registers from e0, inverse butterflies
-  template <int r, int t>
-  __device__ __forceinline__ static void stage_inv(U128 (&v)[R], int e0, uint32_t gt,
-                                                   const uint4* tw, const ModParams& mp) {
-    constexpr int half = 1 << (r - 1 - t);
-#pragma unroll
-    for (int u = 0; u < (1 << t); ++u) {
-      const uint4 tv = __ldg(tw + (gt << t) + u);
-      const U128 w = U128{{tv.x, tv.y, tv.z, tv.w}};
-#pragma unroll
-      for (int k = 0; k < half; ++k) {
-        const int j = e0 + ((u << (r - t)) | k);
-        gs_butterfly<Arith>(v[j], v[j + half], w, mp);
-      }
-    }
   }
 
   template <int P, int LDP>
@@ -461,22 +444,29 @@ struct NttTile {
     for (int i = 0; i < GPT; ++i) {
       const int g = lane + i * TPT;
       const uint32_t gt = (sr.trow << s0) + (uint32_t)(g >> lo);
-      if constexpr (r > 3) stage_inv<r, 3>(v, i * G, gt, sr.tw, mp);
-      if constexpr (r > 2) stage_inv<r, 2>(v, i * G, gt, sr.tw, mp);
-      if constexpr (r > 1) stage_inv<r, 1>(v, i * G, gt, sr.tw, mp);
-      stage_inv<r, 0>(v, i * G, gt, sr.tw, mp);
+      inverse_stages<r, P == 0>(v, i * G, [&](int t, int u) {
+        const uint4 tv = __ldg(sr.tw + (gt << t) + u);
+        return U128{{tv.x, tv.y, tv.z, tv.w}};
+      }, mp.k);
     }
 
-    // ---- N^-1 on the finishing store
+    // ---- canonical results; N^-1 on the finishing store
     if constexpr (P == 0) {
-      if (scale_at && sr.valid) {
+      if (scale_at) {
         const uint4 f = __ldg(scale_at);
         const U128 fs = U128{{f.x, f.y, f.z, f.w}};
 #pragma unroll
         for (int i = 0; i < GPT; ++i)
 #pragma unroll
-          for (int j = 0; j < G / 2; ++j) v[i * G + j] = Arith::mul(v[i * G + j], fs, mp);
+          for (int j = 0; j < G / 2; ++j) v[i * G + j] = mul_lazy(fs, v[i * G + j], mp.k);
+      } else {
+#pragma unroll
+        for (int i = 0; i < GPT; ++i)
+#pragma unroll
+          for (int j = 0; j < G / 2; ++j) v[i * G + j] = fold_top(v[i * G + j], mp.k);
       }
+#pragma unroll
+      for (int j = 0; j < R; ++j) v[j] = reduce_once(v[j], mp.k);
     }
 
     // ---- scatter

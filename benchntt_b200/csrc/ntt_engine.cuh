@@ -70,25 +70,6 @@ struct NttEngine {
   };
   __device__ __forceinline__ static int pad(int l) { return l + (l >> 3); }
 
-  // Stage t of a group of 2^r elements starting at register e0: butterflies
-  // of distance 2^(r-1-t), twiddle T[(gt << t) + u] for the u-th block.
-  template <int r, int t, bool INV>
-  __device__ __forceinline__ static void stage(U128 (&v)[R], int e0, uint32_t gt, const uint4* tw,
-                                               const ModParams& mp) {
-    constexpr int half = 1 << (r - 1 - t);
-#pragma unroll
-    for (int u = 0; u < (1 << t); ++u) {
-      const uint4 tv = __ldg(tw + (gt << t) + u);
-      const U128 w = U128{{tv.x, tv.y, tv.z, tv.w}};
-#pragma unroll
-      for (int k = 0; k < half; ++k) {
-        const int j = e0 + ((u << (r - t)) | k);
-        if constexpr (INV) gs_butterfly<Arith>(v[j], v[j + half], w, mp);
-        else butterfly<Arith>(v[j], v[j + half], w, mp);
-      }
-    }
-  }
-
   // One pass of width r (1 <= r <= LOGR) over the thread's GPT = R / 2^r
   // groups: gather (global on the first pass, else shared), r butterfly
   // stages with static register indices, scatter (global on the last pass).
@@ -165,9 +146,7 @@ struct NttEngine {
       }
     }
     // r stages per group; stage t of the group reads T[(gt << t) + u],
-    // u < 2^t.  The inverse runs them in reverse order; with 3 or 4 stages
-    // each of its stages is a separate instantiation (stage()), since the
-    // compiler otherwise keeps v in local memory for the reversed loop.
+    // u < 2^t.  The inverse runs them in reverse order.
 #pragma unroll
     for (int i = 0; i < GPT; ++i) {
       const int g = lane + i * tpt;
@@ -177,15 +156,14 @@ struct NttEngine {
           const uint4 tv = __ldg(sr.tw + (gt << t) + u);
           return U128{{tv.x, tv.y, tv.z, tv.w}};
         }, mp.k, rerun);
-      } else if constexpr (INV && r > 2) {
-        if constexpr (r > 3) stage<r, 3, true>(v, i * G, gt, sr.tw, mp);
-        stage<r, 2, true>(v, i * G, gt, sr.tw, mp);
-        stage<r, 1, true>(v, i * G, gt, sr.tw, mp);
-        stage<r, 0, true>(v, i * G, gt, sr.tw, mp);
+      } else if constexpr (INV) {
+        inverse_stages<r, false>(v, i * G, [&](int t, int u) {
+          const uint4 tv = __ldg(sr.tw + (gt << t) + u);
+          return U128{{tv.x, tv.y, tv.z, tv.w}};
+        }, mp.k);
       } else {
 #pragma unroll
-        for (int tt = 0; tt < r; ++tt) {
-          const int t = INV ? r - 1 - tt : tt;
+        for (int t = 0; t < r; ++t) {
           const int half = 1 << (r - 1 - t);
 #pragma unroll
           for (int u = 0; u < (1 << t); ++u) {
@@ -194,8 +172,7 @@ struct NttEngine {
 #pragma unroll
             for (int k = 0; k < half; ++k) {
               const int j = (u << (r - t)) | k;
-              if constexpr (INV) gs_butterfly<Arith>(v[i * G + j], v[i * G + j + half], w, mp);
-              else butterfly<Arith>(v[i * G + j], v[i * G + j + half], w, mp);
+              butterfly<Arith>(v[i * G + j], v[i * G + j + half], w, mp);
             }
           }
         }
@@ -220,16 +197,33 @@ struct NttEngine {
         }
       }
     }
-    // the inverse's N^-1 (EPI_SCALE_AT): the upper half of each group holds
-    // y outputs of the last stage, whose table entry carries it already
-    if constexpr ((EPI & EPI_SCALE_AT) != 0) {
-      if (last && ep && sr.valid) {
-        const uint4 f = __ldg(ep->scale_at);
-        const U128 fs = U128{{f.x, f.y, f.z, f.w}};
+    // the inverse's results: N^-1 on the x outputs (EPI_SCALE, EPI_SCALE_AT;
+    // the y outputs carry it through the last stage's table entry), canonical
+    if constexpr (INV) {
+      if (last) {
+        U128 f{};
+        bool scaled = false;
+        if constexpr ((EPI & EPI_SCALE_AT) != 0) {
+          if (ep) {
+            const uint4 t = __ldg(ep->scale_at);
+            f = U128{{t.x, t.y, t.z, t.w}};
+            scaled = true;
+          }
+        }
+        if constexpr ((EPI & EPI_SCALE) != 0) {
+          if (ep && ep->has_scale) {
+            f = ep->scale;
+            scaled = true;
+          }
+        }
 #pragma unroll
         for (int i = 0; i < GPT; ++i)
 #pragma unroll
-          for (int j = 0; j < (INV ? G / 2 : G); ++j) v[i * G + j] = Arith::mul(v[i * G + j], fs, mp);
+          for (int j = 0; j < G; ++j) {
+            U128& e = v[i * G + j];
+            if (j < G / 2) e = scaled ? mul_lazy(f, e, mp.k) : fold_top(e, mp.k);
+            e = reduce_once(e, mp.k);
+          }
       }
     }
     // scatter
@@ -241,18 +235,10 @@ struct NttEngine {
         for (int j = 0; j < G; ++j) {
           if (sr.valid) {
             uint4* yp = gq + (size_t)(j * gstep);
-            if constexpr (EPI != 0) {
-              if (ep) {
-                // the inverse's N^-1: the upper half of the group holds y
-                // outputs of the last stage, whose table entry carries it
-                const bool scaled = !INV || j < G / 2;
-                if constexpr ((EPI & EPI_SCALE) != 0) {
-                  if (ep->has_scale && scaled) v[i * G + j] = Arith::mul(v[i * G + j], ep->scale, mp);
-                }
-                if ((EPI & EPI_MUL) != 0 && ep->mul.b) {
-                  const uint4 bv = __ldg(ep->mul.b + ((uint64_t)(yp - ep->mul.ybase) & ep->mul.bmask));
-                  v[i * G + j] = Arith::mul(v[i * G + j], from_mem(bv, layout), mp);
-                }
+            if constexpr ((EPI & EPI_MUL) != 0) {
+              if (ep && ep->mul.b) {
+                const uint4 bv = __ldg(ep->mul.b + ((uint64_t)(yp - ep->mul.ybase) & ep->mul.bmask));
+                v[i * G + j] = Arith::mul(v[i * G + j], from_mem(bv, layout), mp);
               }
             }
             *yp = to_mem(v[i * G + j], layout);
