@@ -3,7 +3,6 @@
 // instantiated in batch_kfast.cu / batch_kref.cu.
 #include <algorithm>
 #include <atomic>
-#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -13,23 +12,15 @@
 
 namespace bntt {
 
-const void* batch_kernel_fast_minb(int minb, int layout);
+const void* batch_kernel_fast(int layout);
 const void* batch_kernel_ref();
 
-// Resident CTAs per SM the fast batch kernel is compiled for (2 to 5,
-// default 4), read once at start-up from BNTT_BATCH_MINB.
-static const int g_batch_minb = [] {
-  const char* e = getenv("BNTT_BATCH_MINB");
-  const int v = e ? atoi(e) : 4;
-  return v == 2 || v == 3 || v == 5 ? v : 4;
-}();
-
+// Shared memory of an item: the exchange slots of the sub-transforms the
+// threads hold at a time (NttTile::SMEM_SLOTS; one pass needs none).
 size_t shape_smem(int s) {
   const BatchShape& b = kShapes[s];
-  const int npass = (b.m + b.logr - 1) / b.logr;
-  if (npass <= 1) return 0;
-  if (b.m <= 2) return (size_t)b.tpc * ((size_t)1 << b.m) * 16;  // one-thread tiles
-  return NttEngine<kBatchLogR, ArithFast>::smem_slots(b.m, b.map, kBatchThreads) * 16;
+  if (b.m <= b.logr) return 0;
+  return ((size_t)kBatchThreads << b.logr) * 16;
 }
 
 // Resident CTAs per SM of a batch kernel (forward or inverse) at the largest
@@ -111,13 +102,13 @@ void free_schedule(bntt_ctx* c, Schedule& s) {
 }
 
 const void* batch_kernel(bool fast, int layout) {
-  return fast ? batch_kernel_fast_minb(g_batch_minb, layout) : batch_kernel_ref();
+  return fast ? batch_kernel_fast(layout) : batch_kernel_ref();
 }
 
 constexpr int kMaxLog2n = 24;  // plans hold 2^1..2^24 points
 
 // HBM passes of a large batch job: the fewest passes, then the fewest
-// engine passes (a pass of m stages is ceil(m / 2) of them).  A strided pass
+// 4-element tile passes (a pass of m stages is ceil(m / 2) of them).  A strided pass
 // (all but the last) has 5..7 stages, so its tile of 2^(10 - m) adjacent
 // columns covers at least 128 bytes of each row, and needs that many columns
 // (2^(10 - m) <= 2^l); the last, contiguous pass has 3..10 stages.
@@ -193,8 +184,9 @@ static int make_items(const bntt_batch* b, Schedule& sc, const uint32_t per_size
   for (auto& l : sc.later) l.clear();
   sc.nslots = sc.large.size();
   sc.pass_tiles.assign(sc.nslots * kMaxPasses, 0);
+  uint32_t nsmall = 0;
+  for (int n = 1; n <= 10; ++n) nsmall += per_size[n];
   for (size_t slot = 0; slot < sc.large.size(); ++slot) {
-    const uint32_t ji = sc.large[slot];
     const int n = sc.large_n[slot];
     const std::vector<int>& passes = split_of(n);
     BNTT_REQUIRE(!passes.empty() && passes.size() <= (size_t)kMaxPasses, "log2n %d needs too many passes", n);
@@ -215,7 +207,7 @@ static int make_items(const bntt_batch* b, Schedule& sc, const uint32_t per_size
       WorkItem w{};
       w.shape = (uint16_t)shape;
       w.kind = ITEM_PASS;
-      w.a = ji;
+      w.a = nsmall + (uint32_t)slot;  // large jobs' descriptors follow the small ones
       w.pass = (uint16_t)p;
       w.wait = (uint16_t)((run > 0 ? 1 : 0) | (run == 0 ? 2 : 0) | (s0 << 8));
       for (uint32_t t = 0; t < tiles; ++t) {
@@ -262,18 +254,13 @@ static int make_items(const bntt_batch* b, Schedule& sc, const uint32_t per_size
 }
 
 // One validating pass over the jobs: sizes counted per small size, large
-// jobs listed.  `fill` also writes the jobs' device descriptors.
+// jobs listed.
 static int scan_jobs(const bntt_batch* b, Schedule& sc, const bntt_job* jobs, size_t count,
-                     uint32_t per_size[11], bool fill) {
+                     uint32_t per_size[11]) {
   const size_t np = b->plans.size();
-  const uint4* const* tw = sc.plan_tw.data();
   const uint8_t* plog = sc.plan_log2n.data();
   sc.large.clear();
   sc.large_n.clear();
-  if (fill) {
-    sc.djobs.resize(count);
-    sc.job_log2n.resize(count);
-  }
   for (size_t i = 0; i < count; ++i) {
     const bntt_job& jb = jobs[i];
     BNTT_REQUIRE(jb.plan < np, "job %zu: plan index %u out of range", i, jb.plan);
@@ -286,15 +273,6 @@ static int scan_jobs(const bntt_batch* b, Schedule& sc, const bntt_job* jobs, si
       sc.large.push_back((uint32_t)i);
       sc.large_n.push_back((uint8_t)n);
     }
-    if (fill) {
-      DevJob& d = sc.djobs[i];
-      d.x = static_cast<const uint4*>(jb.x);
-      d.y = static_cast<uint4*>(jb.y);
-      d.tw = tw[jb.plan];
-      d.log2n = n;
-      d.slot = n <= 10 ? 0u : (uint32_t)(sc.large.size() - 1);
-      sc.job_log2n[i] = (uint8_t)n;
-    }
   }
   return BNTT_OK;
 }
@@ -303,22 +281,24 @@ int build_schedule(const bntt_batch* b, Schedule& sc, const bntt_job* jobs, size
                    bool inverse) {
   sc.dev_build = false;
   plan_fields(b, sc, inverse);
-  uint32_t per_size[11] = {}, first[11], fill[11];
-  if (int rc = scan_jobs(b, sc, jobs, count, per_size, true)) return rc;
-  // small jobs in size order, largest size first (a counting sort over the
-  // compact size array)
+  uint32_t per_size[11] = {}, first[11], at[11];
+  if (int rc = scan_jobs(b, sc, jobs, count, per_size)) return rc;
+  // descriptors in size order, largest small size first, then the large jobs
   const uint32_t small = size_offsets(per_size, first);
-  std::copy(first, first + 11, fill);
-  sc.order.resize(small);
-  const uint8_t* sizes = sc.job_log2n.data();
+  std::copy(first, first + 11, at);
+  sc.djobs.resize(count);
+  uint32_t slot = 0;
   for (size_t i = 0; i < count; ++i) {
-    const uint32_t n = sizes[i];
-    if (n <= 10) sc.order[fill[n]++] = (uint32_t)i;
+    const bntt_job& jb = jobs[i];
+    const uint32_t n = sc.plan_log2n[jb.plan];
+    const DevJob d{static_cast<const uint4*>(jb.x), static_cast<uint4*>(jb.y), sc.plan_tw[jb.plan], n,
+                   n <= 10 ? 0u : slot};
+    sc.djobs[n <= 10 ? at[n]++ : small + slot++] = d;
   }
   return make_items(b, sc, per_size, first, inverse);
 }
 
-// The host half of a schedule whose job descriptors and size order the
+// The host half of a schedule whose size-ordered job descriptors the
 // device builds (k_build_jobs): validation, sizes, work items, the table of
 // large jobs and the plans' table.  The caller's job array is read again by
 // the upload that follows.
@@ -327,12 +307,11 @@ int build_schedule_dev(const bntt_batch* b, Schedule& sc, const bntt_job* jobs, 
   sc.dev_build = true;
   plan_fields(b, sc, inverse);
   uint32_t per_size[11] = {};
-  if (int rc = scan_jobs(b, sc, jobs, count, per_size, false)) return rc;
+  if (int rc = scan_jobs(b, sc, jobs, count, per_size)) return rc;
   sc.small = size_offsets(per_size, sc.first);
   sc.count = count;
   sc.raw = jobs;
   sc.djobs.clear();
-  sc.order.clear();
   sc.plan_ref.resize(b->plans.size());
   for (size_t k = 0; k < b->plans.size(); ++k) sc.plan_ref[k] = PlanRef{sc.plan_tw[k], sc.plan_log2n[k], 0u};
   sc.large_ref.resize(sc.large.size());
@@ -361,15 +340,13 @@ static int upload(bntt_batch* b, Schedule& sc, cudaStream_t stream, bool inverse
   const size_t ib = sc.items.size() * sizeof(WorkItem), cb = (kCtlHeader + sc.nslots * kMaxPasses) * 4,
                pb = sc.pass_tiles.size() * 4;
   auto r256 = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  // Host-built: [djobs][order][items][pass tiles], all copied.  Device-built:
+  // Host-built: [djobs][items][pass tiles], all copied.  Device-built:
   // [the caller's jobs][plans][large jobs][items][pass tiles] copied, then
-  // [djobs][order][fill counters] written on the device by k_build_jobs.
-  size_t o_jb = 0, o_ob = 0, o_ib = 0, o_pb = 0, staged = 0, total = 0;
+  // [djobs][fill counters] written on the device by k_build_jobs.
+  size_t o_jb = 0, o_ib = 0, o_pb = 0, staged = 0, total = 0;
   size_t o_raw = 0, o_plan = 0, o_large = 0, o_fill = 0;
   if (!sc.dev_build) {
-    const size_t jb = sc.djobs.size() * sizeof(DevJob), ob = sc.order.size() * 4;
-    o_ob = r256(jb);
-    o_ib = o_ob + r256(ob);
+    o_ib = r256(sc.djobs.size() * sizeof(DevJob));
     o_pb = o_ib + r256(ib);
     staged = total = o_pb + r256(pb);
   } else {
@@ -381,8 +358,7 @@ static int upload(bntt_batch* b, Schedule& sc, cudaStream_t stream, bool inverse
     o_pb = o_ib + r256(ib);
     staged = o_pb + r256(pb);
     o_jb = staged;
-    o_ob = o_jb + r256(sc.count * sizeof(DevJob));
-    o_fill = o_ob + r256((size_t)sc.small * 4);
+    o_fill = o_jb + r256(sc.count * sizeof(DevJob));
     total = o_fill + 256;
   }
   if (sc.exec) {
@@ -412,7 +388,6 @@ static int upload(bntt_batch* b, Schedule& sc, cudaStream_t stream, bool inverse
   char* h = static_cast<char*>(sc.stage[si]);
   if (!sc.dev_build) {
     if (!sc.djobs.empty()) memcpy(h + o_jb, sc.djobs.data(), sc.djobs.size() * sizeof(DevJob));
-    if (!sc.order.empty()) memcpy(h + o_ob, sc.order.data(), sc.order.size() * 4);
   } else {
     if (sc.count) memcpy(h + o_raw, sc.raw, sc.count * sizeof(bntt_job));
     sc.staged_raw = reinterpret_cast<const bntt_job*>(h + o_raw);
@@ -431,7 +406,7 @@ static int upload(bntt_batch* b, Schedule& sc, cudaStream_t stream, bool inverse
   char* d = static_cast<char*>(sc.d_sched[set]);
   BNTT_CK(cudaMemcpyAsync(d, h, staged, cudaMemcpyHostToDevice, cs));
   BNTT_CK(cudaEventRecord(sc.stage_done[si], cs));
-  // descriptors and size order, built on the device after the copy, on the
+  // descriptors in size order, built on the device after the copy, on the
   // copy's stream: the build runs while earlier launches finish (it writes
   // only the buffer they do not read), off the path between two launches
   if (sc.dev_build && sc.count) {
@@ -439,8 +414,8 @@ static int upload(bntt_batch* b, Schedule& sc, cudaStream_t stream, bool inverse
     if (int rc = launch_build_jobs(reinterpret_cast<const bntt_job*>(d + o_raw), sc.count,
                                    reinterpret_cast<const PlanRef*>(d + o_plan),
                                    reinterpret_cast<const LargeRef*>(d + o_large),
-                                   (uint32_t)sc.large_ref.size(), sc.first, reinterpret_cast<uint32_t*>(d + o_fill),
-                                   reinterpret_cast<DevJob*>(d + o_jb), reinterpret_cast<uint32_t*>(d + o_ob), cs))
+                                   (uint32_t)sc.large_ref.size(), sc.first, sc.small,
+                                   reinterpret_cast<uint32_t*>(d + o_fill), reinterpret_cast<DevJob*>(d + o_jb), cs))
       return rc;
     c->launches++;
     b->last_launches++;
@@ -471,7 +446,6 @@ static int upload(bntt_batch* b, Schedule& sc, cudaStream_t stream, bool inverse
   ba.items = reinterpret_cast<const WorkItem*>(d + o_ib);
   ba.nitems = (uint32_t)sc.items.size();
   ba.jobs = reinterpret_cast<const DevJob*>(d + o_jb);
-  ba.order = reinterpret_cast<const uint32_t*>(d + o_ob);
   ba.ctl = static_cast<uint32_t*>(sc.d_ctl);
   ba.pass_tiles = reinterpret_cast<const uint32_t*>(d + o_pb);
   ba.wait_polls = b->inject_polls ? b->inject_polls : kWaitPolls;
@@ -567,8 +541,7 @@ int bntt_batch_create(bntt_ctx* c, bntt_batch** out, bntt_plan* const* plans, si
     const int tuned = tuned_batch_small_shape(m);
     b->shapes.small[m] = tuned >= 0 ? tuned : batch_shape_for(m, MAP_CONTIG, 0);
     b->shapes.pass_il[m] = batch_shape_for(m, MAP_INTERLEAVED, 0);
-    b->shapes.pass_contig[m] = batch_shape_for(m, MAP_CONTIG, 4);
-    if (b->shapes.pass_contig[m] < 0) b->shapes.pass_contig[m] = batch_shape_for(m, MAP_CONTIG, 0);
+    b->shapes.pass_contig[m] = batch_shape_for(m, MAP_CONTIG, 0);
   }
   if (cudaError_t e = cudaStreamCreateWithFlags(&b->upload_stream, cudaStreamNonBlocking)) {
     delete b;
@@ -963,10 +936,11 @@ extern "C" int bntt_batch_run_dev_noalloc(bntt_batch* b, const bntt_job* jobs, s
   Schedule sc;  // host-side vectors only
   if (int rc = build_schedule(b, sc, jobs, count)) return rc;
   const size_t cb = (kCtlHeader + sc.nslots * kMaxPasses) * 4, pb = sc.pass_tiles.size() * 4,
-               ib = sc.items.size() * sizeof(WorkItem), ob = sc.order.size() * 4,
-               jb = sc.djobs.size() * sizeof(DevJob);
-  const size_t o_ctl = 0, o_pt = round256(o_ctl + cb), o_it = round256(o_pt + pb),
-               o_or = round256(o_it + ib), o_jb = round256(o_or + ob), need = round256(o_jb + jb);
+               ib = sc.items.size() * sizeof(WorkItem), jb = sc.djobs.size() * sizeof(DevJob);
+  // (four more bytes per transform are reserved, so that the lists the array
+  // takes do not depend on how the schedule is laid out)
+  const size_t o_ctl = 0, o_pt = round256(o_ctl + cb), o_it = round256(o_pt + pb), o_jb = round256(o_it + ib),
+               need = round256(o_jb + jb) + round256((sc.djobs.size() - sc.large.size()) * 4);
   if (need > kNoAllocScratchBytes)
     return set_error(BNTT_EINVAL,
                      "this job list needs %zu bytes of scratch; the no-allocation entry point "
@@ -980,7 +954,6 @@ extern "C" int bntt_batch_run_dev_noalloc(bntt_batch* b, const bntt_job* jobs, s
   b->noalloc_err = reinterpret_cast<const uint32_t*>(s + o_ctl) + 1;
   if (pb) BNTT_CK(cudaMemcpyAsync(s + o_pt, sc.pass_tiles.data(), pb, cudaMemcpyHostToDevice, st));
   if (ib) BNTT_CK(cudaMemcpyAsync(s + o_it, sc.items.data(), ib, cudaMemcpyHostToDevice, st));
-  if (ob) BNTT_CK(cudaMemcpyAsync(s + o_or, sc.order.data(), ob, cudaMemcpyHostToDevice, st));
   if (jb) BNTT_CK(cudaMemcpyAsync(s + o_jb, sc.djobs.data(), jb, cudaMemcpyHostToDevice, st));
   if (sc.items.empty()) return BNTT_OK;
   const void* fn = batch_kernel(b->fast, b->layout);
@@ -996,7 +969,6 @@ extern "C" int bntt_batch_run_dev_noalloc(bntt_batch* b, const bntt_job* jobs, s
   ba.items = reinterpret_cast<const WorkItem*>(s + o_it);
   ba.nitems = (uint32_t)sc.items.size();
   ba.jobs = reinterpret_cast<const DevJob*>(s + o_jb);
-  ba.order = reinterpret_cast<const uint32_t*>(s + o_or);
   ba.ctl = reinterpret_cast<uint32_t*>(s + o_ctl);
   ba.pass_tiles = reinterpret_cast<const uint32_t*>(s + o_pt);
   ba.wait_polls = kWaitPolls;

@@ -1,19 +1,18 @@
 // batch_dev.cuh -- device side of the batch engine: many independent transforms of uneven sizes in one persistent,
 // graph-launched work-queue kernel.
 //
-// Work items (16 bytes each) are tiles of 256 threads:
-//   SMALL   TPC transforms of one size 2^n <= 1024, taken from a list of
-//           jobs sorted by size (one sub-transform per job)
+// Work items (16 bytes each) are tiles of kBatchThreads threads:
+//   SMALL   TPC transforms of one size 2^n <= 1024, consecutive in the
+//           size-sorted job descriptors (one sub-transform per job)
 //   PASS p  TPC sub-transforms of HBM pass p of one large transform
-//           (n > 10, passes from engine_split: at most kBatchMaxPass stages
-//           so strided passes keep >= 8 adjacent columns, and the fewest
-//           engine passes: 2^16 = 8 + 8, 2^20 = 8 + 6 + 6)
+//           (n > 10, passes from batch_split: strided passes of 5..7 stages
+//           keep >= 8 adjacent columns; 2^16 = 6 + 10, 2^20 = 6 + 6 + 8)
 // A CTA takes the next item with an atomic counter.  Queue order is: all
 // first passes of large jobs, then small tiles from the largest size down,
 // then later passes.  Pass p > 0 of a job reads what pass p-1 wrote, so its
 // tiles first wait until the job's pass p-1 counter reaches that pass's tile
 // count.  The wait cannot deadlock: every pass p-1 tile was handed out
-// before any pass p tile and its CTA finishes it without waiting.  The wait is
+// before any pass p tile (see the loop in k_batch).  The wait is
 // still bounded; when it gives up it raises the error word, the tile is
 // skipped, and bntt_batch_status() reports BNTT_ETIMEOUT.
 //
@@ -23,17 +22,18 @@
 #pragma once
 #include "internal.h"
 #include "ntt_core.cuh"
-#include "ntt_engine.cuh"
 
 namespace bntt {
 
-constexpr int kBatchThreads = 256;
-// Largest HBM pass of a large transform (engine_split): a strided pass of
-// 2^m points has 256 >> (m - 3) adjacent columns per tile, and at least 8
-// (128 contiguous bytes per row) keep its loads coalesced.
-constexpr int kBatchMaxPass = 8;
+// 128 threads, 6 resident CTAs per SM (80 registers).  The rate of a tile does
+// not change between 24 and 32 resident warps, and six small CTAs overlap more
+// of each other's item fetches, loads and barriers than four of 256 threads:
+// uneven batch 818 us with 256 threads and 4 CTAs, 804 with 128 and 6 (841
+// with 5, whose 96 registers spill less).
+constexpr int kBatchThreads = 128;
+constexpr int kBatchCtas = 6;
 
-struct DevJob {
+struct alignas(16) DevJob {  // two 16-byte loads
   const uint4* x;
   uint4* y;
   const uint4* tw;
@@ -62,7 +62,7 @@ enum : uint32_t { ITEM_SMALL = 0, ITEM_PASS = 1 };
 struct WorkItem {
   uint16_t shape;   // index into the shape table below
   uint16_t kind;    // ITEM_SMALL or ITEM_PASS
-  uint32_t a;       // SMALL: first position in the size-sorted order; PASS: job index
+  uint32_t a;       // SMALL: first descriptor of the tile; PASS: the job's descriptor
   uint32_t b;       // SMALL: number of jobs in the tile; PASS: first sub-transform id
   uint16_t pass;    // PASS: pass index
   uint16_t wait;    // PASS: bit 0 the tile waits for the pass run before it,
@@ -70,12 +70,17 @@ struct WorkItem {
 };
 static_assert(sizeof(WorkItem) == 16, "work item layout");
 
-// Tile shapes of the persistent kernel (all 256 threads).  Sizes 2^1 and
-// 2^2 use unrolled one-thread tiles; every other size and both mappings run
-// on NttEngine<kBatchLogR> (4 elements per thread), whose code is shared by
-// all of them.  TPC = 256 / (threads per sub-transform).  Interleaved
+// Tile shapes of the persistent kernel: X(id, M, LOGR, TPC, map), TPC
+// sub-transforms per item, of which the CTA's threads hold kBatchThreads >>
+// (M - LOGR) at a time (4-element shapes take two turns).  Interleaved
 // (strided) tiles keep at least 8 adjacent columns (128 bytes of each row).
-constexpr int kBatchLogR = 2;
+// 8 elements per thread run three stages per exchange, with about a fifth
+// fewer index and exchange instructions, but twice the code: the strided
+// passes (two tile passes each) and 2^10 gain from it (64 x 2^16: 1076 ->
+// 1034 us), the contiguous tiles below do not, since the warps then wait for
+// instructions (with 8 elements throughout the uneven batch takes 822 us).
+// A tile engine with the size at run time (one body for all shapes) takes 84
+// instructions per butterfly instead of 66 and 909 us.
 #define BNTT_BATCH_SHAPES(X)               \
   X(0, 1, 1, 256, MAP_CONTIG)              \
   X(1, 2, 2, 256, MAP_CONTIG)              \
@@ -86,10 +91,10 @@ constexpr int kBatchLogR = 2;
   X(6, 7, 2, 8, MAP_CONTIG)                \
   X(7, 8, 2, 4, MAP_CONTIG)                \
   X(8, 9, 2, 2, MAP_CONTIG)                \
-  X(9, 10, 2, 1, MAP_CONTIG)               \
-  X(10, 5, 2, 32, MAP_INTERLEAVED)         \
-  X(11, 6, 2, 16, MAP_INTERLEAVED)         \
-  X(12, 7, 2, 8, MAP_INTERLEAVED)
+  X(9, 10, 3, 1, MAP_CONTIG)               \
+  X(10, 5, 3, 32, MAP_INTERLEAVED)         \
+  X(11, 6, 3, 16, MAP_INTERLEAVED)         \
+  X(12, 7, 3, 8, MAP_INTERLEAVED)
 
 struct BatchShape {
   int m, logr, tpc, map;
@@ -100,22 +105,6 @@ inline constexpr BatchShape kShapes[] = {
 #undef BNTT_SHAPE_ROW
 };
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
-
-// the same table for device code: size and mapping of a shape id
-__device__ __forceinline__ void shape_of(int id, int* m, int* map) {
-  switch (id) {
-#define BNTT_SHAPE_DEV(sid, M, LOGR, TPC, MAP) \
-  case sid:                                    \
-    *m = M;                                    \
-    *map = MAP;                                \
-    break;
-    BNTT_BATCH_SHAPES(BNTT_SHAPE_DEV)
-#undef BNTT_SHAPE_DEV
-    default:
-      *m = 3;
-      *map = MAP_CONTIG;
-  }
-}
 
 // control words: [0] queue head, [1] error word, [2 + 4*slot + p] pass counters
 constexpr int kCtlHeader = 2;
@@ -132,68 +121,70 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
 struct BatchArgs {
   const WorkItem* items;
   uint32_t nitems;
-  const DevJob* jobs;
-  const uint32_t* order;   // job indices sorted by size (SMALL tiles)
+  const DevJob* jobs;  // small jobs sorted by size, then the large jobs
   uint32_t* ctl;
   const uint32_t* pass_tiles;  // [slot * kMaxPasses + p] tile count of pass p
   uint32_t wait_polls;         // give up a dependency wait after this many polls
 };
 
+// A later-pass item waits until its job's earlier pass is complete; returns
+// false when the wait gave up (the error word is set; the tile is skipped).
+// INV: the passes of a large job run last to first (inverse transform), so a
+// pass waits for the pass after it and the last pass is the one that reads the
+// job's input.
+template <bool INV>
+__device__ __forceinline__ bool item_wait(const WorkItem& it, const BatchArgs& ba, int* s_flag) {
+  if (it.kind != ITEM_PASS || !(it.wait & 1)) return true;
+  const uint32_t slot = ba.jobs[it.a].slot;
+  uint32_t* counters = ba.ctl + kCtlHeader + slot * kMaxPasses;
+  const int pred = INV ? (int)it.pass + 1 : (int)it.pass - 1;
+  if (threadIdx.x == 0) {
+    const uint32_t want = ba.pass_tiles[slot * kMaxPasses + pred];
+    uint32_t polls = 0;
+    int ok = 1;
+    while (ld_acquire(&counters[pred]) < want) {
+      if (++polls > ba.wait_polls) {
+        atomicOr(&ba.ctl[1], 1u);
+        ok = 0;
+        break;
+      }
+      __nanosleep(100);
+    }
+    *s_flag = ok;
+  }
+  __syncthreads();
+  return *s_flag != 0;
+}
+
 // The sub-transform a work item hands to thread `sub` of the tile: a whole
-// small job, or one sub-transform of an HBM pass of a large job.  Returns
-// false when the item is a later pass whose wait for its predecessor gave up
-// (the error word is set; the tile is skipped).  INV: the passes of a large
-// job run last to first (inverse transform), so a pass waits for the pass
-// after it and the last pass is the one that reads the job's input.
-template <bool INV = false>
-__device__ __forceinline__ bool item_subref(const WorkItem& it, const BatchArgs& ba, int m, int sub,
-                                            int* s_flag, SubRef* out) {
-  if (it.kind == ITEM_SMALL) {
-    SubRef sr;
+// small job, or one sub-transform of an HBM pass of a large job (whose tiles
+// are always full: batch_split's passes are whole numbers of tiles).
+template <int M, int MAP>
+__device__ __forceinline__ SubRef item_subref(const WorkItem& it, const BatchArgs& ba, int sub) {
+  SubRef sr;
+  if (MAP == MAP_CONTIG && it.kind == ITEM_SMALL) {
     sr.valid = (uint32_t)sub < it.b;
-    const DevJob& j = ba.jobs[ba.order[it.a + (sr.valid ? (uint32_t)sub : 0u)]];
+    const DevJob& j = ba.jobs[it.a + (sr.valid ? (uint32_t)sub : 0u)];
     sr.x = j.x;
     sr.y = j.y;
     sr.tw = j.tw;
     sr.trow = 1;
     sr.lshift = 0;
-    *out = sr;
-    return true;
+    return sr;
   }
   const DevJob& j = ba.jobs[it.a];
-  const int n = (int)j.log2n;
-  const int s0 = it.wait >> 8;  // first stage of this pass (engine_split on the host)
-  if (it.wait & 1) {
-    uint32_t* counters = ba.ctl + kCtlHeader + j.slot * kMaxPasses;
-    const int pred = INV ? (int)it.pass + 1 : (int)it.pass - 1;
-    if (threadIdx.x == 0) {
-      const uint32_t want = ba.pass_tiles[j.slot * kMaxPasses + pred];
-      uint32_t polls = 0;
-      int ok = 1;
-      while (ld_acquire(&counters[pred]) < want) {
-        if (++polls > ba.wait_polls) {
-          atomicOr(&ba.ctl[1], 1u);
-          ok = 0;
-          break;
-        }
-        __nanosleep(100);
-      }
-      *s_flag = ok;
-    }
-    __syncthreads();
-    if (!*s_flag) return false;
-  }
-  SubGeom g;
-  g.x = (it.wait & 2) ? j.x : j.y;
-  g.y = j.y;
-  g.tw = j.tw;
-  g.n = (uint32_t)n;
-  g.s0 = (uint32_t)s0;
-  g.m = (uint32_t)m;
-  g.l = (uint32_t)(n - s0 - m);
-  g.nsub = 1ull << (n - m);
-  *out = make_subref(g, (uint64_t)it.b + (uint64_t)sub);
-  return true;
+  const uint32_t s0 = it.wait >> 8;  // first stage of this pass
+  const uint32_t l = MAP == MAP_CONTIG ? 0u : j.log2n - s0 - M;
+  const uint32_t sid = it.b + (uint32_t)sub;  // (H << L) | c
+  const uint32_t h = sid >> l;
+  const uint32_t off = (h << (l + M)) + (sid & ((1u << l) - 1u));
+  sr.valid = true;
+  sr.x = ((it.wait & 2) ? j.x : j.y) + off;
+  sr.y = j.y + off;
+  sr.tw = j.tw;
+  sr.trow = (1u << s0) + h;
+  sr.lshift = l;
+  return sr;
 }
 
 // A pass tile publishes its completion: every thread's stores, then one
@@ -208,88 +199,60 @@ __device__ __forceinline__ void item_publish(const WorkItem& it, const BatchArgs
   }
 }
 
-// The item functions are templates on the kernel's MINB as well: a
-// non-inlined function is compiled once for all its callers, at the smallest
-// register budget among them, so a kernel variant with more resident CTAs
-// would otherwise make every variant's items spill.
-
-// Sizes 2^1, 2^2: one thread per transform, fully unrolled.
-template <int M, class Arith, int MINB, int LY>
-__device__ __noinline__ void run_item_tiny(const WorkItem& it, const BatchArgs& ba, uint4* smem,
-                                           const ModParams& mp, int layout_arg, int* s_flag) {
+// One item on the compile-time tile of the plan kernels.  Inlined into the
+// kernel: as separate functions the items spilled around the call's fixed
+// registers (848 -> 826 us for the uneven batch).  L2-coherent loads: a later
+// pass reads what other CTAs wrote in this launch.
+template <int M, int LOGR, int TPC, int MAP, class Arith, int LY>
+__device__ __forceinline__ void run_item(const WorkItem& it, const BatchArgs& ba, uint4* smem,
+                                      const ModParams& mp, int layout_arg, int* s_flag) {
   const int layout = LY >= 0 ? LY : layout_arg;
-  using T = NttTile<M, M, kBatchThreads, MAP_CONTIG, Arith>;
-  const int sub = threadIdx.x;
-  SubRef sr;
-  if (!item_subref(it, ba, M, sub, s_flag, &sr)) return;
-  T::template run<LD_NC>(sr, sub, 0, smem, mp, layout);
+  constexpr int HELD = kBatchThreads >> (M - LOGR);  // sub-transforms the threads hold at a time
+  using T = NttTile<M, LOGR, HELD, MAP, Arith>;
+  static_assert(T::THREADS == kBatchThreads && TPC % HELD == 0, "tile shape");
+  if (!item_wait<false>(it, ba, s_flag)) return;
+#pragma unroll 1
+  for (int turn = 0; turn < TPC / HELD; ++turn) {
+    const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
+    const SubRef sr = item_subref<M, MAP>(it, ba, turn * HELD + sub);
+    if (turn > 0) T::sync();  // smem is reused
+    T::template run<LD_CG>(sr, sub, lane, smem, mp, layout);
+  }
   item_publish(it, ba);
 }
 
-// Every other shape: the runtime-size engine.
-template <class Arith, int MINB, int LY>
-__device__ __noinline__ void run_item_engine(const WorkItem& it, const BatchArgs& ba, uint4* smem,
-                                             const ModParams& mp, int layout_arg, int* s_flag) {
-  const int layout = LY >= 0 ? LY : layout_arg;
-  using E = NttEngine<kBatchLogR, Arith>;
-  int m, map;
-  shape_of(it.shape, &m, &map);
-  int sub, lane;
-  E::place(threadIdx.x, m, map, kBatchThreads, &sub, &lane);
-  SubRef sr;
-  if (!item_subref(it, ba, m, sub, s_flag, &sr)) return;
-  // One load policy for every item: L2-coherent loads (a later pass reads what
-  // other CTAs wrote in this launch).  A second instantiation for first
-  // passes would double the engine's code, and instruction fetch is one of
-  // the kernel's main stalls.
-  E::template run<LD_CG>(m, map, kBatchThreads, sr, sub, lane, smem, mp, layout);
-  item_publish(it, ba);
-}
-
-// Items of the shapes that carry most work run on the compile-time tile of the
-// plan kernels (NttTile: strides and pass widths are constants) instead of the
-// runtime-size engine: contiguous 2^7..2^10 (small jobs, the last passes of
-// 2^16 and 2^20 jobs) and the interleaved 2^6 passes of 2^16 and 2^20 jobs.
-// Measured on the uneven batch: 159 -> 168 G butterflies/s (2^10 items +6 %,
-// 2^9 +7 %, 2^8 +7 %, 2^20 jobs +9 %).  Specialising the smaller and the other
-// interleaved shapes as well made the kernel 5 % slower overall (a larger
-// kernel), so they stay on the engine.
-template <int M, int TPC, int MAP, class Arith, int MINB, int LY>
-__device__ __noinline__ void run_item_tile(const WorkItem& it, const BatchArgs& ba, uint4* smem,
-                                           const ModParams& mp, int layout_arg, int* s_flag) {
-  const int layout = LY >= 0 ? LY : layout_arg;
-  using T = NttTile<M, kBatchLogR, TPC, MAP, Arith>;
-  static_assert(T::THREADS == kBatchThreads, "tile shape");
-  const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
-  SubRef sr;
-  if (!item_subref(it, ba, M, sub, s_flag, &sr)) return;
-  T::template run<LD_CG>(sr, sub, lane, smem, mp, layout);
-  item_publish(it, ba);
-}
-
-// MINB: resident CTAs per SM requested from the compiler (register budget).
 // LY: the element layout as a constant (LAYOUT_HILO or LAYOUT_U128), or -1
 // for the `layout` argument.  A constant layout removes the runtime word
 // select of every HBM load and store (measured +0.9 % on the uneven batch).
-template <class Arith, int MINB, int LY = -1>
-__global__ void __launch_bounds__(kBatchThreads, MINB) k_batch(BatchArgs ba, ModParams mp, int layout) {
+template <class Arith, int LY, int CTAS>
+__global__ void __launch_bounds__(kBatchThreads, CTAS) k_batch(BatchArgs ba, ModParams mp, int layout) {
   extern __shared__ uint4 smem[];
   __shared__ uint32_t s_item;
   __shared__ int s_flag;
+  // Thread 0 holds one item more than the CTA runs, so the counter's round
+  // trip overlaps the current item.  A held item waits at most for the
+  // current one, whose waits are for items earlier in the queue: the earliest
+  // unfinished item is always running and has nothing to wait for.
+  uint32_t next = 0;
+  if (threadIdx.x == 0) next = atomicAdd(&ba.ctl[0], 1u);
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(&ba.ctl[0], 1u);
+    if (threadIdx.x == 0) {
+      s_item = next;
+      next = atomicAdd(&ba.ctl[0], 1u);
+    }
     __syncthreads();
     const uint32_t i = s_item;
     if (i >= ba.nitems) break;
     const WorkItem it = ba.items[i];
-    if (it.shape == 0) run_item_tiny<1, Arith, MINB, LY>(it, ba, smem, mp, layout, &s_flag);
-    else if (it.shape == 1) run_item_tiny<2, Arith, MINB, LY>(it, ba, smem, mp, layout, &s_flag);
-    else if (it.shape == 9) run_item_tile<10, 1, MAP_CONTIG, Arith, MINB, LY>(it, ba, smem, mp, layout, &s_flag);
-    else if (it.shape == 8) run_item_tile<9, 2, MAP_CONTIG, Arith, MINB, LY>(it, ba, smem, mp, layout, &s_flag);
-    else if (it.shape == 7) run_item_tile<8, 4, MAP_CONTIG, Arith, MINB, LY>(it, ba, smem, mp, layout, &s_flag);
-    else if (it.shape == 6) run_item_tile<7, 8, MAP_CONTIG, Arith, MINB, LY>(it, ba, smem, mp, layout, &s_flag);
-    else if (it.shape == 11) run_item_tile<6, 16, MAP_INTERLEAVED, Arith, MINB, LY>(it, ba, smem, mp, layout, &s_flag);
-    else run_item_engine<Arith, MINB, LY>(it, ba, smem, mp, layout, &s_flag);
+    switch (it.shape) {
+#define BNTT_RUN_SHAPE(id, M, LOGR, TPC, MAP)                                   \
+  case id:                                                                      \
+    run_item<M, LOGR, TPC, MAP, Arith, LY>(it, ba, smem, mp, layout, &s_flag);  \
+    break;
+      BNTT_BATCH_SHAPES(BNTT_RUN_SHAPE)
+#undef BNTT_RUN_SHAPE
+      default: break;
+    }
     __syncthreads();  // smem and s_item are reused by the next item
   }
 }

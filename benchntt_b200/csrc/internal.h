@@ -83,9 +83,6 @@ int tuned_batch_small_shape(int m);
 // Pass decomposition of a 2^n transform: sizes of HBM passes (each <= max_m).
 // Plans use max_m = 10; the persistent kernel uses kBatchMaxPass.
 std::vector<int> split_passes(int n, int max_m = 10);
-// HBM passes of a 2^n transform (n > 10) on the tile engine (batch kernel,
-// engine plans): fewest passes of <= 8 stages, then fewest engine passes.
-std::vector<int> engine_split(int n);
 // HBM passes of a 2^n transform (11 <= n <= 24) on 4-element tiles, as the
 // persistent kernel splits its large jobs: strided passes of 5..7 stages
 // (2^(10 - m) adjacent columns per tile), then a contiguous pass of up to 10;
@@ -133,10 +130,9 @@ struct bntt_plan {
   int layout = 0;
   void* tw = nullptr;
   bool own_tw = false;
-  // inverse transform: table of inverse twiddles (limb order) and N^-1 mod q,
+  // inverse transform: table of inverse twiddles (limb order; entry 0 is N^-1),
   // built on the first inverse call
   void* tw_inv = nullptr;
-  bntt::U128 ninv{};
   // kernel per HBM pass
   std::vector<int> passes;
   std::vector<const bntt::SubKernel*> kernels;
@@ -155,8 +151,4 @@ int plan_create_common(bntt_ctx* c, bntt_plan** out, unsigned log2n, const bntt_
 // b != nullptr fuses y = y * b into the last pass (MulB in ntt_core.cuh).
 int ntt_forward_on(bntt_plan* plan, void* y, const void* x, size_t batch, cudaStream_t s,
                    const void* b = nullptr, uint64_t bmask = 0);
-// The same on the runtime-size tile engine (fast multiply, log2n >= 3);
-// ntt_forward_on uses it above 2^10 points.
-int engine_forward_on(bntt_plan* plan, void* y, const void* x, size_t batch, cudaStream_t s,
-                      const void* b, uint64_t bmask);
 }  // namespace bntt

@@ -63,17 +63,6 @@ struct MulB {
   uint64_t bmask = 0;
 };
 
-// What the last store of an engine kernel applies (ntt_engine.cuh): an
-// optional scalar multiply (the inverse transform's N^-1, held here or read
-// at the store from device memory), then an optional pointwise product
-// (MulB).
-struct Epilogue {
-  U128 scale{};
-  int has_scale = 0;
-  const uint4* scale_at = nullptr;  // EPI_SCALE_AT: the scalar, limb order
-  MulB mul;
-};
-
 // Where a tile's first pass finds its inputs and every pass its twiddles.
 //   SRC_STAGED  the inputs were copied into the tile's shared-memory slots
 //               beforehand (cp.async, k_ntt_sub_staged); the first pass
@@ -97,6 +86,12 @@ __device__ __forceinline__ uint4 lds128(const uint4* p) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
   return v;
+}
+
+// Table entry i (i < 2^24): the byte offset fits 32 bits, so the address is
+// one shift and one 64-bit add.
+__device__ __forceinline__ const uint4* tw_at(const uint4* tw, uint32_t i) {
+  return reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(tw) + (i << 4));
 }
 
 template <int M, int LOGR, int TPC, int MAP, class Arith>
@@ -129,8 +124,7 @@ struct NttTile {
     if constexpr (MAP == MAP_INTERLEAVED) {
       return j * TPC + sub;
     } else {
-      const int sw = (M >= 3) ? (j ^ ((j >> 3) & 7)) : j;
-      return (sub << M) | sw;
+      return swz((sub << M) | j);
     }
   }
 
@@ -139,16 +133,23 @@ struct NttTile {
     else __syncthreads();
   }
 
+  // Contiguous tiles: linear index L of the tile -> slot.  The 8 lanes of one
+  // quarter of a 16-byte access vary three bits of L, which ones depends on
+  // the pass (bits lo.. of the group number skip the pass's own bits); adding
+  // 3, 6 and 4 to the slot's low three bits for L's bits 3, 4 and 5 makes them
+  // hit eight different banks for passes of 2 or 3 stages at every lo (with
+  // L ^ ((L >> 3) & 7) the two-stage pass at lo = 2 hit four).
+  __host__ __device__ static constexpr int swz(int l) {
+    return M >= 3 ? l ^ (((l >> 3) ^ ((l >> 2) & 6)) & 7) : l;
+  }
   // slot(sub, base | c) from sb = slot(sub, base) when base and c share no
-  // bit and c is a constant (c = j << lo in a pass): the swizzle
-  // x ^ ((x >> 3) & 7) is linear over XOR, so a contiguous tile's slot is
-  // sb ^ swizzle(c); without swizzle, and for interleaved tiles, the parts
-  // add.  One operation per element, with the constant folded.
-  __host__ __device__ static constexpr int swz(int c) { return (M >= 3) ? (c ^ ((c >> 3) & 7)) : c; }
+  // bit and c is a constant (c = j << lo in a pass): the swizzle is linear
+  // over XOR, so a contiguous tile's slot is sb ^ swz(c), with c above the
+  // swizzled bits sb + c; for interleaved tiles the parts add.  One operation
+  // per element at most, with the constant folded.
   __device__ __forceinline__ static int slot_at(int sb, int c) {
     if constexpr (MAP == MAP_INTERLEAVED) return sb + c * TPC;
-    else if constexpr (M >= 3) return sb ^ swz(c);
-    else return sb + c;
+    else return swz(c) == c && (c & 63) == 0 ? sb + c : sb ^ swz(c);
   }
 
   // Lowest local bit pass p touches.
@@ -207,7 +208,8 @@ struct NttTile {
     static_assert(GPT >= 1, "pass wider than the register tile");
     static_assert(r <= kLazyStages, "pass wider than the partly reduced range");
     // element j of a group in HBM: the group's first element plus j * gstep
-    const size_t gstep = (size_t)1 << (lo + sr.lshift);
+    const uint32_t lshift = MAP == MAP_CONTIG ? 0u : sr.lshift;  // L, 0 for contiguous tiles
+    const size_t gstep = (size_t)1 << (lo + lshift);
     const uint32_t k = mp.k;
 
     // element j of the group at local index base, slot sb
@@ -216,7 +218,7 @@ struct NttTile {
         return from_mem(smem[slot_at(sb, j << lo)], layout);  // staged in memory order
       } else if constexpr (P == 0) {
         if (!sr.valid) return U128{{0u, 0u, 0u, 0u}};
-        return from_mem(ld_data<LDP>(sr.x + ((size_t)base << sr.lshift) + (size_t)j * gstep), layout);
+        return from_mem(ld_data<LDP>(sr.x + ((size_t)base << lshift) + (size_t)j * gstep), layout);
       } else {
         const uint4 t = smem[slot_at(sb, j << lo)];
         return U128{{t.x, t.y, t.z, t.w}};
@@ -246,7 +248,7 @@ struct NttTile {
       const uint32_t gt = gt_of(i);
       lazy_stages<r>(v, i * G, [&](int t, int u) {
         // tables are stored in limb order (LAYOUT_U128) by the plan
-        const uint4* twt = sr.tw + (gt << t);  // u as an immediate offset
+        const uint4* twt = tw_at(sr.tw, gt << t);  // u as an immediate offset
         const uint4 tv = (SRC & TW_SHARED) != 0 ? lds128(twt + u) : __ldg(twt + u);
         return U128{{tv.x, tv.y, tv.z, tv.w}};
       }, k, rerun);
@@ -282,7 +284,7 @@ struct NttTile {
       for (int j = 0; j < G; ++j) {
         if constexpr (last) {
           if (sr.valid) {
-            uint4* yp = sr.y + ((size_t)base << sr.lshift) + (size_t)j * gstep;
+            uint4* yp = sr.y + ((size_t)base << lshift) + (size_t)j * gstep;
             U128 o = v[i * G + j];
             if (mb.b) {
               const uint4 bv = __ldg(mb.b + ((uint64_t)(yp - mb.ybase) & mb.bmask));
@@ -415,7 +417,8 @@ struct NttTile {
     constexpr int G = 1 << r;
     constexpr int GPT = R / G;
     static_assert(GPT >= 1 && r <= 4, "pass shape");
-    const size_t gstep = (size_t)1 << (lo + sr.lshift);  // HBM distance of j and j + 1
+    const uint32_t lshift = MAP == MAP_CONTIG ? 0u : sr.lshift;
+    const size_t gstep = (size_t)1 << (lo + lshift);  // HBM distance of j and j + 1
 
     // ---- gather: the inverse reads its input in the last pass's order
 #pragma unroll
@@ -427,7 +430,7 @@ struct NttTile {
       for (int j = 0; j < G; ++j) {
         if constexpr (P == NPASS - 1) {
           if (sr.valid) {
-            v[i * G + j] = from_mem(ld_data<LDP>(sr.x + ((size_t)base << sr.lshift) + (size_t)j * gstep), layout);
+            v[i * G + j] = from_mem(ld_data<LDP>(sr.x + ((size_t)base << lshift) + (size_t)j * gstep), layout);
           } else {
 #pragma unroll
             for (int w = 0; w < 4; ++w) v[i * G + j].w[w] = 0u;
@@ -445,7 +448,7 @@ struct NttTile {
       const int g = lane + i * TPT;
       const uint32_t gt = (sr.trow << s0) + (uint32_t)(g >> lo);
       inverse_stages<r, P == 0>(v, i * G, [&](int t, int u) {
-        const uint4 tv = __ldg(sr.tw + (gt << t) + u);
+        const uint4 tv = __ldg(tw_at(sr.tw, gt << t) + u);
         return U128{{tv.x, tv.y, tv.z, tv.w}};
       }, mp.k);
     }
@@ -478,7 +481,7 @@ struct NttTile {
 #pragma unroll
       for (int j = 0; j < G; ++j) {
         if constexpr (P == 0) {
-          if (sr.valid) sr.y[((size_t)base << sr.lshift) + (size_t)j * gstep] = to_mem(v[i * G + j], layout);
+          if (sr.valid) sr.y[((size_t)base << lshift) + (size_t)j * gstep] = to_mem(v[i * G + j], layout);
         } else {
           const U128& e = v[i * G + j];
           smem[slot_at(sb, j << lo)] = make_uint4(e.w[0], e.w[1], e.w[2], e.w[3]);
@@ -520,6 +523,21 @@ __device__ __forceinline__ SubRef make_subref(const SubGeom& g, uint64_t sid) {
   r.tw = g.tw;
   r.trow = (1u << g.s0) + (uint32_t)hbits;
   r.lshift = g.l;
+  return r;
+}
+
+// The same for contiguous sub-transforms (L = 0): sub-transform sid is the
+// 2^M elements from sid << M on.
+template <int M>
+__device__ __forceinline__ SubRef make_subref_contig(const SubGeom& g, uint64_t sid) {
+  SubRef r;
+  r.valid = sid < g.nsub;
+  const uint64_t s = r.valid ? sid : 0;
+  r.x = g.x + (s << M);
+  r.y = g.y + (s << M);
+  r.tw = g.tw;
+  r.trow = (1u << g.s0) + ((uint32_t)s & ((1u << g.s0) - 1u));
+  r.lshift = 0;
   return r;
 }
 

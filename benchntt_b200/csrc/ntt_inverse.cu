@@ -1,5 +1,4 @@
-// ntt_engine_plan.cu -- plan transforms on the runtime-size tile engine:
-// the inverse transform, and the forward transform above 2^10 points.
+// ntt_inverse.cu -- the inverse transform of a plan.
 //
 // The reference has no inverse transform.  The forward network
 // (src/ntt_scalar.c:582-627, in its in-place form: stage s pairs indices
@@ -17,96 +16,43 @@
 // pseudo-Mersenne multiply is required (q = 2^124 - k, k < 2^28).
 //
 // Kernels: the compile-time tile in inverse mode (k_ntt_tile_inv), one
-// launch for N = 2^3..2^10 and above that one launch per HBM pass of the
+// launch for N up to 2^10 and above that one launch per HBM pass of the
 // persistent kernel's split (tile_split), in reverse pass order (the pass
-// over the low index bits first); a one-thread-per-transform kernel for N = 2
-// and 4.  The runtime-size tile engine (ntt_engine.cuh) in inverse mode
-// remains for splits without a tile kernel, and in forward mode for the
-// forward transforms above 2^10 points (engine_forward_on) likewise: passes
-// of at most 8 stages keep the strided passes coalesced.
-#include <algorithm>
-#include <atomic>
+// over the low index bits first).
 #include <vector>
 
 #include "internal.h"
 #include "ntt_core.cuh"
-#include "ntt_engine.cuh"
 
 namespace bntt {
 namespace {
 
-// Tiles of 256 threads; the HBM passes of a large transform come from
-// engine_split (at most 8 stages each, so a strided tile covers at least 8
-// adjacent columns: 128 contiguous bytes per row).
-constexpr int kEngThreads = 256;
-
-using PlanEngine = NttEngine<3, ArithFast>;
-
-// One HBM pass of a plan transform on the tile engine: tiles of 256 threads,
-// persistent over the pass's tiles.  INV selects the inverse network; `ep`
-// is applied by the last store when use_ep is set.
-template <bool INV>
-__global__ void __launch_bounds__(kEngThreads, 3)
-    k_ntt_engine(SubGeom g, ModParams mp, int layout, int m, int map, Epilogue ep, int use_ep) {
-  extern __shared__ uint4 smem[];
-  int sub, lane;
-  PlanEngine::place(threadIdx.x, m, map, kEngThreads, &sub, &lane);
-  const int tpc = kEngThreads >> (m - 3);
-  const uint64_t ntiles = (g.nsub + (uint64_t)tpc - 1) / (uint64_t)tpc;
-  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const SubRef sr = make_subref(g, tile * (uint64_t)tpc + (uint64_t)sub);
-    PlanEngine::run<LD_CG, INV, INV ? EPI_SCALE : EPI_MUL>(m, map, kEngThreads, sr, sub, lane, smem, mp, layout,
-                                      use_ep ? &ep : nullptr);
-    __syncthreads();  // shared memory is reused by the next tile
-  }
-}
-
-// N = 2 or 4: one thread per transform, stages in reverse order, then N^-1.
-__global__ void __launch_bounds__(256)
-    k_ntt_inv_tiny(uint4* x, const uint4* y, const uint4* tw, uint64_t count, int n, ModParams mp,
-                   int layout, U128 scale) {
-  const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  const int N = 1 << n;
-  U128 v[4];
-  for (int i = 0; i < N; ++i) v[i] = from_mem(__ldcg(y + t * N + i), layout);
-  for (int s = n - 1; s >= 0; --s) {
-    const int half = N >> (s + 1);
-    for (int i = 0; i < N; ++i) {
-      if (i & half) continue;
-      const uint4 tv = __ldg(tw + (1 << s) + (i >> (n - s)));
-      gs_butterfly<ArithFast>(v[i], v[i + half], U128{{tv.x, tv.y, tv.z, tv.w}}, mp);
-    }
-  }
-  // the second half already carries N^-1 through table entry 1
-  for (int i = 0; i < N; ++i) x[t * N + i] = to_mem(i < N / 2 ? ArithFast::mul(v[i], scale, mp) : v[i], layout);
-}
-
 // One HBM pass of the inverse on the compile-time tile (NttTile::run_inv, 4
 // elements per thread, 256-thread CTAs of 256 / 2^(M-2) sub-transforms, 4
 // resident per SM), one CTA per tile like the forward k_ntt_sub:
-// whole transforms of 2^3..2^10 points (contiguous), or one pass of a larger
+// whole transforms of up to 2^10 points (contiguous), or one pass of a larger
 // transform (interleaved for the strided passes).  `finishing` marks the
 // pass that ends the transform (stage 0 inside it), which applies N^-1 from
 // entry 0 of the inverse table.
 template <int M, int MAP>
 __global__ void __launch_bounds__(256, 4)
     k_ntt_tile_inv(SubGeom g, ModParams mp, int layout, int finishing) {
-  constexpr int TPC = 256 >> (M - 2);
-  using T = NttTile<M, 2, TPC, MAP, ArithFast>;
+  constexpr int LOGR = M < 2 ? M : 2, TPC = 256 >> (M - LOGR);
+  using T = NttTile<M, LOGR, TPC, MAP, ArithFast>;
   static_assert(T::THREADS == 256, "tile shape");
   extern __shared__ uint4 smem[];
   const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
   const uint4* scale_at = finishing ? g.tw : nullptr;
-  const SubRef sr = make_subref(g, (uint64_t)blockIdx.x * TPC + (uint64_t)sub);
+  const uint64_t sid = (uint64_t)blockIdx.x * TPC + (uint64_t)sub;
+  const SubRef sr = MAP == MAP_CONTIG ? make_subref_contig<M>(g, sid) : make_subref(g, sid);
   if (layout == LAYOUT_HILO) T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_HILO, scale_at);
   else T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
 }
 
 template <int M, int MAP>
 int launch_tile_inv(bntt_plan* p, const SubGeom& g, int finishing, cudaStream_t s) {
-  constexpr int TPC = 256 >> (M - 2);
-  using T = NttTile<M, 2, TPC, MAP, ArithFast>;
+  constexpr int LOGR = M < 2 ? M : 2, TPC = 256 >> (M - LOGR);
+  using T = NttTile<M, LOGR, TPC, MAP, ArithFast>;
   constexpr size_t smem = (size_t)T::SMEM_SLOTS * 16;
   const uint64_t ntiles = (g.nsub + TPC - 1) / TPC;
   BNTT_REQUIRE(ntiles <= 0x7fffffffu, "%llu tiles are more than one launch takes", (unsigned long long)ntiles);
@@ -116,7 +62,7 @@ int launch_tile_inv(bntt_plan* p, const SubGeom& g, int finishing, cudaStream_t 
   return BNTT_OK;
 }
 
-// One pass of m stages (a whole transform of 2^3..2^10 points, a strided
+// One pass of m stages (a whole transform of up to 2^10 points, a strided
 // pass of 5..7 or a contiguous last pass of a larger one); EINVAL for a shape
 // without a tile kernel.
 int tile_inv_pass(bntt_plan* p, const SubGeom& g, int finishing, cudaStream_t s) {
@@ -129,6 +75,8 @@ int tile_inv_pass(bntt_plan* p, const SubGeom& g, int finishing, cudaStream_t s)
     }
   } else {
     switch (g.m) {
+      case 1: return launch_tile_inv<1, MAP_CONTIG>(p, g, finishing, s);
+      case 2: return launch_tile_inv<2, MAP_CONTIG>(p, g, finishing, s);
       case 3: return launch_tile_inv<3, MAP_CONTIG>(p, g, finishing, s);
       case 4: return launch_tile_inv<4, MAP_CONTIG>(p, g, finishing, s);
       case 5: return launch_tile_inv<5, MAP_CONTIG>(p, g, finishing, s);
@@ -141,58 +89,6 @@ int tile_inv_pass(bntt_plan* p, const SubGeom& g, int finishing, cudaStream_t s)
     }
   }
   return set_error(BNTT_EINVAL, "no inverse tile for a pass of %u stages", g.m);
-}
-
-template <bool INV>
-int engine_blocks_per_sm(size_t smem) {
-  static std::atomic<int> cached[2];  // per smem class; relaxed: same value from any thread
-  const int slot = smem > 0 ? 1 : 0;
-  if (const int c = cached[slot].load(std::memory_order_relaxed)) return c;
-  int b = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &b, (const void*)k_ntt_engine<INV>, kEngThreads, smem);
-  if (e != cudaSuccess) return -cuda_error(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-  cached[slot].store(std::max(1, b), std::memory_order_relaxed);
-  return std::max(1, b);
-}
-
-// The HBM passes of a 2^n transform (n >= 3) on the engine: forward in pass
-// order, inverse in reverse order.  The first pass run reads `in`, every
-// pass writes `out` (in place after the first), and the last pass run
-// applies `ep` when use_ep is set.
-template <bool INV>
-int engine_passes(bntt_plan* p, void* out, const void* in, size_t batch, const void* tw,
-                  const Epilogue& ep, int use_ep, cudaStream_t s) {
-  const int n = (int)p->log2n;
-  const std::vector<int> passes = n <= 10 ? std::vector<int>{n} : engine_split(n);
-  const int np = (int)passes.size();
-  std::vector<int> starts(np, 0);
-  for (int i = 1; i < np; ++i) starts[i] = starts[i - 1] + passes[i - 1];
-  for (int k = 0; k < np; ++k) {
-    const int i = INV ? np - 1 - k : k;
-    const int m = passes[i];
-    SubGeom g;
-    g.x = static_cast<const uint4*>(k == 0 ? in : out);
-    g.y = static_cast<uint4*>(out);
-    g.tw = static_cast<const uint4*>(tw);
-    g.n = (uint32_t)n;
-    g.s0 = (uint32_t)starts[i];
-    g.m = (uint32_t)m;
-    g.l = (uint32_t)(n - starts[i] - m);
-    g.nsub = (uint64_t)batch << (n - m);
-    const int map = g.l > 0 ? MAP_INTERLEAVED : MAP_CONTIG;
-    const size_t smem = PlanEngine::smem_slots(m, map, kEngThreads) * 16;
-    const int bps = engine_blocks_per_sm<INV>(smem);
-    if (bps < 0) return -bps;
-    const int tpc = kEngThreads >> (m - 3);
-    const uint64_t ntiles = (g.nsub + (uint64_t)tpc - 1) / (uint64_t)tpc;
-    const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)bps * p->ctx->sms);
-    k_ntt_engine<INV><<<grid, kEngThreads, smem, s>>>(g, p->mp, p->layout, m, map, ep,
-                                                      (k == np - 1 && use_ep) ? 1 : 0);
-    BNTT_CK(cudaGetLastError());
-    p->ctx->launches++;
-  }
-  return BNTT_OK;
 }
 
 // Inverse table (T[k]^-1, limb order) and N^-1, built once per plan: the
@@ -256,48 +152,32 @@ int ensure_inverse(bntt_plan* p) {
     return cuda_error(e, "copy of the inverse twiddles");
   }
   p->tw_inv = d;
-  p->ninv = to_limbs(ninv);
   return BNTT_OK;
 }
 
 int inverse_on(bntt_plan* p, void* x, const void* y, size_t batch, cudaStream_t s) {
   const int n = (int)p->log2n;
-  if (n <= 2) {
-    const unsigned grid = (unsigned)((batch + 255) / 256);
-    k_ntt_inv_tiny<<<grid, 256, 0, s>>>(static_cast<uint4*>(x), static_cast<const uint4*>(y),
-                                        static_cast<const uint4*>(p->tw_inv), (uint64_t)batch, n,
-                                        p->mp, p->layout, p->ninv);
-    BNTT_CK(cudaGetLastError());
-    p->ctx->launches++;
-    return BNTT_OK;
-  }
   // up to 2^10 points one tile pass; above, the persistent kernel's split
   // (strided passes of 5..7 stages, then a contiguous one), run last pass
   // first, the first run reading y and every run writing x
   const std::vector<int> split = n <= 10 ? std::vector<int>{n} : tile_split(n);
-  if (!split.empty()) {
-    const int np = (int)split.size();
-    std::vector<int> starts(np, 0);
-    for (int i = 1; i < np; ++i) starts[i] = starts[i - 1] + split[i - 1];
-    for (int k = 0; k < np; ++k) {
-      const int i = np - 1 - k;
-      SubGeom g;
-      g.x = static_cast<const uint4*>(k == 0 ? y : x);
-      g.y = static_cast<uint4*>(x);
-      g.tw = static_cast<const uint4*>(p->tw_inv);
-      g.n = (uint32_t)n;
-      g.s0 = (uint32_t)starts[i];
-      g.m = (uint32_t)split[i];
-      g.l = (uint32_t)(n - starts[i] - split[i]);
-      g.nsub = (uint64_t)batch << (n - split[i]);
-      if (int rc = tile_inv_pass(p, g, i == 0 ? 1 : 0, s)) return rc;
-    }
-    return BNTT_OK;
+  const int np = (int)split.size();
+  std::vector<int> starts(np, 0);
+  for (int i = 1; i < np; ++i) starts[i] = starts[i - 1] + split[i - 1];
+  for (int k = 0; k < np; ++k) {
+    const int i = np - 1 - k;
+    SubGeom g;
+    g.x = static_cast<const uint4*>(k == 0 ? y : x);
+    g.y = static_cast<uint4*>(x);
+    g.tw = static_cast<const uint4*>(p->tw_inv);
+    g.n = (uint32_t)n;
+    g.s0 = (uint32_t)starts[i];
+    g.m = (uint32_t)split[i];
+    g.l = (uint32_t)(n - starts[i] - split[i]);
+    g.nsub = (uint64_t)batch << (n - split[i]);
+    if (int rc = tile_inv_pass(p, g, i == 0 ? 1 : 0, s)) return rc;
   }
-  Epilogue ep;
-  ep.scale = p->ninv;
-  ep.has_scale = 1;
-  return engine_passes<true>(p, x, y, batch, p->tw_inv, ep, 1, s);
+  return BNTT_OK;
 }
 
 }  // namespace
@@ -305,17 +185,6 @@ int inverse_on(bntt_plan* p, void* x, const void* y, size_t batch, cudaStream_t 
 int plan_ensure_inverse(bntt_plan* p) {
   if (!p->fast) return set_error(BNTT_EINVAL, "the inverse transform needs q = 2^124 - k (k < 2^28), mu = floor(2^251/q)");
   return ensure_inverse(p);
-}
-
-// Forward transform of a plan on the engine (fast multiply, n >= 3), with
-// the optional fused pointwise product of MulB on the last pass.
-int engine_forward_on(bntt_plan* p, void* y, const void* x, size_t batch, cudaStream_t s,
-                      const void* b, uint64_t bmask) {
-  Epilogue ep;
-  ep.mul.b = static_cast<const uint4*>(b);
-  ep.mul.ybase = static_cast<const uint4*>(y);
-  ep.mul.bmask = bmask;
-  return engine_passes<false>(p, y, x, batch, p->tw, ep, b ? 1 : 0, s);
 }
 
 }  // namespace bntt

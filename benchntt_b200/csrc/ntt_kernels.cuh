@@ -23,7 +23,8 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, Arith>::THREADS, MI
   extern __shared__ uint4 smem[];
   const int tid = threadIdx.x;
   const int sub = T::sub_of(tid), lane = T::lane_of(tid);
-  const SubRef sr = make_subref(g, (uint64_t)blockIdx.x * TPC + (uint64_t)sub);
+  const uint64_t sid = (uint64_t)blockIdx.x * TPC + (uint64_t)sub;
+  const SubRef sr = MAP == MAP_CONTIG ? make_subref_contig<M>(g, sid) : make_subref(g, sid);
   // the element layout as a constant in each branch: no word select per
   // HBM load and store
   if (layout == LAYOUT_HILO) T::template run<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_HILO, MulB{g.b, g.y, g.bmask});
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP_CONTIG, Arith>::THRE
     cp_async_commit();
     cp_async_wait<1>();  // every group but the newest: this tile's copies
     __syncthreads();
-    SubRef sr = make_subref(g, tile * TPC + (uint64_t)sub);
+    SubRef sr = make_subref_contig<M>(g, tile * TPC + (uint64_t)sub);
     sr.tw = tw;
     if (layout == LAYOUT_HILO)
       T::template run<LD_NC, SRC | SRC_STAGED>(sr, sub, lane, smem + b * TILE, mp, LAYOUT_HILO,

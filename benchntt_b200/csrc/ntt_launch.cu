@@ -1,7 +1,6 @@
 // ntt_launch.cu -- registry of compiled sub-transform kernels, the HBM pass
 // split, and the stream-ordered forward transform.
 #include <algorithm>
-#include <functional>
 #include <mutex>
 
 #include "internal.h"
@@ -94,47 +93,6 @@ std::vector<int> split_passes(int n, int max_m) {
   return p;
 }
 
-// Split of a 2^n transform (n > 10) for the tile engine: the fewest HBM
-// passes of at most 8 stages, and among those the split with the fewest
-// engine passes (each engine pass covers at most 3 stages, so a pass of 6
-// stages costs 2 and one of 7 costs 3), then the widest first pass.  For
-// 2^20 that is 8 + 6 + 6 (7 engine passes) instead of 7 + 7 + 6 (8).
-std::vector<int> engine_split(int n) {
-  const int k = (n + 7) / 8;
-  std::vector<int> best, cur(k, 0);
-  int best_cost = 1 << 30;
-  // enumerate compositions of n into k parts in [1, 8], first part largest first
-  std::vector<int> stack;
-  std::function<void(int, int)> rec = [&](int i, int left) {
-    if (i == k - 1) {
-      if (left < 1 || left > 8) return;
-      cur[i] = left;
-      int cost = 0, s0 = 0;
-      for (int j = 0; j < k; ++j) {
-        const int m = cur[j], l = n - s0 - m;
-        if (m < 3) return;  // the engine needs >= 2^3 points
-        // a strided pass: at least 2^5 points (the interleaved tile shapes),
-        // and its 256 >> (m - 3) columns per tile must exist (<= 2^l)
-        if (l > 0 && (m < 5 || 11 - m > l)) return;
-        cost += (m + 2) / 3;
-        s0 += m;
-      }
-      if (cost < best_cost) {
-        best_cost = cost;
-        best = cur;
-      }
-      return;
-    }
-    for (int m = 8; m >= 1; --m) {
-      if (left - m < (k - 1 - i) || left - m > 8 * (k - 1 - i)) continue;
-      cur[i] = m;
-      rec(i + 1, left - m);
-    }
-  };
-  rec(0, n);
-  return best;
-}
-
 int plan_choose_kernels(bntt_plan* p) {
   const int n = (int)p->log2n;
   p->passes = split_passes(n);
@@ -179,11 +137,9 @@ int ntt_forward_on(bntt_plan* plan, void* y, const void* x, size_t batch, cudaSt
   if (batch == 0) return BNTT_OK;
   const int n = (int)plan->log2n;
   // above 2^10 points: the persistent kernel's split on 4-element tiles
-  // (strided passes of 5..7 stages over 2^(10-m) adjacent columns, 256 B or
-  // more per row, then a contiguous pass), else the runtime-size engine with
-  // passes of at most 8 stages.  Measured at 2^16: 0.83 against 0.73 of the
-  // IMAD roofline for the engine; compiled tiles with 10-stage passes, whose
-  // strided passes touch 2 or 4 columns per row, were 1.5x slower than that.
+  // (strided passes of 5..7 stages over 2^(10-m) adjacent columns, 128 B or
+  // more per row, then a contiguous pass).  Compiled tiles with 10-stage
+  // passes, whose strided passes touch 2 or 4 columns per row, were 2x slower.
   if (n > 10 && arith_fast(plan->ctx, plan->fast)) {
     const std::vector<int> split = tile_split(n);
     std::vector<const SubKernel*> ks;
@@ -199,7 +155,7 @@ int ntt_forward_on(bntt_plan* plan, void* y, const void* x, size_t batch, cudaSt
       ks.push_back(found);
       s0 += m;
     }
-    if (split.empty() || ks.size() != split.size()) return engine_forward_on(plan, y, x, batch, s, b, bmask);
+    if (split.empty() || ks.size() != split.size()) return set_error(BNTT_EINVAL, "no tile kernels for 2^%d points", n);
     s0 = 0;
     for (size_t i = 0; i < split.size(); ++i) {
       const int m = split[i];

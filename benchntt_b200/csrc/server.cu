@@ -164,11 +164,9 @@ static int launch_slot(bntt_server* s, Slot& slot) {
     Schedule& sc = slot.sched;
     if (int rc = build_schedule(s->engine, sc, jobs.data(), jobs.size())) return rc;
     const size_t cb = (kCtlHeader + sc.nslots * kMaxPasses) * 4, pb = sc.pass_tiles.size() * 4,
-                 ib = sc.items.size() * sizeof(WorkItem), ob = sc.order.size() * 4,
-                 jb = sc.djobs.size() * sizeof(DevJob);
+                 ib = sc.items.size() * sizeof(WorkItem), jb = sc.djobs.size() * sizeof(DevJob);
     auto r256 = [](size_t v) { return (v + 255) & ~(size_t)255; };
-    const size_t o_pt = r256(cb), o_it = r256(o_pt + pb), o_or = r256(o_it + ib),
-                 o_jb = r256(o_or + ob), need = r256(o_jb + jb);
+    const size_t o_pt = r256(cb), o_it = r256(o_pt + pb), o_jb = r256(o_it + ib), need = r256(o_jb + jb);
     if (slot.pinned_cap < need || slot.dev_cap < need) {  // not reached within kLaunchBytes
       void *h = nullptr, *d = nullptr;
       BNTT_CK(cudaMallocHost(&h, need * 2));
@@ -186,7 +184,6 @@ static int launch_slot(bntt_server* s, Slot& slot) {
     memset(h, 0, cb);  // control words start at zero
     memcpy(h + o_pt, sc.pass_tiles.data(), pb);
     memcpy(h + o_it, sc.items.data(), ib);
-    memcpy(h + o_or, sc.order.data(), ob);
     memcpy(h + o_jb, sc.djobs.data(), jb);
     char* d = static_cast<char*>(slot.dev);
     BNTT_CK(cudaMemcpyAsync(d, h, need, cudaMemcpyHostToDevice, slot.stream));
@@ -200,7 +197,6 @@ static int launch_slot(bntt_server* s, Slot& slot) {
     ba.items = reinterpret_cast<const WorkItem*>(d + o_it);
     ba.nitems = (uint32_t)sc.items.size();
     ba.jobs = reinterpret_cast<const DevJob*>(d + o_jb);
-    ba.order = reinterpret_cast<const uint32_t*>(d + o_or);
     ba.ctl = reinterpret_cast<uint32_t*>(d);
     ba.pass_tiles = reinterpret_cast<const uint32_t*>(d + o_pt);
     ba.wait_polls = kWaitPolls;
