@@ -355,39 +355,276 @@ __device__ __forceinline__ U128 from_w(W128 a) {
 // product of the quotient estimate likewise (:151-171), the low product keeps
 // its cross terms to 64 bits (:130-149), and one conditional subtraction ends
 // it (:194-196).
+inline __device__ __noinline__ U128 mulmod_words(const U128 ua, const U128 ub, const U128 uq, const U128 umu) {
+  const W128 a = to_w(ua), b = to_w(ub), q = to_w(uq), mu = to_w(umu);
+  // product
+  W128 p00 = w_mul64(a.lo, b.lo), p01 = w_mul64(a.lo, b.hi);
+  W128 p10 = w_mul64(a.hi, b.lo), p11 = w_mul64(a.hi, b.hi);
+  W128 mid = w_add(w_add(p01, p10), W128{0, p00.hi});
+  W128 ph = w_add(p11, W128{0, mid.hi});
+  W128 pl = W128{mid.lo, p00.lo};
+  // quotient estimate from bits 122.. of the product
+  // t = (P >> 122) mod 2^128 = (ph << 6) | (pl >> 122)
+  W128 t = W128{(ph.hi << 6) | (ph.lo >> 58), (ph.lo << 6) | (pl.hi >> 58)};
+  uint64_t top = ph.hi >> 58;
+  W128 m01 = w_mul64(t.lo, mu.hi), m10 = w_mul64(t.hi, mu.lo), m11 = w_mul64(t.hi, mu.hi);
+  W128 mm = w_add(w_add(m01, m10), W128{0, __umul64hi(t.lo, mu.lo)});
+  W128 qm = w_add(w_add(m11, W128{0, mm.hi}), W128{0, top * mu.lo});
+  W128 qq = W128{qm.hi >> 1, (qm.lo >> 1) | (qm.hi << 63)};
+  // low product qq*q
+  W128 l00 = w_mul64(qq.lo, q.lo);
+  uint64_t cross = qq.lo * q.hi + qq.hi * q.lo + l00.hi;
+  W128 qql = W128{cross, l00.lo};
+  // r = pl - qql mod 2^128
+  W128 r;
+  r.lo = pl.lo - qql.lo;
+  r.hi = pl.hi - qql.hi - (pl.lo < qql.lo ? 1ull : 0ull);
+  const bool lt = (r.hi < q.hi) || (r.hi == q.hi && r.lo < q.lo);
+  if (!lt) {
+    uint64_t lo2 = r.lo - q.lo;
+    r.hi = r.hi - q.hi - (r.lo < q.lo ? 1ull : 0ull);
+    r.lo = lo2;
+  }
+  return from_w(r);
+}
+
+// The two columns of a 128 x 128-bit product (see mul_lazy): E at limbs 0..7
+// in e, O at limbs 1..7 in o[1..7], P = E + O*2^32 with the carries out of the
+// columns already in.
+__device__ __forceinline__ void mul_columns(const U128& a, const U128& b, uint32_t (&e)[8], uint32_t (&o)[8]) {
+  asm("mul.lo.u32 %0, %4, %5;\n\t"
+      "mul.hi.u32 %1, %4, %5;\n\t"
+      "mul.lo.u32 %2, %4, %6;\n\t"
+      "mul.hi.u32 %3, %4, %6;\n\t"
+      : "=&r"(e[0]), "=&r"(e[1]), "=&r"(e[2]), "=&r"(e[3])
+      : "r"(a.w[0]), "r"(b.w[0]), "r"(b.w[2]));
+  asm("mul.lo.u32 %0, %4, %5;\n\t"
+      "mul.hi.u32 %1, %4, %5;\n\t"
+      "mul.lo.u32 %2, %4, %6;\n\t"
+      "mul.hi.u32 %3, %4, %6;\n\t"
+      : "=&r"(o[1]), "=&r"(o[2]), "=&r"(o[3]), "=&r"(o[4])
+      : "r"(a.w[0]), "r"(b.w[1]), "r"(b.w[3]));
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;\n\t"
+      : "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "=r"(o[5])
+      : "r"(a.w[1]), "r"(b.w[0]), "r"(b.w[2]));
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, 0;\n\t"
+      "madc.hi.u32    %3, %4, %6, 0;\n\t"
+      : "+r"(e[2]), "+r"(e[3]), "=&r"(e[4]), "=&r"(e[5])
+      : "r"(a.w[1]), "r"(b.w[1]), "r"(b.w[3]));
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;\n\t"
+      : "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "=r"(e[6])
+      : "r"(a.w[2]), "r"(b.w[0]), "r"(b.w[2]));
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, %2;\n\t"
+      "madc.hi.u32    %3, %4, %6, 0;\n\t"
+      : "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "=&r"(o[6])
+      : "r"(a.w[2]), "r"(b.w[1]), "r"(b.w[3]));
+  asm("mad.lo.cc.u32  %0, %5, %6, %0;\n\t"
+      "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
+      "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
+      "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
+      "addc.u32       %4, 0, 0;\n\t"
+      : "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "=r"(o[7])
+      : "r"(a.w[3]), "r"(b.w[0]), "r"(b.w[2]));
+  asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+      "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+      "madc.lo.cc.u32 %2, %4, %6, %2;\n\t"
+      "madc.hi.u32    %3, %4, %6, 0;\n\t"
+      : "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "=&r"(e[7])
+      : "r"(a.w[3]), "r"(b.w[1]), "r"(b.w[3]));
+}
+
+// mulmod_words on 32-bit limbs with the carries inside the multiply-adds, for
+// operands below 2^127 (their middle sum cannot leave 128 bits; larger ones
+// take mulmod_words).  38 wide products and about 70 other instructions,
+// where the 64-bit words' products (each a low and a high product of their
+// own) cost about twice that.  The quotient estimate's middle sum M is kept
+// to 128 bits as in the reference: the carry out of its top limb is dropped.
 struct ArithRef {
   static constexpr bool kFast = false;
-  __device__ __forceinline__ static U128 mul(const U128& ua, const U128& ub, const ModParams& m) {
-    const W128 a = to_w(ua), b = to_w(ub), q = to_w(m.q), mu = to_w(m.mu);
-    // product
-    W128 p00 = w_mul64(a.lo, b.lo), p01 = w_mul64(a.lo, b.hi);
-    W128 p10 = w_mul64(a.hi, b.lo), p11 = w_mul64(a.hi, b.hi);
-    W128 mid = w_add(w_add(p01, p10), W128{0, p00.hi});
-    W128 ph = w_add(p11, W128{0, mid.hi});
-    W128 pl = W128{mid.lo, p00.lo};
-    // quotient estimate from bits 122.. of the product
-    // t = (P >> 122) mod 2^128 = (ph << 6) | (pl >> 122)
-    W128 t = W128{(ph.hi << 6) | (ph.lo >> 58), (ph.lo << 6) | (pl.hi >> 58)};
-    uint64_t top = ph.hi >> 58;
-    W128 m01 = w_mul64(t.lo, mu.hi), m10 = w_mul64(t.hi, mu.lo), m11 = w_mul64(t.hi, mu.hi);
-    W128 mm = w_add(w_add(m01, m10), W128{0, __umul64hi(t.lo, mu.lo)});
-    W128 qm = w_add(w_add(m11, W128{0, mm.hi}), W128{0, top * mu.lo});
-    W128 qq = W128{qm.hi >> 1, (qm.lo >> 1) | (qm.hi << 63)};
-    // low product qq*q
-    W128 l00 = w_mul64(qq.lo, q.lo);
-    uint64_t cross = qq.lo * q.hi + qq.hi * q.lo + l00.hi;
-    W128 qql = W128{cross, l00.lo};
-    // r = pl - qql mod 2^128
-    W128 r;
-    r.lo = pl.lo - qql.lo;
-    r.hi = pl.hi - qql.hi - (pl.lo < qql.lo ? 1ull : 0ull);
-    const bool lt = (r.hi < q.hi) || (r.hi == q.hi && r.lo < q.lo);
-    if (!lt) {
-      uint64_t lo2 = r.lo - q.lo;
-      r.hi = r.hi - q.hi - (r.lo < q.lo ? 1ull : 0ull);
-      r.lo = lo2;
+  __device__ __forceinline__ static U128 mul(const U128& a, const U128& b, const ModParams& m) {
+    if (__builtin_expect((a.w[3] | b.w[3]) >> 31, 0)) return mulmod_words(a, b, m.q, m.mu);
+    uint32_t p[8];  // the product
+    {
+      uint32_t e[8], o[8];
+      mul_columns(a, b, e, o);
+      p[0] = e[0];
+      asm("add.cc.u32  %0, %7, %14;\n\t"
+          "addc.cc.u32 %1, %8, %15;\n\t"
+          "addc.cc.u32 %2, %9, %16;\n\t"
+          "addc.cc.u32 %3, %10, %17;\n\t"
+          "addc.cc.u32 %4, %11, %18;\n\t"
+          "addc.cc.u32 %5, %12, %19;\n\t"
+          "addc.u32    %6, %13, %20;\n\t"
+          : "=&r"(p[1]), "=&r"(p[2]), "=&r"(p[3]), "=&r"(p[4]), "=&r"(p[5]), "=&r"(p[6]), "=&r"(p[7])
+          : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(o[1]), "r"(o[2]),
+            "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]));
     }
-    return from_w(r);
+    // t = (P >> 122) mod 2^128; the 6 bits above it
+    uint32_t t[4], top = p[7] >> 26;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = __funnelshift_r(p[3 + i], p[4 + i], 26);
+    const uint32_t* u = m.mu.w;
+    // limbs 2 and 3 of t_lo * mu_lo
+    uint32_t c1, c2, c3;
+    {
+      uint32_t e1, e2, e3, o1, o2, o3;
+      asm("mul.hi.u32 %0, %1, %2;\n\t" : "=r"(e1) : "r"(t[0]), "r"(u[0]));
+      asm("mul.lo.u32 %0, %4, %6;\n\t"
+          "mul.hi.u32 %1, %4, %6;\n\t"
+          "mul.lo.u32 %2, %5, %6;\n\t"
+          "mul.hi.u32 %3, %5, %6;\n\t"
+          : "=&r"(o1), "=&r"(o2), "=&r"(e2), "=&r"(e3)
+          : "r"(t[0]), "r"(t[1]), "r"(u[1]));
+      asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+          "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+          "addc.u32       %2, 0, 0;\n\t"
+          : "+r"(o1), "+r"(o2), "=r"(o3)
+          : "r"(t[1]), "r"(u[0]));
+      asm("add.cc.u32  %0, %3, %6;\n\t"
+          "addc.cc.u32 %1, %4, %7;\n\t"
+          "addc.u32    %2, %5, %8;\n\t"
+          : "=&r"(c1), "=&r"(c2), "=&r"(c3)
+          : "r"(e1), "r"(e2), "r"(e3), "r"(o1), "r"(o2), "r"(o3));
+    }
+    // M = that + t_lo * mu_hi + t_hi * mu_lo at limbs 2..5, columns E (2, 4)
+    // and O (3, 5); carries out of limb 5 are dropped
+    uint32_t e4, e5, o3, o4, o5;
+    asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+        "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+        "madc.lo.cc.u32 %2, %6, %7, 0;\n\t"
+        "madc.hi.u32    %3, %6, %7, 0;\n\t"
+        : "+r"(c2), "+r"(c3), "=&r"(e4), "=&r"(e5)
+        : "r"(t[0]), "r"(u[2]), "r"(t[1]), "r"(u[3]));
+    asm("mad.lo.cc.u32  %0, %4, %5, %0;\n\t"
+        "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
+        "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
+        "madc.hi.u32    %3, %6, %7, %3;\n\t"
+        : "+r"(c2), "+r"(c3), "+r"(e4), "+r"(e5)
+        : "r"(t[2]), "r"(u[0]), "r"(t[3]), "r"(u[1]));
+    asm("mul.lo.u32 %0, %2, %3;\n\t"
+        "mul.hi.u32 %1, %2, %3;\n\t"
+        : "=&r"(o3), "=&r"(o4)
+        : "r"(t[0]), "r"(u[3]));
+    asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32       %2, 0, 0;\n\t"
+        : "+r"(o3), "+r"(o4), "=r"(o5)
+        : "r"(t[1]), "r"(u[2]));
+    asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32       %2, %2, 0;\n\t"
+        : "+r"(o3), "+r"(o4), "+r"(o5)
+        : "r"(t[2]), "r"(u[1]));
+    asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32       %2, %2, 0;\n\t"
+        : "+r"(o3), "+r"(o4), "+r"(o5)
+        : "r"(t[3]), "r"(u[0]));
+    uint32_t m4, m5;
+    asm("{\n\t.reg .u32 lim3;\n\t"
+        "add.cc.u32  lim3, %2, %5;\n\t"
+        "addc.cc.u32 %0, %3, %6;\n\t"
+        "addc.u32    %1, %4, %7;\n\t}"
+        : "=&r"(m4), "=&r"(m5)
+        : "r"(c3), "r"(e4), "r"(e5), "r"(o3), "r"(o4), "r"(o5));
+    // Q = t_hi * mu_hi + M's high word + top * mu_lo, at limbs 4..7
+    uint32_t q4, q5, q6, q7, r5, r6, r7;
+    asm("mad.lo.cc.u32  %0, %4, %5, %8;\n\t"
+        "madc.hi.cc.u32 %1, %4, %5, %9;\n\t"
+        "madc.lo.cc.u32 %2, %6, %7, 0;\n\t"
+        "madc.hi.u32    %3, %6, %7, 0;\n\t"
+        : "=&r"(q4), "=&r"(q5), "=&r"(q6), "=&r"(q7)
+        : "r"(t[2]), "r"(u[2]), "r"(t[3]), "r"(u[3]), "r"(m4), "r"(m5));
+    asm("mul.lo.u32 %0, %2, %3;\n\t"
+        "mul.hi.u32 %1, %2, %3;\n\t"
+        : "=&r"(r5), "=&r"(r6)
+        : "r"(t[2]), "r"(u[3]));
+    asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32       %2, 0, 0;\n\t"
+        : "+r"(r5), "+r"(r6), "=r"(r7)
+        : "r"(t[3]), "r"(u[2]));
+    asm("add.cc.u32  %0, %0, %3;\n\t"
+        "addc.cc.u32 %1, %1, %4;\n\t"
+        "addc.u32    %2, %2, %5;\n\t"
+        : "+r"(q5), "+r"(q6), "+r"(q7)
+        : "r"(r5), "r"(r6), "r"(r7));
+    if (__builtin_expect(top != 0u, 0)) {  // P >= 2^250
+      const uint64_t x = (uint64_t)top * (((uint64_t)u[1] << 32) | u[0]);
+      asm("add.cc.u32  %0, %0, %4;\n\t"
+          "addc.cc.u32 %1, %1, %5;\n\t"
+          "addc.cc.u32 %2, %2, 0;\n\t"
+          "addc.u32    %3, %3, 0;\n\t"
+          : "+r"(q4), "+r"(q5), "+r"(q6), "+r"(q7)
+          : "r"((uint32_t)x), "r"((uint32_t)(x >> 32)));
+    }
+    // (Q >> 1) * q mod 2^128
+    const uint32_t h0 = __funnelshift_r(q4, q5, 1), h1 = __funnelshift_r(q5, q6, 1),
+                   h2 = __funnelshift_r(q6, q7, 1), h3 = q7 >> 1;
+    const uint32_t* q = m.q.w;
+    uint32_t l0, l1, l2, l3, s1, s2, s3;
+    asm("mul.lo.u32 %0, %4, %6;\n\t"
+        "mul.hi.u32 %1, %4, %6;\n\t"
+        "mul.lo.u32 %2, %5, %7;\n\t"
+        "mul.hi.u32 %3, %5, %7;\n\t"
+        : "=&r"(l0), "=&r"(l1), "=&r"(l2), "=&r"(l3)
+        : "r"(h0), "r"(h1), "r"(q[0]), "r"(q[1]));
+    asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\t"
+        "madc.hi.u32   %1, %2, %3, %1;\n\t"
+        : "+r"(l2), "+r"(l3)
+        : "r"(h0), "r"(q[2]));
+    asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\t"
+        "madc.hi.u32   %1, %2, %3, %1;\n\t"
+        : "+r"(l2), "+r"(l3)
+        : "r"(h2), "r"(q[0]));
+    asm("mul.lo.u32 %0, %2, %3;\n\t"
+        "mul.hi.u32 %1, %2, %3;\n\t"
+        : "=&r"(s1), "=&r"(s2)
+        : "r"(h0), "r"(q[1]));
+    asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32       %2, 0, 0;\n\t"
+        : "+r"(s1), "+r"(s2), "=r"(s3)
+        : "r"(h1), "r"(q[0]));
+    s3 += h0 * q[3] + h1 * q[2] + h2 * q[1] + h3 * q[0];
+    asm("add.cc.u32  %0, %0, %3;\n\t"
+        "addc.cc.u32 %1, %1, %4;\n\t"
+        "addc.u32    %2, %2, %5;\n\t"
+        : "+r"(l1), "+r"(l2), "+r"(l3)
+        : "r"(s1), "r"(s2), "r"(s3));
+    // r = P - that mod 2^128, less q unless r < q
+    U128 r;
+    uint32_t d0, d1, d2, d3, lt;
+    asm("sub.cc.u32  %0, %4, %8;\n\t"
+        "subc.cc.u32 %1, %5, %9;\n\t"
+        "subc.cc.u32 %2, %6, %10;\n\t"
+        "subc.u32    %3, %7, %11;\n\t"
+        : "=&r"(r.w[0]), "=&r"(r.w[1]), "=&r"(r.w[2]), "=&r"(r.w[3])
+        : "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]), "r"(l0), "r"(l1), "r"(l2), "r"(l3));
+    asm("sub.cc.u32  %0, %5, %9;\n\t"
+        "subc.cc.u32 %1, %6, %10;\n\t"
+        "subc.cc.u32 %2, %7, %11;\n\t"
+        "subc.cc.u32 %3, %8, %12;\n\t"
+        "subc.u32    %4, 0, 0;\n\t"
+        : "=&r"(d0), "=&r"(d1), "=&r"(d2), "=&r"(d3), "=r"(lt)
+        : "r"(r.w[0]), "r"(r.w[1]), "r"(r.w[2]), "r"(r.w[3]), "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3]));
+    r.w[0] = lt ? r.w[0] : d0;
+    r.w[1] = lt ? r.w[1] : d1;
+    r.w[2] = lt ? r.w[2] : d2;
+    r.w[3] = lt ? r.w[3] : d3;
+    return r;
   }
 };
 
