@@ -224,8 +224,8 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const BatchArgs& ba
 // LY: the element layout as a constant (LAYOUT_HILO or LAYOUT_U128), or -1
 // for the `layout` argument.  A constant layout removes the runtime word
 // select of every HBM load and store (measured +0.9 % on the uneven batch).
-template <class Arith, int LY, int CTAS>
-__global__ void __launch_bounds__(kBatchThreads, CTAS) k_batch(BatchArgs ba, ModParams mp, int layout) {
+template <class Arith, int LY>
+__global__ void __launch_bounds__(kBatchThreads, kBatchCtas) k_batch(BatchArgs ba, ModParams mp, int layout) {
   extern __shared__ uint4 smem[];
   __shared__ uint32_t s_item;
   __shared__ int s_flag;

@@ -4,7 +4,7 @@
 
 namespace bntt {
 const void* batch_kernel_fast(int layout) {
-  return layout == LAYOUT_HILO ? (const void*)&k_batch<ArithFast, LAYOUT_HILO, kBatchCtas>
-                               : (const void*)&k_batch<ArithFast, LAYOUT_U128, kBatchCtas>;
+  return layout == LAYOUT_HILO ? (const void*)&k_batch<ArithFast, LAYOUT_HILO>
+                               : (const void*)&k_batch<ArithFast, LAYOUT_U128>;
 }
 }  // namespace bntt

@@ -66,27 +66,37 @@ struct SubKernel {
   int max_blocks_per_sm;  // filled lazily
   int minb;               // __launch_bounds__ minimum resident CTAs
   int src = 0;            // SRC_STAGED / TW_SHARED (k_ntt_sub_staged), else 0
+  int use = 0;            // USE_* below: where it is the default
 };
 
+// Launches a shape is the default of: none (an autotuner candidate), those of
+// fewer than kManyElems elements, the others, or both.
+enum : int { USE_TUNED = 0, USE_FEW = 1, USE_MANY = 2, USE_ALL = 3 };
+// A launch below 2^21 elements does not fill the SMs' thread slots several
+// times over: 4 elements per thread in small CTAs spread it over more warps
+// (37 x 2^13 points: 8.3 -> 6.2 us for the pass).  Above, 8 elements per
+// thread save index and exchange instructions (65,536 x 2^10: 3 %; a strided
+// pass of 6 stages 7 %).  Both are equal within 3 % from 2^20 to 2^22.
+constexpr uint64_t kManyElems = 1ull << 21;
+
 const std::vector<SubKernel>& sub_kernels();
-// Default shape for (m, map, fast); nullptr if none compiled.
-const SubKernel* pick_sub_kernel(int m, int map, int fast, int logr_pref = 0, int tpc_pref = 0);
-// Launch over a geometry; returns BNTT status.
+// Default shape of a pass of m stages over `elems` elements; nullptr if none
+// is compiled.
+const SubKernel* default_sub_kernel(int m, int map, int fast, uint64_t elems);
+// Launch over a geometry; returns BNTT status.  finishing: the inverse kernels'
+// last argument.
 int launch_sub(bntt_ctx* ctx, const SubKernel* k, const void* geom, const ModParams& mp,
-               int layout, cudaStream_t stream);
+               int layout, cudaStream_t stream, int finishing = 0);
 int blocks_per_sm(const SubKernel* k);
 
 // Autotuner choices (nullptr / -1 when not tuned).
 const SubKernel* tuned_sub_kernel(int m, int map, int fast, int l);
 int tuned_batch_small_shape(int m);
 
-// Pass decomposition of a 2^n transform: sizes of HBM passes (each <= max_m).
-// Plans use max_m = 10; the persistent kernel uses kBatchMaxPass.
-std::vector<int> split_passes(int n, int max_m = 10);
-// HBM passes of a 2^n transform (11 <= n <= 24) on 4-element tiles, as the
-// persistent kernel splits its large jobs: strided passes of 5..7 stages
-// (2^(10 - m) adjacent columns per tile), then a contiguous pass of up to 10;
-// the fewest passes, then the fewest tile passes.  Empty outside that range.
+// HBM passes of a 2^n transform (11 <= n <= 24), as the persistent kernel
+// splits its large jobs: strided passes of 5..7 stages (2^(10 - m) adjacent
+// columns per tile), then a contiguous pass of up to 10; the fewest passes,
+// then the fewest tile passes.  Empty outside that range.
 std::vector<int> tile_split(int n);
 
 int launch_blas(bntt_ctx* ctx, int op, void* c, const void* a, const void* b, U128 x, size_t len,
@@ -133,9 +143,9 @@ struct bntt_plan {
   // inverse transform: table of inverse twiddles (limb order; entry 0 is N^-1),
   // built on the first inverse call
   void* tw_inv = nullptr;
-  // kernel per HBM pass
-  std::vector<int> passes;
-  std::vector<const bntt::SubKernel*> kernels;
+  std::vector<int> passes;                   // stages of each HBM pass
+  bool created_fast = false;                 // arithmetic chosen when the plan was created
+  const bntt::SubKernel* tuned = nullptr;    // one pass: the autotuner's shape, if it ran
 };
 
 namespace bntt {

@@ -1,9 +1,7 @@
 // Instantiations: ArithFast, contiguous shapes with 4 (or 8) elements per
 // thread, so a transform spreads over more threads (an N = 16 transform on 4
 // threads instead of 1, an N = 1024 transform on 256 instead of 128):
-// autotuner candidates and the untuned defaults for 2^3..2^10.  At 2^9 and
-// 2^10 they also cut the latency of a lone transform (one CTA: fewer
-// dependent butterflies per thread).
+// autotuner candidates.
 #include "ntt_kernels.cuh"
 
 namespace bntt {

@@ -21,25 +21,21 @@
 // over the low index bits first).
 #include <vector>
 
-#include "internal.h"
-#include "ntt_core.cuh"
+#include "ntt_kernels.cuh"
 
 namespace bntt {
 namespace {
 
-// One HBM pass of the inverse on the compile-time tile (NttTile::run_inv, 4
-// elements per thread, 256-thread CTAs of 256 / 2^(M-2) sub-transforms, 4
-// resident per SM), one CTA per tile like the forward k_ntt_sub:
+// One HBM pass of the inverse on the compile-time tile (NttTile::run_inv), one
+// CTA per tile, in the shapes of the forward transform (BNTT_PLAN_SHAPES):
 // whole transforms of up to 2^10 points (contiguous), or one pass of a larger
 // transform (interleaved for the strided passes).  `finishing` marks the
 // pass that ends the transform (stage 0 inside it), which applies N^-1 from
 // entry 0 of the inverse table.
-template <int M, int MAP>
-__global__ void __launch_bounds__(256, 4)
+template <int M, int LOGR, int TPC, int MAP, int MINB>
+__global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, ArithFast>::THREADS, MINB)
     k_ntt_tile_inv(SubGeom g, ModParams mp, int layout, int finishing) {
-  constexpr int LOGR = M < 2 ? M : 2, TPC = 256 >> (M - LOGR);
   using T = NttTile<M, LOGR, TPC, MAP, ArithFast>;
-  static_assert(T::THREADS == 256, "tile shape");
   extern __shared__ uint4 smem[];
   const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
   const uint4* scale_at = finishing ? g.tw : nullptr;
@@ -49,46 +45,17 @@ __global__ void __launch_bounds__(256, 4)
   else T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
 }
 
-template <int M, int MAP>
-int launch_tile_inv(bntt_plan* p, const SubGeom& g, int finishing, cudaStream_t s) {
-  constexpr int LOGR = M < 2 ? M : 2, TPC = 256 >> (M - LOGR);
-  using T = NttTile<M, LOGR, TPC, MAP, ArithFast>;
-  constexpr size_t smem = (size_t)T::SMEM_SLOTS * 16;
-  const uint64_t ntiles = (g.nsub + TPC - 1) / TPC;
-  BNTT_REQUIRE(ntiles <= 0x7fffffffu, "%llu tiles are more than one launch takes", (unsigned long long)ntiles);
-  k_ntt_tile_inv<M, MAP><<<(unsigned)ntiles, 256, smem, s>>>(g, p->mp, p->layout, finishing);
-  BNTT_CK(cudaGetLastError());
-  p->ctx->launches++;
-  return BNTT_OK;
-}
-
-// One pass of m stages (a whole transform of up to 2^10 points, a strided
-// pass of 5..7 or a contiguous last pass of a larger one); EINVAL for a shape
-// without a tile kernel.
-int tile_inv_pass(bntt_plan* p, const SubGeom& g, int finishing, cudaStream_t s) {
-  if (g.l > 0) {
-    switch (g.m) {
-      case 5: return launch_tile_inv<5, MAP_INTERLEAVED>(p, g, finishing, s);
-      case 6: return launch_tile_inv<6, MAP_INTERLEAVED>(p, g, finishing, s);
-      case 7: return launch_tile_inv<7, MAP_INTERLEAVED>(p, g, finishing, s);
-      default: break;
-    }
-  } else {
-    switch (g.m) {
-      case 1: return launch_tile_inv<1, MAP_CONTIG>(p, g, finishing, s);
-      case 2: return launch_tile_inv<2, MAP_CONTIG>(p, g, finishing, s);
-      case 3: return launch_tile_inv<3, MAP_CONTIG>(p, g, finishing, s);
-      case 4: return launch_tile_inv<4, MAP_CONTIG>(p, g, finishing, s);
-      case 5: return launch_tile_inv<5, MAP_CONTIG>(p, g, finishing, s);
-      case 6: return launch_tile_inv<6, MAP_CONTIG>(p, g, finishing, s);
-      case 7: return launch_tile_inv<7, MAP_CONTIG>(p, g, finishing, s);
-      case 8: return launch_tile_inv<8, MAP_CONTIG>(p, g, finishing, s);
-      case 9: return launch_tile_inv<9, MAP_CONTIG>(p, g, finishing, s);
-      case 10: return launch_tile_inv<10, MAP_CONTIG>(p, g, finishing, s);
-      default: break;
-    }
-  }
-  return set_error(BNTT_EINVAL, "no inverse tile for a pass of %u stages", g.m);
+// The shape for a pass of m stages over `elems` elements.
+const SubKernel* inverse_kernel(int m, int map, uint64_t elems) {
+  static const SubKernel kernels[] = {
+#define BNTT_ADD(M, LOGR, TPC, MAP, MINB, USE) \
+  BNTT_SUBK_FN(M, LOGR, TPC, MAP, ArithFast, MINB, (k_ntt_tile_inv<M, LOGR, TPC, MAP, MINB>), USE),
+      BNTT_PLAN_SHAPES(BNTT_ADD)
+#undef BNTT_ADD
+  };
+  for (const SubKernel& k : kernels)
+    if (k.m == m && k.map == map && (k.use & (elems >= kManyElems ? USE_MANY : USE_FEW))) return &k;
+  return nullptr;
 }
 
 // Inverse table (T[k]^-1, limb order) and N^-1, built once per plan: the
@@ -175,7 +142,9 @@ int inverse_on(bntt_plan* p, void* x, const void* y, size_t batch, cudaStream_t 
     g.m = (uint32_t)split[i];
     g.l = (uint32_t)(n - starts[i] - split[i]);
     g.nsub = (uint64_t)batch << (n - split[i]);
-    if (int rc = tile_inv_pass(p, g, i == 0 ? 1 : 0, s)) return rc;
+    const SubKernel* kern = inverse_kernel(split[i], g.l > 0 ? MAP_INTERLEAVED : MAP_CONTIG, (uint64_t)batch << n);
+    if (!kern) return set_error(BNTT_EINVAL, "no inverse tile for a pass of %d stages", split[i]);
+    if (int rc = launch_sub(p->ctx, kern, &g, p->mp, p->layout, s, i == 0 ? 1 : 0)) return rc;
   }
   return BNTT_OK;
 }

@@ -95,12 +95,44 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP_CONTIG, Arith>::THRE
 
 }  // namespace bntt
 
-#define BNTT_SUBK_B(M, LOGR, TPC, MAP, ARITH, MINB)                                       \
+// Default shapes of the plan transforms with the fast multiply, forward and
+// inverse: X(M, LOGR, TPC, map, resident CTAs per SM, use).  CTAs of 64 or 128
+// threads: with one CTA per tile, smaller ones keep an SM's warps in more
+// different phases (2^24 elements of 2^8: 256 threads 250 us, 64 threads 234).
+// Interleaved tiles keep at least 8 columns (128 bytes of a row).
+#define BNTT_PLAN_SHAPES(X)                      \
+  X(1, 1, 256, MAP_CONTIG, 4, USE_ALL)           \
+  X(2, 2, 256, MAP_CONTIG, 4, USE_ALL)           \
+  X(3, 2, 32, MAP_CONTIG, 16, USE_ALL)           \
+  X(4, 2, 16, MAP_CONTIG, 16, USE_ALL)           \
+  X(5, 2, 8, MAP_CONTIG, 16, USE_FEW)            \
+  X(5, 3, 16, MAP_CONTIG, 12, USE_MANY)          \
+  X(6, 2, 4, MAP_CONTIG, 16, USE_FEW)            \
+  X(6, 3, 8, MAP_CONTIG, 12, USE_MANY)           \
+  X(7, 2, 2, MAP_CONTIG, 16, USE_FEW)            \
+  X(7, 3, 4, MAP_CONTIG, 12, USE_MANY)           \
+  X(8, 2, 1, MAP_CONTIG, 16, USE_ALL)            \
+  X(9, 2, 1, MAP_CONTIG, 8, USE_FEW)             \
+  X(9, 3, 1, MAP_CONTIG, 10, USE_MANY)           \
+  X(10, 2, 1, MAP_CONTIG, 4, USE_FEW)            \
+  X(10, 3, 1, MAP_CONTIG, 6, USE_MANY)           \
+  X(5, 2, 16, MAP_INTERLEAVED, 8, USE_FEW)       \
+  X(5, 3, 32, MAP_INTERLEAVED, 6, USE_MANY)      \
+  X(6, 2, 8, MAP_INTERLEAVED, 8, USE_FEW)        \
+  X(6, 3, 16, MAP_INTERLEAVED, 6, USE_MANY)      \
+  X(7, 2, 8, MAP_INTERLEAVED, 4, USE_FEW)        \
+  X(7, 3, 8, MAP_INTERLEAVED, 6, USE_MANY)
+
+#define BNTT_SUBK_FN(M, LOGR, TPC, MAP, ARITH, MINB, FN, USE)                             \
   ::bntt::SubKernel {                                                                     \
     M, LOGR, TPC, MAP, ARITH::kFast ? 1 : 0, ::bntt::NttTile<M, LOGR, TPC, MAP, ARITH>::THREADS, \
         (size_t)::bntt::NttTile<M, LOGR, TPC, MAP, ARITH>::SMEM_SLOTS * 16u,              \
-        (const void*)&::bntt::k_ntt_sub<M, LOGR, TPC, MAP, ARITH, MINB>, 0, MINB          \
+        (const void*)&FN, 0, MINB, 0, USE                                                 \
   }
+#define BNTT_SUBK_U(M, LOGR, TPC, MAP, ARITH, MINB, USE) \
+  BNTT_SUBK_FN(M, LOGR, TPC, MAP, ARITH, MINB, (::bntt::k_ntt_sub<M, LOGR, TPC, MAP, ARITH, MINB>), USE)
+#define BNTT_SUBK_B(M, LOGR, TPC, MAP, ARITH, MINB) \
+  BNTT_SUBK_U(M, LOGR, TPC, MAP, ARITH, MINB, ::bntt::USE_TUNED)
 #define BNTT_SUBK(M, LOGR, TPC, MAP, ARITH) BNTT_SUBK_B(M, LOGR, TPC, MAP, ARITH, 1)
 // staged contiguous kernels: two tile buffers (+ the table with TW_SHARED)
 #define BNTT_SUBK_STAGED(M, LOGR, TPC, ARITH, MINB, SRC)                                       \
