@@ -10,6 +10,7 @@
 #include <atomic>
 
 #include "internal.h"
+#include "ntt_core.cuh"
 
 namespace bntt {
 
@@ -19,6 +20,7 @@ template <int OP, class Arith, int U>
 __global__ void __launch_bounds__(256) k_blas(uint4* c, const uint4* a, const uint4* b, size_t n,
                                               ModParams mp, U128 x, int layout) {
   const size_t step = (size_t)blockDim.x * U;
+  stream_wait();
   for (size_t base = (size_t)blockIdx.x * step + threadIdx.x; base < n;
        base += (size_t)gridDim.x * step) {
     uint4 va[U], vb[U];
@@ -89,9 +91,7 @@ int launch_blas(bntt_ctx* ctx, int op, void* c, const void* a, const void* b, U1
   U128 xx = x;
   int lay = layout;
   void* args[] = {&cc, &aa, &bb, &n, &m, &xx, &lay};
-  BNTT_CK(cudaLaunchKernel(fn, dim3(grid), dim3(kBlasThreads), args, 0, stream));
-  ctx->launches++;
-  return BNTT_OK;
+  return launch_overlapped(ctx, fn, grid, kBlasThreads, 0, args, stream);
 }
 
 }  // namespace bntt

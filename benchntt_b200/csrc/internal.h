@@ -88,6 +88,10 @@ const SubKernel* default_sub_kernel(int m, int map, int fast, uint64_t elems);
 int launch_sub(bntt_ctx* ctx, const SubKernel* k, const void* geom, const ModParams& mp,
                int layout, cudaStream_t stream, int finishing = 0);
 int blocks_per_sm(const SubKernel* k);
+// Launches a kernel that starts with stream_wait() (ntt_core.cuh): its CTAs may
+// become resident while the kernel before it in the stream still runs.
+int launch_overlapped(bntt_ctx* ctx, const void* fn, unsigned grid, unsigned threads, size_t smem, void** args,
+                      cudaStream_t stream);
 
 // Autotuner choices (nullptr / -1 when not tuned).
 const SubKernel* tuned_sub_kernel(int m, int map, int fast, int l);

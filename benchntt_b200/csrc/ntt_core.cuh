@@ -42,14 +42,22 @@ struct SubRef {
   bool valid;
 };
 
-// Load policy for the first pass's HBM reads: the read-only path, or L2 only
-// (coherent with writes made earlier in the same kernel by other CTAs).
-enum : int { LD_NC = 0, LD_CG = 1 };
+// Data and tables are read with coherent loads, data through L2 only: a
+// transform's input may have been written earlier in the same launch (later
+// passes of the persistent kernel) or by the kernel before it, which a plan
+// kernel overlaps (stream_wait).
+__device__ __forceinline__ uint4 ld_data(const uint4* p) { return __ldcg(p); }
 
-template <int LDP>
-__device__ __forceinline__ uint4 ld_data(const uint4* p) {
-  if constexpr (LDP == LD_CG) return __ldcg(p);
-  else return __ldg(p);
+// Programmatic dependent launch: the plan and vector kernels are launched as
+// soon as the kernel before them in the stream has started its last CTA, and
+// wait here until that kernel has completed and its writes are visible;
+// nothing is read or written before.  The wait comes first, so a kernel lets
+// the next one in only after its own predecessor has completed.  Without it
+// the end of one kernel and the start of the next cost a small launch about
+// 2 us (2^15 elements of 2^9 points back to back: 6.2 -> 4.0 us).
+__device__ __forceinline__ void stream_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // Optional pointwise product fused into the store of a transform's last
@@ -173,13 +181,13 @@ struct NttTile {
   // Runs the whole sub-transform.  Every thread of the tile must call it
   // (it synchronises); threads whose sub-transform is not valid compute on
   // zeros and store nothing.
-  template <int LDP, int SRC = SRC_GLOBAL>
+  template <int SRC = SRC_GLOBAL>
   __device__ __forceinline__ static void run(const SubRef& sr, int sub, int lane, uint4* smem,
                                              const ModParams& mp, int layout,
                                              const MulB& mb = MulB{}) {
     U128 v[R];
-    if constexpr (Arith::kFast) pass_lazy<0, LDP, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
-    else pass<0, LDP>(v, sr, sub, lane, smem, mp, layout, mb);
+    if constexpr (Arith::kFast) pass_lazy<0, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
+    else pass<0>(v, sr, sub, lane, smem, mp, layout, mb);
   }
 
   // Stages run on partly reduced values (u128.cuh) before pass p since they
@@ -195,7 +203,7 @@ struct NttTile {
   // One pass on partly reduced values (fast moduli).  Only the elements that
   // the first stage adds to need a base of 8q; the ones it multiplies are
   // taken as they are.
-  template <int P, int LDP, int SRC>
+  template <int P, int SRC>
   __device__ __forceinline__ static void pass_lazy(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                                    uint4* smem, const ModParams& mp, int layout,
                                                    const MulB& mb) {
@@ -218,7 +226,7 @@ struct NttTile {
         return from_mem(smem[slot_at(sb, j << lo)], layout);  // staged in memory order
       } else if constexpr (P == 0) {
         if (!sr.valid) return U128{{0u, 0u, 0u, 0u}};
-        return from_mem(ld_data<LDP>(sr.x + ((size_t)base << lshift) + (size_t)j * gstep), layout);
+        return from_mem(ld_data(sr.x + ((size_t)base << lshift) + (size_t)j * gstep), layout);
       } else {
         const uint4 t = smem[slot_at(sb, j << lo)];
         return U128{{t.x, t.y, t.z, t.w}};
@@ -249,7 +257,7 @@ struct NttTile {
       lazy_stages<r>(v, i * G, [&](int t, int u) {
         // tables are stored in limb order (LAYOUT_U128) by the plan
         const uint4* twt = tw_at(sr.tw, gt << t);  // u as an immediate offset
-        const uint4 tv = (SRC & TW_SHARED) != 0 ? lds128(twt + u) : __ldg(twt + u);
+        const uint4 tv = (SRC & TW_SHARED) != 0 ? lds128(twt + u) : twt[u];
         return U128{{tv.x, tv.y, tv.z, tv.w}};
       }, k, rerun);
     }
@@ -287,7 +295,7 @@ struct NttTile {
             uint4* yp = sr.y + ((size_t)base << lshift) + (size_t)j * gstep;
             U128 o = v[i * G + j];
             if (mb.b) {
-              const uint4 bv = __ldg(mb.b + ((uint64_t)(yp - mb.ybase) & mb.bmask));
+              const uint4 bv = mb.b[(uint64_t)(yp - mb.ybase) & mb.bmask];
               o = reduce_once(mul_lazy(from_mem(bv, layout), o, k), k);
             }
             *yp = to_mem(o, layout);
@@ -300,12 +308,12 @@ struct NttTile {
     }
     if constexpr (P + 1 < NPASS) {
       sync_between<P, P + 1>();
-      pass_lazy<P + 1, LDP, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
+      pass_lazy<P + 1, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
     }
   }
 
   // One pass in the replica arithmetic (ArithRef).
-  template <int P, int LDP>
+  template <int P>
   __device__ __forceinline__ static void pass(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                               uint4* smem, const ModParams& mp, int layout,
                                               const MulB& mb) {
@@ -328,7 +336,7 @@ struct NttTile {
       for (int j = 0; j < G; ++j) {
         if constexpr (P == 0) {
           if (sr.valid) {
-            v[i * G + j] = from_mem(ld_data<LDP>(sr.x + ((size_t)base << sr.lshift) + (size_t)j * gstep), layout);
+            v[i * G + j] = from_mem(ld_data(sr.x + ((size_t)base << sr.lshift) + (size_t)j * gstep), layout);
           } else {
 #pragma unroll
             for (int w = 0; w < 4; ++w) v[i * G + j].w[w] = 0u;
@@ -352,7 +360,7 @@ struct NttTile {
         for (int u = 0; u < (1 << t); ++u) {
           // tables are stored in limb order (LAYOUT_U128) by the plan
           const uint4* twt = sr.tw + (gt << t);  // u as an immediate offset
-          const uint4 tv = __ldg(twt + u);
+          const uint4 tv = twt[u];
           const U128 w = U128{{tv.x, tv.y, tv.z, tv.w}};
 #pragma unroll
           for (int k = 0; k < half; ++k) {
@@ -376,7 +384,7 @@ struct NttTile {
             uint4* yp = sr.y + ((size_t)base << sr.lshift) + (size_t)j * gstep;
             U128 o = v[i * G + j];
             if (mb.b) {
-              const uint4 bv = __ldg(mb.b + ((uint64_t)(yp - mb.ybase) & mb.bmask));
+              const uint4 bv = mb.b[(uint64_t)(yp - mb.ybase) & mb.bmask];
               o = Arith::mul(o, from_mem(bv, layout), mp);
             }
             *yp = to_mem(o, layout);
@@ -389,7 +397,7 @@ struct NttTile {
     }
     if constexpr (P + 1 < NPASS) {
       sync_between<P, P + 1>();
-      pass<P + 1, LDP>(v, sr, sub, lane, smem, mp, layout, mb);
+      pass<P + 1>(v, sr, sub, lane, smem, mp, layout, mb);
     }
   }
 
@@ -399,15 +407,14 @@ struct NttTile {
   // multiplies the lower half of each group -- the x outputs of stage 0 --
   // by *scale_at (N^-1) when scale_at is not null; the upper half gets N^-1
   // through the inverse table's entry 1.  Fast moduli only.
-  template <int LDP>
   __device__ __forceinline__ static void run_inv(const SubRef& sr, int sub, int lane, uint4* smem,
                                                  const ModParams& mp, int layout,
                                                  const uint4* scale_at) {
     U128 v[R];
-    pass_inv<NPASS - 1, LDP>(v, sr, sub, lane, smem, mp, layout, scale_at);
+    pass_inv<NPASS - 1>(v, sr, sub, lane, smem, mp, layout, scale_at);
   }
 
-  template <int P, int LDP>
+  template <int P>
   __device__ __forceinline__ static void pass_inv(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                                   uint4* smem, const ModParams& mp, int layout,
                                                   const uint4* scale_at) {
@@ -430,7 +437,7 @@ struct NttTile {
       for (int j = 0; j < G; ++j) {
         if constexpr (P == NPASS - 1) {
           if (sr.valid) {
-            v[i * G + j] = from_mem(ld_data<LDP>(sr.x + ((size_t)base << lshift) + (size_t)j * gstep), layout);
+            v[i * G + j] = from_mem(ld_data(sr.x + ((size_t)base << lshift) + (size_t)j * gstep), layout);
           } else {
 #pragma unroll
             for (int w = 0; w < 4; ++w) v[i * G + j].w[w] = 0u;
@@ -448,7 +455,7 @@ struct NttTile {
       const int g = lane + i * TPT;
       const uint32_t gt = (sr.trow << s0) + (uint32_t)(g >> lo);
       inverse_stages<r, P == 0>(v, i * G, [&](int t, int u) {
-        const uint4 tv = __ldg(tw_at(sr.tw, gt << t) + u);
+        const uint4 tv = tw_at(sr.tw, gt << t)[u];
         return U128{{tv.x, tv.y, tv.z, tv.w}};
       }, mp.k);
     }
@@ -456,7 +463,7 @@ struct NttTile {
     // ---- canonical results; N^-1 on the finishing store
     if constexpr (P == 0) {
       if (scale_at) {
-        const uint4 f = __ldg(scale_at);
+        const uint4 f = *scale_at;
         const U128 fs = U128{{f.x, f.y, f.z, f.w}};
 #pragma unroll
         for (int i = 0; i < GPT; ++i)
@@ -490,7 +497,7 @@ struct NttTile {
     }
     if constexpr (P > 0) {
       sync_between<P, P - 1>();
-      pass_inv<P - 1, LDP>(v, sr, sub, lane, smem, mp, layout, scale_at);
+      pass_inv<P - 1>(v, sr, sub, lane, smem, mp, layout, scale_at);
     }
   }
 };

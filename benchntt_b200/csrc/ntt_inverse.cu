@@ -39,10 +39,11 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, ArithFast>::THREADS
   extern __shared__ uint4 smem[];
   const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
   const uint4* scale_at = finishing ? g.tw : nullptr;
+  stream_wait();
   const uint64_t sid = (uint64_t)blockIdx.x * TPC + (uint64_t)sub;
   const SubRef sr = MAP == MAP_CONTIG ? make_subref_contig<M>(g, sid) : make_subref(g, sid);
-  if (layout == LAYOUT_HILO) T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_HILO, scale_at);
-  else T::template run_inv<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
+  if (layout == LAYOUT_HILO) T::run_inv(sr, sub, lane, smem, mp, LAYOUT_HILO, scale_at);
+  else T::run_inv(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
 }
 
 // The shape for a pass of m stages over `elems` elements.

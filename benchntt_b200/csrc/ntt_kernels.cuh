@@ -23,12 +23,13 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, Arith>::THREADS, MI
   extern __shared__ uint4 smem[];
   const int tid = threadIdx.x;
   const int sub = T::sub_of(tid), lane = T::lane_of(tid);
+  stream_wait();
   const uint64_t sid = (uint64_t)blockIdx.x * TPC + (uint64_t)sub;
   const SubRef sr = MAP == MAP_CONTIG ? make_subref_contig<M>(g, sid) : make_subref(g, sid);
   // the element layout as a constant in each branch: no word select per
   // HBM load and store
-  if (layout == LAYOUT_HILO) T::template run<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_HILO, MulB{g.b, g.y, g.bmask});
-  else T::template run<LD_NC>(sr, sub, lane, smem, mp, LAYOUT_U128, MulB{g.b, g.y, g.bmask});
+  if (layout == LAYOUT_HILO) T::run(sr, sub, lane, smem, mp, LAYOUT_HILO, MulB{g.b, g.y, g.bmask});
+  else T::run(sr, sub, lane, smem, mp, LAYOUT_U128, MulB{g.b, g.y, g.bmask});
 }
 
 // Contiguous sub-transforms (L = 0: tile t is the 16-byte elements
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP_CONTIG, Arith>::THRE
   const int tid = threadIdx.x;
   const int sub = T::sub_of(tid), lane = T::lane_of(tid);
   const uint64_t ntiles = (g.nsub + TPC - 1) / TPC;
+  stream_wait();
   // tile t's valid elements, copied into `dst` in slot order
   auto stage = [&](uint64_t t, uint4* dst) {
     const uint64_t first = t * TPC;
@@ -68,7 +70,7 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP_CONTIG, Arith>::THRE
   const uint4* tw = g.tw;
   if constexpr ((SRC & TW_SHARED) != 0) {
     uint4* const tws = smem + 2 * TILE;
-    for (int e = tid; e < N; e += T::THREADS) tws[e] = __ldg(g.tw + e);
+    for (int e = tid; e < N; e += T::THREADS) tws[e] = g.tw[e];
     tw = tws;  // made visible by the barrier before the first tile
   }
   uint64_t tile = blockIdx.x;
@@ -83,10 +85,10 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP_CONTIG, Arith>::THRE
     SubRef sr = make_subref_contig<M>(g, tile * TPC + (uint64_t)sub);
     sr.tw = tw;
     if (layout == LAYOUT_HILO)
-      T::template run<LD_NC, SRC | SRC_STAGED>(sr, sub, lane, smem + b * TILE, mp, LAYOUT_HILO,
+      T::template run<SRC | SRC_STAGED>(sr, sub, lane, smem + b * TILE, mp, LAYOUT_HILO,
                                                MulB{g.b, g.y, g.bmask});
     else
-      T::template run<LD_NC, SRC | SRC_STAGED>(sr, sub, lane, smem + b * TILE, mp, LAYOUT_U128,
+      T::template run<SRC | SRC_STAGED>(sr, sub, lane, smem + b * TILE, mp, LAYOUT_U128,
                                                MulB{g.b, g.y, g.bmask});
     __syncthreads();  // this buffer is refilled by the next iteration's copy
   }

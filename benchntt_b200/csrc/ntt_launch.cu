@@ -84,7 +84,22 @@ int launch_sub(bntt_ctx* ctx, const SubKernel* k, const void* geom, const ModPar
   ModParams mm = mp;
   int lay = layout;
   void* args[] = {&gg, &mm, &lay, &finishing};  // the forward kernels take the first three
-  BNTT_CK(cudaLaunchKernel(k->fn, dim3((unsigned)grid), dim3(k->threads), args, k->smem, stream));
+  return launch_overlapped(ctx, k->fn, (unsigned)grid, (unsigned)k->threads, k->smem, args, stream);
+}
+
+int launch_overlapped(bntt_ctx* ctx, const void* fn, unsigned grid, unsigned threads, size_t smem, void** args,
+                      cudaStream_t stream) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  BNTT_CK(cudaLaunchKernelExC(&cfg, fn, args));
   ctx->launches++;
   return BNTT_OK;
 }
