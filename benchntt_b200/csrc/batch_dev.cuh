@@ -216,7 +216,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const BatchArgs& ba
     const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
     const SubRef sr = item_subref<M, MAP>(it, ba, turn * HELD + sub);
     if (turn > 0) T::sync();  // smem is reused
-    T::run(sr, sub, lane, smem, mp, layout);
+    T::template run<TW_CONST>(sr, sub, lane, smem, mp, layout);
   }
   item_publish(it, ba);
 }

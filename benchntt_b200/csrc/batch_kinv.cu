@@ -25,7 +25,7 @@ __device__ __forceinline__ void run_item_inv(const WorkItem& it, const BatchArgs
     const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
     const SubRef sr = item_subref<M, MAP>(it, ba, turn * HELD + sub);
     if (turn > 0) T::sync();  // smem is reused
-    T::run_inv(sr, sub, lane, smem, mp, LY, finishes ? sr.tw : nullptr);
+    T::template run_inv<TW_CONST>(sr, sub, lane, smem, mp, LY, finishes ? sr.tw : nullptr);
   }
   item_publish(it, ba);
 }

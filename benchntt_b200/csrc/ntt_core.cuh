@@ -76,7 +76,10 @@ struct MulB {
 //               beforehand (cp.async, k_ntt_sub_staged); the first pass
 //               gathers from there like the later passes
 //   TW_SHARED   sr.tw points at a copy of the table in shared memory
-enum : int { SRC_GLOBAL = 0, SRC_STAGED = 1, TW_SHARED = 2 };
+//   TW_CONST    no kernel still running may write the table: read-only loads,
+//               which the compiler may move over the exchanges (kernels
+//               without stream_wait)
+enum : int { SRC_GLOBAL = 0, SRC_STAGED = 1, TW_SHARED = 2, TW_CONST = 4 };
 
 // 16-byte asynchronous copy global -> shared (cp.async, L2 only), and the
 // group commit / wait that order them.
@@ -257,7 +260,7 @@ struct NttTile {
       lazy_stages<r>(v, i * G, [&](int t, int u) {
         // tables are stored in limb order (LAYOUT_U128) by the plan
         const uint4* twt = tw_at(sr.tw, gt << t);  // u as an immediate offset
-        const uint4 tv = (SRC & TW_SHARED) != 0 ? lds128(twt + u) : twt[u];
+        const uint4 tv = (SRC & TW_SHARED) != 0 ? lds128(twt + u) : (SRC & TW_CONST) != 0 ? __ldg(twt + u) : twt[u];
         return U128{{tv.x, tv.y, tv.z, tv.w}};
       }, k, rerun);
     }
@@ -407,14 +410,15 @@ struct NttTile {
   // multiplies the lower half of each group -- the x outputs of stage 0 --
   // by *scale_at (N^-1) when scale_at is not null; the upper half gets N^-1
   // through the inverse table's entry 1.  Fast moduli only.
+  template <int SRC = SRC_GLOBAL>
   __device__ __forceinline__ static void run_inv(const SubRef& sr, int sub, int lane, uint4* smem,
                                                  const ModParams& mp, int layout,
                                                  const uint4* scale_at) {
     U128 v[R];
-    pass_inv<NPASS - 1>(v, sr, sub, lane, smem, mp, layout, scale_at);
+    pass_inv<NPASS - 1, SRC>(v, sr, sub, lane, smem, mp, layout, scale_at);
   }
 
-  template <int P>
+  template <int P, int SRC>
   __device__ __forceinline__ static void pass_inv(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                                   uint4* smem, const ModParams& mp, int layout,
                                                   const uint4* scale_at) {
@@ -455,7 +459,8 @@ struct NttTile {
       const int g = lane + i * TPT;
       const uint32_t gt = (sr.trow << s0) + (uint32_t)(g >> lo);
       inverse_stages<r, P == 0>(v, i * G, [&](int t, int u) {
-        const uint4 tv = tw_at(sr.tw, gt << t)[u];
+        const uint4* twt = tw_at(sr.tw, gt << t);
+        const uint4 tv = (SRC & TW_CONST) != 0 ? __ldg(twt + u) : twt[u];
         return U128{{tv.x, tv.y, tv.z, tv.w}};
       }, mp.k);
     }
@@ -497,7 +502,7 @@ struct NttTile {
     }
     if constexpr (P > 0) {
       sync_between<P, P - 1>();
-      pass_inv<P - 1>(v, sr, sub, lane, smem, mp, layout, scale_at);
+      pass_inv<P - 1, SRC>(v, sr, sub, lane, smem, mp, layout, scale_at);
     }
   }
 };
