@@ -107,32 +107,37 @@ const void* batch_kernel(bool fast, int layout) {
 
 constexpr int kMaxLog2n = 24;  // plans hold 2^1..2^24 points
 
-// HBM passes of a large batch job: the fewest passes, then the fewest
-// 4-element tile passes (a pass of m stages is ceil(m / 2) of them).  A strided pass
+// HBM passes of a large transform: the fewest, then of least cost.  A strided pass
 // (all but the last) has 5..7 stages, so its tile of 2^(10 - m) adjacent
 // columns covers at least 128 bytes of each row, and needs that many columns
-// (2^(10 - m) <= 2^l); the last, contiguous pass has 3..10 stages.
+// (2^(10 - m) <= 2^l); the last, contiguous pass has 3..10 stages.  Costs: us
+// for 2^22 elements on the plan kernels.  A pass's cost is not its stages
+// alone: exchanges and the reduction at its end count too, so 2^11 = 6 + 5
+// (86.0) beats 7 + 4 (89.0) and 2^13 = 5 + 8 (99.2) beats 7 + 6 (101.9).
 static std::vector<int> batch_split(int n) {
+  static const double strided[8] = {0, 0, 0, 0, 0, 39.7, 45.4, 55.6};
+  static const double contiguous[11] = {0, 0, 0, 31.9, 33.4, 40.6, 46.3, 54.9, 59.5, 67.3, 75.1};
   std::vector<int> best, cur;
-  int best_passes = 1 << 30, best_cost = 1 << 30;
-  std::function<void(int, int, int)> rec = [&](int s0, int cost, int depth) {
+  size_t best_passes = ~(size_t)0;
+  double best_cost = 1e30;
+  std::function<void(int, double, int)> rec = [&](int s0, double cost, int depth) {
     const int left = n - s0;
     if (left >= 3 && left <= 10) {  // finish with a contiguous pass
-      cur.push_back(left);
-      const int passes = (int)cur.size(), c = cost + (left + 1) / 2;
+      const size_t passes = cur.size() + 1;
+      const double c = cost + contiguous[left];
       if (passes < best_passes || (passes == best_passes && c < best_cost)) {
         best_passes = passes;
         best_cost = c;
         best = cur;
+        best.push_back(left);
       }
-      cur.pop_back();
     }
     if (depth + 1 >= kMaxPasses) return;
     for (int m = 7; m >= 5; --m) {
       const int l = n - s0 - m;
       if (l < 3 || 10 - m > l) continue;
       cur.push_back(m);
-      rec(s0 + m, cost + (m + 1) / 2, depth + 1);
+      rec(s0 + m, cost + strided[m], depth + 1);
       cur.pop_back();
     }
   };

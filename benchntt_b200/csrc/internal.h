@@ -69,15 +69,20 @@ struct SubKernel {
   int use = 0;            // USE_* below: where it is the default
 };
 
-// Launches a shape is the default of: none (an autotuner candidate), those of
-// fewer than kManyElems elements, the others, or both.
-enum : int { USE_TUNED = 0, USE_FEW = 1, USE_MANY = 2, USE_ALL = 3 };
+// Launches a shape is the default of, by their elements: up to kLoneElems,
+// below kManyElems, the others; 0 for an autotuner candidate.
+enum : int { USE_TUNED = 0, USE_LONE = 1, USE_FEW = 2, USE_MANY = 4, USE_ALL = 7 };
 // A launch below 2^21 elements does not fill the SMs' thread slots several
 // times over: 4 elements per thread in small CTAs spread it over more warps
 // (37 x 2^13 points: 8.3 -> 6.2 us for the pass).  Above, 8 elements per
 // thread save index and exchange instructions (65,536 x 2^10: 3 %; a strided
 // pass of 6 stages 7 %).  Both are equal within 3 % from 2^20 to 2^22.
 constexpr uint64_t kManyElems = 1ull << 21;
+// Up to 2^17 elements an SM holds at most a quarter of its warps, and a pass's
+// table loads are latency: TW_AHEAD (one transform of 2^9 points 4.0 -> 3.25
+// us, of 2^10 5.4 -> 4.8).  At 2^18 its registers cost as much as it gives.
+constexpr uint64_t kLoneElems = 1ull << 17;
+inline int use_of(uint64_t elems) { return elems <= kLoneElems ? USE_LONE : elems < kManyElems ? USE_FEW : USE_MANY; }
 
 const std::vector<SubKernel>& sub_kernels();
 // Default shape of a pass of m stages over `elems` elements; nullptr if none
@@ -99,8 +104,8 @@ int tuned_batch_small_shape(int m);
 
 // HBM passes of a 2^n transform (11 <= n <= 24), as the persistent kernel
 // splits its large jobs: strided passes of 5..7 stages (2^(10 - m) adjacent
-// columns per tile), then a contiguous pass of up to 10; the fewest passes,
-// then the fewest tile passes.  Empty outside that range.
+// columns per tile), then a contiguous pass of up to 10.  Empty outside that
+// range.
 std::vector<int> tile_split(int n);
 
 int launch_blas(bntt_ctx* ctx, int op, void* c, const void* a, const void* b, U128 x, size_t len,

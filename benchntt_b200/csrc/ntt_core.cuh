@@ -79,7 +79,10 @@ struct MulB {
 //   TW_CONST    no kernel still running may write the table: read-only loads,
 //               which the compiler may move over the exchanges (kernels
 //               without stream_wait)
-enum : int { SRC_GLOBAL = 0, SRC_STAGED = 1, TW_SHARED = 2, TW_CONST = 4 };
+//   TW_AHEAD    the entries of every pass are loaded into registers together
+//               with the input (launches that do not fill the SMs, where a
+//               table load per pass is latency nothing hides)
+enum : int { SRC_GLOBAL = 0, SRC_STAGED = 1, TW_SHARED = 2, TW_CONST = 4, TW_AHEAD = 8 };
 
 // 16-byte asynchronous copy global -> shared (cp.async, L2 only), and the
 // group commit / wait that order them.
@@ -189,8 +192,55 @@ struct NttTile {
                                              const ModParams& mp, int layout,
                                              const MulB& mb = MulB{}) {
     U128 v[R];
-    if constexpr (Arith::kFast) pass_lazy<0, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
-    else pass<0>(v, sr, sub, lane, smem, mp, layout, mb);
+    if constexpr (Arith::kFast) {
+      Table<SRC> tw;
+      load_table<0, SRC>(tw, sr, lane);
+      pass_lazy<0, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw);
+    } else {
+      pass<0>(v, sr, sub, lane, smem, mp, layout, mb);
+    }
+  }
+
+  // The thread's table entries: with TW_AHEAD those of all passes in registers
+  // (entry u of stage t of group i at (i << r) + 2^t - 1 + u), else none.
+  template <int SRC>
+  struct Table {
+    static constexpr bool kAhead = (SRC & TW_AHEAD) != 0;
+    uint4 at[kAhead ? NPASS : 1][kAhead ? R : 1];
+  };
+  __device__ __forceinline__ static uint32_t table_row(const SubRef& sr, int lane, int i, int s0, int lo) {
+    return (sr.trow << s0) + (uint32_t)((lane + i * TPT) >> lo);
+  }
+  template <int P, int SRC>
+  __device__ __forceinline__ static void load_table(Table<SRC>& a, const SubRef& sr, int lane) {
+    if constexpr (Table<SRC>::kAhead) {
+      constexpr int r = bits(P);
+#pragma unroll
+      for (int i = 0; i < (R >> r); ++i) {
+        const uint32_t gt = table_row(sr, lane, i, start(P), low(P));
+#pragma unroll
+        for (int t = 0; t < r; ++t)
+#pragma unroll
+          for (int u = 0; u < (1 << t); ++u) a.at[P][(i << r) + (1 << t) - 1 + u] = tw_at(sr.tw, gt << t)[u];
+      }
+      if constexpr (P + 1 < NPASS) load_table<P + 1, SRC>(a, sr, lane);
+    }
+  }
+  // entry u of stage t of group i in pass P; gt: the group's table_row
+  template <int P, int SRC>
+  __device__ __forceinline__ static U128 table_entry(const Table<SRC>& a, const SubRef& sr, uint32_t gt, int i, int t,
+                                                     int u) {
+    uint4 v;
+    if constexpr (Table<SRC>::kAhead) {
+      v = a.at[P][(i << bits(P)) + (1 << t) - 1 + u];
+    } else {
+      // tables are stored in limb order (LAYOUT_U128) by the plan
+      const uint4* p = tw_at(sr.tw, gt << t) + u;  // u as an immediate offset
+      if constexpr ((SRC & TW_SHARED) != 0) v = lds128(p);
+      else if constexpr ((SRC & TW_CONST) != 0) v = __ldg(p);
+      else v = *p;
+    }
+    return U128{{v.x, v.y, v.z, v.w}};
   }
 
   // Stages run on partly reduced values (u128.cuh) before pass p since they
@@ -209,7 +259,7 @@ struct NttTile {
   template <int P, int SRC>
   __device__ __forceinline__ static void pass_lazy(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                                    uint4* smem, const ModParams& mp, int layout,
-                                                   const MulB& mb) {
+                                                   const MulB& mb, const Table<SRC>& tw) {
     constexpr int r = bits(P);
     constexpr int s0 = start(P);
     constexpr int lo = M - s0 - r;        // lowest local bit this pass touches
@@ -239,7 +289,7 @@ struct NttTile {
       const int g = lane + i * TPT;
       return (g & ((1 << lo) - 1)) | ((g >> lo) << (lo + r));
     };
-    auto gt_of = [&](int i) { return (sr.trow << s0) + (uint32_t)((lane + i * TPT) >> lo); };
+    auto gt_of = [&](int i) { return table_row(sr, lane, i, s0, lo); };
 
 #pragma unroll
     for (int i = 0; i < GPT; ++i) {
@@ -257,12 +307,7 @@ struct NttTile {
         else if constexpr (rebase(P)) x = add_8q(fold_top(x, k), k);
       }
       const uint32_t gt = gt_of(i);
-      lazy_stages<r>(v, i * G, [&](int t, int u) {
-        // tables are stored in limb order (LAYOUT_U128) by the plan
-        const uint4* twt = tw_at(sr.tw, gt << t);  // u as an immediate offset
-        const uint4 tv = (SRC & TW_SHARED) != 0 ? lds128(twt + u) : (SRC & TW_CONST) != 0 ? __ldg(twt + u) : twt[u];
-        return U128{{tv.x, tv.y, tv.z, tv.w}};
-      }, k, rerun);
+      lazy_stages<r>(v, i * G, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, gt, i, t, u); }, k, rerun);
     }
     // the transform's outputs: below q unless the top limb says otherwise
     if constexpr (last) {
@@ -311,7 +356,7 @@ struct NttTile {
     }
     if constexpr (P + 1 < NPASS) {
       sync_between<P, P + 1>();
-      pass_lazy<P + 1, SRC>(v, sr, sub, lane, smem, mp, layout, mb);
+      pass_lazy<P + 1, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw);
     }
   }
 
@@ -415,13 +460,15 @@ struct NttTile {
                                                  const ModParams& mp, int layout,
                                                  const uint4* scale_at) {
     U128 v[R];
-    pass_inv<NPASS - 1, SRC>(v, sr, sub, lane, smem, mp, layout, scale_at);
+    Table<SRC> tw;
+    load_table<0, SRC>(tw, sr, lane);
+    pass_inv<NPASS - 1, SRC>(v, sr, sub, lane, smem, mp, layout, scale_at, tw);
   }
 
   template <int P, int SRC>
   __device__ __forceinline__ static void pass_inv(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                                   uint4* smem, const ModParams& mp, int layout,
-                                                  const uint4* scale_at) {
+                                                  const uint4* scale_at, const Table<SRC>& tw) {
     constexpr int r = bits(P);
     constexpr int s0 = start(P);
     constexpr int lo = M - s0 - r;
@@ -456,13 +503,9 @@ struct NttTile {
     // ---- r stages on each group, the last first
 #pragma unroll
     for (int i = 0; i < GPT; ++i) {
-      const int g = lane + i * TPT;
-      const uint32_t gt = (sr.trow << s0) + (uint32_t)(g >> lo);
-      inverse_stages<r, P == 0>(v, i * G, [&](int t, int u) {
-        const uint4* twt = tw_at(sr.tw, gt << t);
-        const uint4 tv = (SRC & TW_CONST) != 0 ? __ldg(twt + u) : twt[u];
-        return U128{{tv.x, tv.y, tv.z, tv.w}};
-      }, mp.k);
+      const uint32_t gt = table_row(sr, lane, i, s0, lo);
+      inverse_stages<r, P == 0>(
+          v, i * G, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, gt, i, t, u); }, mp.k);
     }
 
     // ---- canonical results; N^-1 on the finishing store
@@ -502,7 +545,7 @@ struct NttTile {
     }
     if constexpr (P > 0) {
       sync_between<P, P - 1>();
-      pass_inv<P - 1, SRC>(v, sr, sub, lane, smem, mp, layout, scale_at);
+      pass_inv<P - 1, SRC>(v, sr, sub, lane, smem, mp, layout, scale_at, tw);
     }
   }
 };

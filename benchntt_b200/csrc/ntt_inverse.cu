@@ -32,7 +32,7 @@ namespace {
 // transform (interleaved for the strided passes).  `finishing` marks the
 // pass that ends the transform (stage 0 inside it), which applies N^-1 from
 // entry 0 of the inverse table.
-template <int M, int LOGR, int TPC, int MAP, int MINB>
+template <int M, int LOGR, int TPC, int MAP, int MINB, int SRC>
 __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, ArithFast>::THREADS, MINB)
     k_ntt_tile_inv(SubGeom g, ModParams mp, int layout, int finishing) {
   using T = NttTile<M, LOGR, TPC, MAP, ArithFast>;
@@ -42,20 +42,20 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, ArithFast>::THREADS
   stream_wait();
   const uint64_t sid = (uint64_t)blockIdx.x * TPC + (uint64_t)sub;
   const SubRef sr = MAP == MAP_CONTIG ? make_subref_contig<M>(g, sid) : make_subref(g, sid);
-  if (layout == LAYOUT_HILO) T::run_inv(sr, sub, lane, smem, mp, LAYOUT_HILO, scale_at);
-  else T::run_inv(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
+  if (layout == LAYOUT_HILO) T::template run_inv<SRC>(sr, sub, lane, smem, mp, LAYOUT_HILO, scale_at);
+  else T::template run_inv<SRC>(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
 }
 
 // The shape for a pass of m stages over `elems` elements.
 const SubKernel* inverse_kernel(int m, int map, uint64_t elems) {
   static const SubKernel kernels[] = {
-#define BNTT_ADD(M, LOGR, TPC, MAP, MINB, USE) \
-  BNTT_SUBK_FN(M, LOGR, TPC, MAP, ArithFast, MINB, (k_ntt_tile_inv<M, LOGR, TPC, MAP, MINB>), USE),
+#define BNTT_ADD(M, LOGR, TPC, MAP, MINB, SRC, USE) \
+  BNTT_SUBK_FN(M, LOGR, TPC, MAP, ArithFast, MINB, (k_ntt_tile_inv<M, LOGR, TPC, MAP, MINB, SRC>), USE),
       BNTT_PLAN_SHAPES(BNTT_ADD)
 #undef BNTT_ADD
   };
   for (const SubKernel& k : kernels)
-    if (k.m == m && k.map == map && (k.use & (elems >= kManyElems ? USE_MANY : USE_FEW))) return &k;
+    if (k.m == m && k.map == map && (k.use & use_of(elems))) return &k;
   return nullptr;
 }
 

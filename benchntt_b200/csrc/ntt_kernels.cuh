@@ -16,7 +16,7 @@ namespace bntt {
 // resident CTAs lies between (1282, 1247, 1229).
 // MINB > 0 asks for at least MINB resident CTAs per SM (fewer registers per
 // thread, more warps to hide the latency of the carry chains).
-template <int M, int LOGR, int TPC, int MAP, class Arith, int MINB>
+template <int M, int LOGR, int TPC, int MAP, class Arith, int MINB, int SRC = SRC_GLOBAL>
 __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, Arith>::THREADS, MINB)
     k_ntt_sub(SubGeom g, ModParams mp, int layout) {
   using T = NttTile<M, LOGR, TPC, MAP, Arith>;
@@ -28,8 +28,8 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, Arith>::THREADS, MI
   const SubRef sr = MAP == MAP_CONTIG ? make_subref_contig<M>(g, sid) : make_subref(g, sid);
   // the element layout as a constant in each branch: no word select per
   // HBM load and store
-  if (layout == LAYOUT_HILO) T::run(sr, sub, lane, smem, mp, LAYOUT_HILO, MulB{g.b, g.y, g.bmask});
-  else T::run(sr, sub, lane, smem, mp, LAYOUT_U128, MulB{g.b, g.y, g.bmask});
+  if (layout == LAYOUT_HILO) T::template run<SRC>(sr, sub, lane, smem, mp, LAYOUT_HILO, MulB{g.b, g.y, g.bmask});
+  else T::template run<SRC>(sr, sub, lane, smem, mp, LAYOUT_U128, MulB{g.b, g.y, g.bmask});
 }
 
 // Contiguous sub-transforms (L = 0: tile t is the 16-byte elements
@@ -98,32 +98,40 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP_CONTIG, Arith>::THRE
 }  // namespace bntt
 
 // Default shapes of the plan transforms with the fast multiply, forward and
-// inverse: X(M, LOGR, TPC, map, resident CTAs per SM, use).  CTAs of 64 or 128
-// threads: with one CTA per tile, smaller ones keep an SM's warps in more
+// inverse: X(M, LOGR, TPC, map, resident CTAs per SM, SRC, use).  CTAs of 64 or
+// 128 threads: with one CTA per tile, smaller ones keep an SM's warps in more
 // different phases (2^24 elements of 2^8: 256 threads 250 us, 64 threads 234).
 // Interleaved tiles keep at least 8 columns (128 bytes of a row).
-#define BNTT_PLAN_SHAPES(X)                      \
-  X(1, 1, 256, MAP_CONTIG, 4, USE_ALL)           \
-  X(2, 2, 256, MAP_CONTIG, 4, USE_ALL)           \
-  X(3, 2, 32, MAP_CONTIG, 16, USE_ALL)           \
-  X(4, 2, 16, MAP_CONTIG, 16, USE_ALL)           \
-  X(5, 2, 8, MAP_CONTIG, 16, USE_FEW)            \
-  X(5, 3, 16, MAP_CONTIG, 12, USE_MANY)          \
-  X(6, 2, 4, MAP_CONTIG, 16, USE_FEW)            \
-  X(6, 3, 8, MAP_CONTIG, 12, USE_MANY)           \
-  X(7, 2, 2, MAP_CONTIG, 16, USE_FEW)            \
-  X(7, 3, 4, MAP_CONTIG, 12, USE_MANY)           \
-  X(8, 2, 1, MAP_CONTIG, 16, USE_ALL)            \
-  X(9, 2, 1, MAP_CONTIG, 8, USE_FEW)             \
-  X(9, 3, 1, MAP_CONTIG, 10, USE_MANY)           \
-  X(10, 2, 1, MAP_CONTIG, 4, USE_FEW)            \
-  X(10, 3, 1, MAP_CONTIG, 6, USE_MANY)           \
-  X(5, 2, 16, MAP_INTERLEAVED, 8, USE_FEW)       \
-  X(5, 3, 32, MAP_INTERLEAVED, 6, USE_MANY)      \
-  X(6, 2, 8, MAP_INTERLEAVED, 8, USE_FEW)        \
-  X(6, 3, 16, MAP_INTERLEAVED, 6, USE_MANY)      \
-  X(7, 2, 8, MAP_INTERLEAVED, 4, USE_FEW)        \
-  X(7, 3, 8, MAP_INTERLEAVED, 6, USE_MANY)
+#define BNTT_PLAN_SHAPES(X)                                          \
+  X(1, 1, 256, MAP_CONTIG, 4, SRC_GLOBAL, USE_ALL)                   \
+  X(2, 2, 256, MAP_CONTIG, 4, SRC_GLOBAL, USE_ALL)                   \
+  X(3, 2, 32, MAP_CONTIG, 16, SRC_GLOBAL, USE_ALL)                   \
+  X(4, 2, 16, MAP_CONTIG, 16, SRC_GLOBAL, USE_ALL)                   \
+  X(5, 2, 8, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
+  X(5, 2, 8, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
+  X(5, 3, 16, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)                  \
+  X(6, 2, 4, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
+  X(6, 2, 4, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
+  X(6, 3, 8, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)                   \
+  X(7, 2, 2, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
+  X(7, 2, 2, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
+  X(7, 3, 4, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)                   \
+  X(8, 2, 1, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
+  X(8, 2, 1, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW | USE_MANY)         \
+  X(9, 2, 1, MAP_CONTIG, 4, TW_AHEAD, USE_LONE)                      \
+  X(9, 2, 1, MAP_CONTIG, 8, SRC_GLOBAL, USE_FEW)                     \
+  X(9, 3, 1, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)                   \
+  X(10, 2, 1, MAP_CONTIG, 2, TW_AHEAD, USE_LONE)                     \
+  X(10, 2, 1, MAP_CONTIG, 4, SRC_GLOBAL, USE_FEW)                    \
+  X(10, 3, 1, MAP_CONTIG, 6, SRC_GLOBAL, USE_MANY)                   \
+  X(5, 2, 16, MAP_INTERLEAVED, 8, SRC_GLOBAL, USE_LONE | USE_FEW)    \
+  X(5, 3, 32, MAP_INTERLEAVED, 6, SRC_GLOBAL, USE_MANY)              \
+  X(6, 2, 8, MAP_INTERLEAVED, 4, TW_AHEAD, USE_LONE)                 \
+  X(6, 2, 8, MAP_INTERLEAVED, 8, SRC_GLOBAL, USE_FEW)                \
+  X(6, 3, 16, MAP_INTERLEAVED, 6, SRC_GLOBAL, USE_MANY)              \
+  X(7, 2, 8, MAP_INTERLEAVED, 2, TW_AHEAD, USE_LONE)                 \
+  X(7, 2, 8, MAP_INTERLEAVED, 4, SRC_GLOBAL, USE_FEW)                \
+  X(7, 3, 8, MAP_INTERLEAVED, 6, SRC_GLOBAL, USE_MANY)
 
 #define BNTT_SUBK_FN(M, LOGR, TPC, MAP, ARITH, MINB, FN, USE)                             \
   ::bntt::SubKernel {                                                                     \

@@ -37,16 +37,16 @@ const std::vector<SubKernel>& sub_kernels() {
 
 const SubKernel* default_sub_kernel(int m, int map, int fast, uint64_t elems) {
   struct Table {
-    const SubKernel* at[11][2][2][2] = {};
+    const SubKernel* at[11][2][2][8] = {};
   };
   static const Table table = [] {
     Table t;
     for (const SubKernel& k : sub_kernels())
-      for (int many = 0; many < 2; ++many)
-        if (k.use & (many ? USE_MANY : USE_FEW)) t.at[k.m][k.map][k.fast][many] = &k;
+      for (int use : {USE_LONE, USE_FEW, USE_MANY})
+        if (k.use & use) t.at[k.m][k.map][k.fast][use] = &k;
     return t;
   }();
-  return m >= 1 && m <= 10 ? table.at[m][map][fast][elems >= kManyElems ? 1 : 0] : nullptr;
+  return m >= 1 && m <= 10 ? table.at[m][map][fast][use_of(elems)] : nullptr;
 }
 
 int blocks_per_sm(const SubKernel* k) {
