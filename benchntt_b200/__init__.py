@@ -23,6 +23,7 @@ where modulus / mu / m / x are Python ints.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import numpy as np
@@ -571,9 +572,16 @@ class Server:
 
 
 # ------------------------------------------------------------- BLAS helpers
+@functools.lru_cache(maxsize=64)
+def _modulus_arg(q: int, mu: int):
+    """The C argument for a modulus, by value: building the structure anew
+    took a third of a short vector call."""
+    return ctypes.byref(modulus(q, mu))
+
+
 def blas(ctx: Context, op: str, c, a, b, q: int, mu: int, x: int = 0,
          layout: int = LAYOUT_HILO) -> None:
-    m = modulus(q, mu)
+    m = _modulus_arg(q, mu)
     L = lib()
     if _is_cuda_tensor(a):
         n = a.numel() // 2
@@ -585,9 +593,9 @@ def blas(ctx: Context, op: str, c, a, b, q: int, mu: int, x: int = 0,
         kind = "host"
     fn = getattr(L, f"bntt_{op}_{kind}")
     if op == "axpy":
-        check(fn(ctx.handle, *ptrs, U128.of(x), n, ctypes.byref(m), layout))
+        check(fn(ctx.handle, *ptrs, U128.of(x), n, m, layout))
     else:
-        check(fn(ctx.handle, *ptrs, n, ctypes.byref(m), layout))
+        check(fn(ctx.handle, *ptrs, n, m, layout))
 
 
 def fill_uniform(seed: int, count: int, q: int, offset: int = 0) -> np.ndarray:
