@@ -25,13 +25,15 @@
 
 namespace bntt {
 
-// 128 threads, 6 resident CTAs per SM (80 registers).  The rate of a tile does
-// not change between 24 and 32 resident warps, and six small CTAs overlap more
-// of each other's item fetches, loads and barriers than four of 256 threads:
-// uneven batch 818 us with 256 threads and 4 CTAs, 804 with 128 and 6 (841
-// with 5, whose 96 registers spill less).
+// 128 threads, 7 resident CTAs per SM (72 registers; the general multiply 6 at
+// 80).  The rate of a tile does not change between 24 and 32 resident warps,
+// and small CTAs overlap more of each other's item fetches, loads and barriers
+// (818 us for the uneven batch with 4 CTAs of 256 threads, 804 with 6 of 128).
+// Uneven batch and ragged inverse batch, us, with 5, 6 and 7 CTAs: 813 and 533,
+// 793 and 520, 791 and 513.
 constexpr int kBatchThreads = 128;
-constexpr int kBatchCtas = 6;
+template <class Arith>
+constexpr int kBatchCtas = Arith::kFast ? 7 : 6;
 
 struct alignas(16) DevJob {  // two 16-byte loads
   const uint4* x;
@@ -225,7 +227,7 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const BatchArgs& ba
 // for the `layout` argument.  A constant layout removes the runtime word
 // select of every HBM load and store (measured +0.9 % on the uneven batch).
 template <class Arith, int LY>
-__global__ void __launch_bounds__(kBatchThreads, kBatchCtas) k_batch(BatchArgs ba, ModParams mp, int layout) {
+__global__ void __launch_bounds__(kBatchThreads, kBatchCtas<Arith>) k_batch(BatchArgs ba, ModParams mp, int layout) {
   extern __shared__ uint4 smem[];
   __shared__ uint32_t s_item;
   __shared__ int s_flag;

@@ -32,7 +32,7 @@ __device__ __forceinline__ void run_item_inv(const WorkItem& it, const BatchArgs
 
 // LY: the element layout as a constant, as in k_batch.
 template <int LY>
-__global__ void __launch_bounds__(kBatchThreads, kBatchCtas) k_batch_inv(BatchArgs ba, ModParams mp, int) {
+__global__ void __launch_bounds__(kBatchThreads, kBatchCtas<ArithFast>) k_batch_inv(BatchArgs ba, ModParams mp, int) {
   extern __shared__ uint4 smem[];
   __shared__ uint32_t s_item;
   __shared__ int s_flag;

@@ -82,7 +82,9 @@ struct MulB {
 //   TW_AHEAD    the entries of every pass are loaded into registers together
 //               with the input (launches that do not fill the SMs, where a
 //               table load per pass is latency nothing hides)
-enum : int { SRC_GLOBAL = 0, SRC_STAGED = 1, TW_SHARED = 2, TW_CONST = 4, TW_AHEAD = 8 };
+//   NO_LOOK     passes do not look for zeros before they run (pass_lazy): a vote
+//               per pass, 0.4 us of a lone transform
+enum : int { SRC_GLOBAL = 0, SRC_STAGED = 1, TW_SHARED = 2, TW_CONST = 4, TW_AHEAD = 8, NO_LOOK = 16 };
 
 // 16-byte asynchronous copy global -> shared (cp.async, L2 only), and the
 // group commit / wait that order them.
@@ -184,6 +186,17 @@ struct NttTile {
     else __syncthreads();
   }
 
+  // The same, and whether `flag` is set in a thread that takes part.
+  template <int A, int B>
+  __device__ __forceinline__ static bool any_between(bool flag) {
+    if constexpr (warp_exchange(A, B)) {
+      __syncwarp();
+      return __any_sync(0xFFFFFFFFu, flag);
+    } else {
+      return __syncthreads_or(flag) != 0;
+    }
+  }
+
   // Runs the whole sub-transform.  Every thread of the tile must call it
   // (it synchronises); threads whose sub-transform is not valid compute on
   // zeros and store nothing.
@@ -195,7 +208,7 @@ struct NttTile {
     if constexpr (Arith::kFast) {
       Table<SRC> tw;
       load_table<0, SRC>(tw, sr, lane);
-      pass_lazy<0, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw);
+      pass_lazy<0, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw, false);
     } else {
       pass<0>(v, sr, sub, lane, smem, mp, layout, mb);
     }
@@ -253,110 +266,181 @@ struct NttTile {
   }
   __host__ __device__ static constexpr bool rebase(int p) { return lazy_before(p) + bits(p) > kLazyStages; }
 
+  // Local index and slot of group i of pass P, and its elements before the pass.
+  template <int P>
+  __device__ __forceinline__ static int base_of(int lane, int i) {
+    constexpr int lo = low(P);
+    const int g = lane + i * TPT;
+    return (g & ((1 << lo) - 1)) | ((g >> lo) << (lo + bits(P)));
+  }
+  template <int P, int SRC>
+  __device__ __forceinline__ static U128 gather(const SubRef& sr, const uint4* smem, int layout, int base, int sb, int j) {
+    if constexpr (P == 0 && (SRC & SRC_STAGED) != 0) {
+      return from_mem(smem[slot_at(sb, j << low(P))], layout);  // staged in memory order
+    } else if constexpr (P == 0) {
+      if (!sr.valid) return U128{{0u, 0u, 0u, 0u}};
+      const uint32_t lshift = MAP == MAP_CONTIG ? 0u : sr.lshift;  // L, 0 for contiguous tiles
+      return from_mem(ld_data(sr.x + ((size_t)base << lshift) + (size_t)j * ((size_t)1 << (low(P) + lshift))), layout);
+    } else {
+      const uint4 t = smem[slot_at(sb, j << low(P))];
+      return U128{{t.x, t.y, t.z, t.w}};
+    }
+  }
+  // Element j of group i after the pass: to the next pass's slots, or to HBM
+  // (times its element of b).
+  template <int P>
+  __device__ __forceinline__ static void scatter(const SubRef& sr, uint4* smem, int layout, const MulB& mb, uint32_t k,
+                                                 int base, int sb, int j, const U128& e) {
+    if constexpr (P == NPASS - 1) {
+      if (!sr.valid) return;
+      const uint32_t lshift = MAP == MAP_CONTIG ? 0u : sr.lshift;
+      uint4* yp = sr.y + ((size_t)base << lshift) + (size_t)j * ((size_t)1 << (low(P) + lshift));
+      U128 o = e;
+      if (mb.b) {
+        const uint4 bv = mb.b[(uint64_t)(yp - mb.ybase) & mb.bmask];
+        o = reduce_once(mul_lazy(from_mem(bv, layout), o, k), k);
+      }
+      *yp = to_mem(o, layout);
+    } else {
+      smem[slot_at(sb, j << low(P))] = make_uint4(e.w[0], e.w[1], e.w[2], e.w[3]);
+    }
+  }
+
+  // The second limbs by which a pass knows a multiplicand of its first stage
+  // that may be zero: 0 in the input, all ones in what an exact pass left.
+  template <int P>
+  __device__ __forceinline__ static void see_limb(uint32_t& limb, const U128& e) {
+    limb = P == 0 ? min(limb, e.w[1]) : max(limb, e.w[1]);
+  }
+  template <int P>
+  static constexpr uint32_t kNoLimb = P == 0 ? 0xFFFFFFFFu : 0u;
+
+  // The thread's part of pass P with the reference's butterflies, from its
+  // gather to its scatter; with `look`, only if its warp holds such a
+  // multiplicand.  Returns whether it ran.  A function of its own, without
+  // register results, so that the common path carries no registers for it
+  // (inlined in every pass it cost 3 % of a plan transform and 6 % of the
+  // persistent kernel).
+  template <int P, int SRC>
+  __device__ __noinline__ static bool exact_pass(const SubRef sr, int sub, int lane, uint4* smem, uint32_t k, int layout,
+                                                 const MulB mb, bool look) {
+    constexpr int r = bits(P), G = 1 << r;
+    if (look) {
+      uint32_t limb = kNoLimb<P>;
+#pragma unroll 1
+      for (int i = 0; i < R / G; ++i) {
+        const int base = base_of<P>(lane, i), sb = slot(sub, base);
+#pragma unroll
+        for (int j = G / 2; j < G; ++j) see_limb<P>(limb, gather<P, SRC>(sr, smem, layout, base, sb, j));
+      }
+      if (!__any_sync(0xFFFFFFFFu, sr.valid && limb == ~kNoLimb<P>)) return false;
+    }
+#pragma unroll 1
+    for (int i = 0; i < R / G; ++i) {
+      const int base = base_of<P>(lane, i), sb = slot(sub, base);
+      const uint32_t gt = table_row(sr, lane, i, start(P), low(P));
+      U128 e[G];
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        e[j] = gather<P, SRC>(sr, smem, layout, base, sb, j);
+        if constexpr (P > 0) e[j] = lazy_value(e[j], k);
+      }
+      exact_stages<r>(e, [&](int t, int u) {
+        const uint4 v = (tw_at(sr.tw, gt << t))[u];  // generic: the table may be in shared memory
+        return U128{{v.x, v.y, v.z, v.w}};
+      }, k);
+#pragma unroll
+      for (int j = 0; j < G; ++j)
+        scatter<P>(sr, smem, layout, mb, k, base, sb, j, P == NPASS - 1 ? e[j] : add_8q(e[j], k));
+    }
+    return true;
+  }
+
   // One pass on partly reduced values (fast moduli).  Only the elements that
   // the first stage adds to need a base of 8q; the ones it multiplies are
   // taken as they are.
+  //
+  // A zero among the latter makes its sum the element it is added to, and
+  // small values and zeros (sparse or short-coefficient polynomials) then look
+  // like the corner cases.  A warp that finds one takes the exact pass at once
+  // instead of running the stages twice; after the first pass it looks only if
+  // a thread it exchanges with ran an exact pass (`suspect`).  16,384 x 2^10,
+  // us: spread residues 282, ternary 343, all zero 454 (434 and 846 without
+  // looking; the exact arithmetic of every stage took 433 for any values).
   template <int P, int SRC>
   __device__ __forceinline__ static void pass_lazy(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                                    uint4* smem, const ModParams& mp, int layout,
-                                                   const MulB& mb, const Table<SRC>& tw) {
+                                                   const MulB& mb, const Table<SRC>& tw, bool suspect) {
     constexpr int r = bits(P);
-    constexpr int s0 = start(P);
-    constexpr int lo = M - s0 - r;        // lowest local bit this pass touches
     constexpr int G = 1 << r;             // elements per group
     constexpr int GPT = R / G;            // groups per thread
     constexpr bool last = P == NPASS - 1;
     static_assert(GPT >= 1, "pass wider than the register tile");
     static_assert(r <= kLazyStages, "pass wider than the partly reduced range");
-    // element j of a group in HBM: the group's first element plus j * gstep
-    const uint32_t lshift = MAP == MAP_CONTIG ? 0u : sr.lshift;  // L, 0 for contiguous tiles
-    const size_t gstep = (size_t)1 << (lo + lshift);
     const uint32_t k = mp.k;
 
-    // element j of the group at local index base, slot sb
-    auto gather = [&](int base, int sb, int j) -> U128 {
-      if constexpr (P == 0 && (SRC & SRC_STAGED) != 0) {
-        return from_mem(smem[slot_at(sb, j << lo)], layout);  // staged in memory order
-      } else if constexpr (P == 0) {
-        if (!sr.valid) return U128{{0u, 0u, 0u, 0u}};
-        return from_mem(ld_data(sr.x + ((size_t)base << lshift) + (size_t)j * gstep), layout);
-      } else {
-        const uint4 t = smem[slot_at(sb, j << lo)];
-        return U128{{t.x, t.y, t.z, t.w}};
-      }
-    };
-    auto base_of = [&](int i) {
-      const int g = lane + i * TPT;
-      return (g & ((1 << lo) - 1)) | ((g >> lo) << (lo + r));
-    };
-    auto gt_of = [&](int i) { return table_row(sr, lane, i, s0, lo); };
-
-#pragma unroll
-    for (int i = 0; i < GPT; ++i) {
-      const int base = base_of(i), sb = slot(sub, base);
-#pragma unroll
-      for (int j = 0; j < G; ++j) v[i * G + j] = gather(base, sb, j);
+    bool ran = false;  // an exact pass
+    if constexpr (P > 0 && (SRC & NO_LOOK) == 0) {
+      if (__builtin_expect(suspect, 0)) ran = exact_pass<P, SRC>(sr, sub, lane, smem, k, layout, mb, true);
     }
-    bool rerun = false;
-#pragma unroll
-    for (int i = 0; i < GPT; ++i) {
-#pragma unroll
-      for (int j = 0; j < G / 2; ++j) {
-        U128& x = v[i * G + j];
-        if constexpr (P == 0) x = add_8q(x, k);
-        else if constexpr (rebase(P)) x = add_8q(fold_top(x, k), k);
-      }
-      const uint32_t gt = gt_of(i);
-      lazy_stages<r>(v, i * G, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, gt, i, t, u); }, k, rerun);
-    }
-    // the transform's outputs: below q unless the top limb says otherwise
-    if constexpr (last) {
-      if (!mb.b) {
-#pragma unroll
-        for (int j = 0; j < R; ++j) {
-          v[j] = fold_top(v[j], k);
-          rerun |= v[j].w[3] >= 0x0FFFFFFFu;
-        }
-      }
-    }
-    if (__builtin_expect(rerun && sr.valid, 0)) {
-      // the pass's inputs are still where they were gathered from
+    if (__builtin_expect(!ran, 1)) {
 #pragma unroll
       for (int i = 0; i < GPT; ++i) {
-        const int base = base_of(i), sb = slot(sub, base);
-        U128 t[G];
+        const int base = base_of<P>(lane, i), sb = slot(sub, base);
 #pragma unroll
-        for (int j = 0; j < G; ++j) t[j] = gather(base, sb, j);
-        exact_stages<r>(t, sr.tw, gt_of(i), mp, P > 0);
-#pragma unroll
-        for (int j = 0; j < G; ++j) v[i * G + j] = last ? t[j] : add_8q(t[j], k);
+        for (int j = 0; j < G; ++j) v[i * G + j] = gather<P, SRC>(sr, smem, layout, base, sb, j);
       }
-    }
-
+      bool exact = false;
+      if constexpr (P == 0 && (SRC & NO_LOOK) == 0) {
+        uint32_t limb = kNoLimb<P>;
 #pragma unroll
-    for (int i = 0; i < GPT; ++i) {
-      const int base = base_of(i), sb = slot(sub, base);
+        for (int i = 0; i < GPT; ++i)
 #pragma unroll
-      for (int j = 0; j < G; ++j) {
-        if constexpr (last) {
-          if (sr.valid) {
-            uint4* yp = sr.y + ((size_t)base << lshift) + (size_t)j * gstep;
-            U128 o = v[i * G + j];
-            if (mb.b) {
-              const uint4 bv = mb.b[(uint64_t)(yp - mb.ybase) & mb.bmask];
-              o = reduce_once(mul_lazy(from_mem(bv, layout), o, k), k);
-            }
-            *yp = to_mem(o, layout);
+          for (int j = G / 2; j < G; ++j) see_limb<P>(limb, v[i * G + j]);
+        exact = __any_sync(0xFFFFFFFFu, sr.valid && limb == ~kNoLimb<P>);
+      }
+      if (__builtin_expect(!exact, 1)) {
+        bool rerun = false;
+#pragma unroll
+        for (int i = 0; i < GPT; ++i) {
+#pragma unroll
+          for (int j = 0; j < G / 2; ++j) {
+            U128& x = v[i * G + j];
+            if constexpr (P == 0) x = add_8q(x, k);
+            else if constexpr (rebase(P)) x = add_8q(fold_top(x, k), k);
           }
-        } else {
-          const U128& e = v[i * G + j];
-          smem[slot_at(sb, j << lo)] = make_uint4(e.w[0], e.w[1], e.w[2], e.w[3]);
+          const uint32_t gt = table_row(sr, lane, i, start(P), low(P));
+          lazy_stages<r>(v, i * G, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, gt, i, t, u); }, k, rerun);
+        }
+        // the transform's outputs: below q unless the top limb says otherwise
+        if constexpr (last) {
+          if (!mb.b) {
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+              v[j] = fold_top(v[j], k);
+              rerun |= v[j].w[3] >= 0x0FFFFFFFu;
+            }
+          }
+        }
+        exact = rerun && sr.valid;
+      }
+      if (__builtin_expect(exact, 0)) {
+        // the pass's inputs are still where they were gathered from
+        ran = exact_pass<P, SRC>(sr, sub, lane, smem, k, layout, mb, false);
+      } else {
+#pragma unroll
+        for (int i = 0; i < GPT; ++i) {
+          const int base = base_of<P>(lane, i), sb = slot(sub, base);
+#pragma unroll
+          for (int j = 0; j < G; ++j) scatter<P>(sr, smem, layout, mb, k, base, sb, j, v[i * G + j]);
         }
       }
     }
     if constexpr (P + 1 < NPASS) {
-      sync_between<P, P + 1>();
-      pass_lazy<P + 1, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw);
+      bool next = false;
+      if constexpr ((SRC & NO_LOOK) != 0) sync_between<P, P + 1>();
+      else next = any_between<P, P + 1>(ran);
+      pass_lazy<P + 1, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw, next);
     }
   }
 

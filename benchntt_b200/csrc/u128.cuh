@@ -743,28 +743,22 @@ __device__ __forceinline__ void lazy_stages(U128 (&v)[R], int e0, const Tw& tw, 
   }
 }
 
-// The same stages with the reference's butterflies, on a group in memory:
-// stage t of the group reads tw[(gt << t) + u].  `carried`: the values come
-// from an earlier pass (lazy_value), else they are canonical.  The results
-// are the reference's.
-template <int r>
-__device__ __noinline__ void exact_stages(U128* v, const uint4* tw, uint32_t gt, const ModParams mp, bool carried) {
-  constexpr int G = 1 << r;
-  if (carried) {
-#pragma unroll 1
-    for (int j = 0; j < G; ++j) v[j] = lazy_value(v[j], mp.k);
-  }
-#pragma unroll 1
+// The same stages with the reference's butterflies, on exact values.
+template <int r, int R, class Tw>
+__device__ __forceinline__ void exact_stages(U128 (&v)[R], const Tw& tw, uint32_t k) {
+#pragma unroll
   for (int t = 0; t < r; ++t) {
-    const int half = G >> (t + 1);
-#pragma unroll 1
-    for (int i = 0; i < G / 2; ++i) {
-      const int u = i / half, j = (i % half) + 2 * half * u;
-      const uint4 tv = tw[(gt << t) + u];
-      U128 x = v[j], y = v[j + half];
-      butterfly<ArithFast>(x, y, U128{{tv.x, tv.y, tv.z, tv.w}}, mp);
-      v[j] = x;
-      v[j + half] = y;
+    const int half = 1 << (r - 1 - t);
+#pragma unroll
+    for (int u = 0; u < (1 << t); ++u) {
+      const U128 w = tw(t, u);
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        U128 &x = v[(u << (r - t)) | i], &y = v[((u << (r - t)) | i) + half];
+        const U128 p = reduce_once(mul_lazy(w, y, k), k);
+        y = submod_pm(x, p, 0u - k);
+        x = addmod_pm(x, p, 0u - k);
+      }
     }
   }
 }

@@ -125,3 +125,47 @@ def test_batch_matches_oracle(ctx, kind, layout):
         p.close()
     dx.free()
     dy.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["edges", "sparse", "ternary"])
+@pytest.mark.parametrize("logn", [3, 4, 5, 6, 7, 8, 9, 10, 11, 13, 16, 17])
+@pytest.mark.parametrize("elems", [1 << 17, 1 << 18, 1 << 21], ids=["lone", "few", "many"])
+def test_every_launch_size_matches_oracle(ctx, kind, logn, elems):
+    """The plan kernels of each launch size (up to 2^17 elements, below 2^21, above), with a ragged last
+    tile: a few distinct transforms repeated, so the oracle computes only those."""
+    q = C.Q_NTT
+    rows = max(1, min(7, 4096 >> logn))
+    x, t = values(kind, q, logn, rows)
+    batch = elems >> logn if elems == 1 << 17 else (elems >> logn) + 3
+    at = (np.arange(batch) % rows)[:, None] * (1 << logn) + np.arange(1 << logn)
+    plan = bn.Plan(ctx, logn, q, mu_of(q), t)
+    dx, dy = DevBuf.from_array(ctx, x[at.reshape(-1)]), DevBuf(ctx, batch * 16 << logn)
+    bn.check(bn.lib().bntt_ntt_forward_dev(plan.handle, dy.ptr, dx.ptr, batch))
+    want = C.oracle_ntt(x, t, logn, q, mu_of(q), form=1, threads=8)
+    assert np.array_equal(dy.to_array(), want[at.reshape(-1)])
+    dx.free()
+    dy.free()
+    plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("logn", [1, 2, 3, 5, 6, 7, 8, 9, 10, 11, 13, 16])
+@pytest.mark.parametrize("elems", [1 << 17, 1 << 18, 1 << 21], ids=["lone", "few", "many"])
+def test_inverse_of_every_launch_size(ctx, logn, elems):
+    """The inverse kernels of each launch size on special values, against the oracle."""
+    q = Q_NC
+    rows = max(1, min(7, 4096 >> logn))
+    y = values("ternary", q, logn, rows)[0]
+    y[y.shape[0] // 2:] = C.uniform_pairs(5, y.shape[0] - y.shape[0] // 2, q)
+    t = C.uniform_pairs(6 + logn, 1 << logn, q)
+    batch = elems >> logn if elems == 1 << 17 else (elems >> logn) + 3
+    at = (np.arange(batch) % rows)[:, None] * (1 << logn) + np.arange(1 << logn)
+    plan = bn.Plan(ctx, logn, q, mu_of(q), t)
+    dy, dx = DevBuf.from_array(ctx, y[at.reshape(-1)]), DevBuf(ctx, batch * 16 << logn)
+    bn.check(bn.lib().bntt_ntt_inverse_dev(plan.handle, dx.ptr, dy.ptr, batch))
+    want = C.oracle_ntt_inverse(y, t, logn, q, mu_of(q))
+    assert np.array_equal(dx.to_array(), want[at.reshape(-1)])
+    dx.free()
+    dy.free()
+    plan.close()
