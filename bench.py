@@ -1042,8 +1042,9 @@ def serving_bench(args, ctx) -> dict:
         return row
 
     out["rate_50k"] = replay(50_000.0)
-    out["rate_50k"]["note"] = ("one call at a time cannot sustain 50k req/s: its queue grows through the "
-                               "replay, so its latency measures the replay's length")
+    if out["rate_50k"]["one_call_at_a_time"]["throughput_req_s"] < 49_000.0:
+        out["rate_50k"]["note"] = ("one call at a time cannot sustain 50k req/s here: its queue grows through "
+                                   "the replay, so its latency measures the replay's length")
     # the rate the one-call-at-a-time path sustains: 80 % of its measured throughput
     sustainable = 0.8 * out["rate_50k"]["one_call_at_a_time"]["throughput_req_s"]
     out["rate_serial_sustainable"] = replay(round(sustainable, -2))

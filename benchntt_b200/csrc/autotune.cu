@@ -1,11 +1,11 @@
 // autotune.cu -- measured choice of kernel shapes per transform size.
 //
 // For every size the library has several compiled shapes: elements per thread
-// (radix 8 or 16 register tiles, which also sets the number of shared-memory
-// passes), transforms per CTA (CTA shape), register budgets (two or three
-// resident CTAs per SM), inputs read from HBM by the first pass or staged
-// into shared memory a tile ahead, and the twiddle table read through L1 or
-// copied into shared memory per CTA (twiddle placement).  The tuner times each candidate on this device with
+// (4, 8 or 16, which also sets the number of shared-memory passes), transforms
+// per CTA (CTA shape), register budgets (resident CTAs per SM), inputs read
+// from HBM by the first pass or staged into shared memory a tile ahead, and the
+// twiddle table read through L1 or copied into shared memory per CTA (twiddle
+// placement).  The tuner times each candidate on this device with
 // seeded data larger than L2 and makes the fastest the default for plans and
 // batches created afterwards in the process.  Choices can be written to and
 // read from a small text file (keyed by device name and SM count).

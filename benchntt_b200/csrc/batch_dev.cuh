@@ -8,8 +8,8 @@
 //           (n > 10, passes from batch_split: strided passes of 5..7 stages
 //           keep >= 8 adjacent columns; 2^16 = 6 + 10, 2^20 = 6 + 6 + 8)
 // A CTA takes the next item with an atomic counter.  Queue order is: all
-// first passes of large jobs, then small tiles from the largest size down,
-// then later passes.  Pass p > 0 of a job reads what pass p-1 wrote, so its
+// first passes of large jobs, then small tiles from the largest size down, cut
+// into one segment before each later pass group, then the smallest.  Pass p > 0 of a job reads what pass p-1 wrote, so its
 // tiles first wait until the job's pass p-1 counter reaches that pass's tile
 // count.  The wait cannot deadlock: every pass p-1 tile was handed out
 // before any pass p tile (see the loop in k_batch).  The wait is

@@ -15,8 +15,8 @@
 // whose stage S0 + s multiplies by
 //     T[((2^S0 + H) << s) + (j >> (M - s))].
 // A small transform is one sub-transform (S0 = L = 0).  Large transforms run
-// as passes over HBM: for 2^20, pass A has S0 = 0, M = 10, L = 10 (columns)
-// and pass B has S0 = 10, M = 10, L = 0 (rows).  This holds for any table T
+// as passes over HBM: for 2^16, pass A has S0 = 0, M = 6, L = 10 (columns)
+// and pass B has S0 = 6, M = 10, L = 0 (rows).  This holds for any table T
 // because it only regroups the network's data flow.
 //
 // Inside a sub-transform each thread holds R = 2^LOGR elements in registers.

@@ -629,19 +629,14 @@ struct ArithRef {
 };
 
 // One butterfly of the network: (x, y) <- (x + w*y, x - w*y) with the
-// reference's addmod / submod (src/ntt_scalar.c:586-588).
+// reference's addmod / submod (src/ntt_scalar.c:586-588).  The kernels with the
+// general multiply run it; a fast modulus takes lazy_stages below.
 template <class Arith>
 __device__ __forceinline__ void butterfly(U128& x, U128& y, const U128& w, const ModParams& m) {
   const U128 p = Arith::mul(w, y, m);
-  if constexpr (Arith::kFast) {  // q = 2^124 - k: limbs 1..3 are constants
-    const U128 s = addmod_pm(x, p, m.q.w[0]);
-    y = submod_pm(x, p, m.q.w[0]);
-    x = s;
-  } else {
-    const U128 s = addmod_ref(x, p, m.q);
-    y = submod_ref(x, p, m.q);
-    x = s;
-  }
+  const U128 s = addmod_ref(x, p, m.q);
+  y = submod_ref(x, p, m.q);
+  x = s;
 }
 
 // ---------------------------------------------------- partly reduced values
