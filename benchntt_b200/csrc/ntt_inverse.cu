@@ -62,9 +62,8 @@ const SubKernel* inverse_kernel(int m, int map, uint64_t elems) {
 // out[k] = tw[k]^-1 = tw[k]^(q-2) mod q for k >= 1, out[1] times ninv as well;
 // out[0].x becomes nonzero if an entry is not a residue above 0 or its power is
 // not its inverse.  One thread per entry: about 230 dependent products, so a
-// 2^20 table takes under a millisecond and a small one 40 us, where the host
-// took 40 ms for the former (two sequential products per entry) and two copies
-// of the table.
+// 2^20 table takes under a millisecond, where the host took 40 ms (two
+// sequential products per entry) and two copies of the table.
 __global__ void __launch_bounds__(128) k_invert_table(uint4* out, const uint4* tw, uint32_t n, U128 ninv, ModParams mp) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k == 0 || k >= n) return;
@@ -94,9 +93,9 @@ __global__ void __launch_bounds__(128) k_invert_table(uint4* out, const uint4* t
 // inverse kernel then scales only the first half of its outputs (the x outputs
 // of the last stage).
 //
-// On the host, for tables the device build does not finish (an entry without
-// an inverse, q not prime) and for its errors: one modular exponentiation and
-// three multiplies per entry (batch inversion).
+// On the host, for small tables, for those the device build does not finish (an
+// entry without an inverse, q not prime) and for their errors: one modular
+// exponentiation and three multiplies per entry (batch inversion).
 static u128 entry_of(const std::vector<uint32_t>& t, size_t k) {
   u128 v = 0;
   for (int l = 3; l >= 0; --l) v = (v << 32) | t[4 * k + l];
@@ -155,6 +154,10 @@ int ensure_inverse_host(bntt_plan* p) {
 
 int ensure_inverse(bntt_plan* p) {
   if (p->tw_inv) return BNTT_OK;
+  // below 2^10 entries the host is quicker: the device build's chain of products
+  // takes its time whatever the size (first inverse call, host and device, us:
+  // 2^4 48 and 83, 2^9 79 and 84, 2^10 109 and 86, 2^14 723 and 88)
+  if (p->log2n < 10) return ensure_inverse_host(p);
   const u128 q = to_u128(p->mod.q), mu = to_u128(p->mod.mu);
   const size_t n = (size_t)1 << p->log2n;
   const u128 ninv = host_powmod((u128)n % q, q - 2, q, mu);

@@ -169,3 +169,33 @@ def test_inverse_of_every_launch_size(ctx, logn, elems):
     dx.free()
     dy.free()
     plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("logn", [9, 10, 13])   # inverse table built on the host, on the device
+@pytest.mark.parametrize("entry", [1, 2, "last"])
+def test_tables_without_an_inverse_are_refused(logn, entry):
+    """A zero twiddle anywhere, and a composite modulus, are refused whichever
+    side builds the inverse table; entry 0, which no stage reads, may be 0."""
+    ctx = bn.Context(0)
+    n = 1 << logn
+    d = DevBuf.from_array(ctx, C.uniform_pairs(5, n, C.Q_NTT))
+    t = C.uniform_pairs(6, n, C.Q_NTT)
+    t[0] = 0
+    good = bn.Plan(ctx, logn, C.Q_NTT, C.MU_NTT, t)
+    assert bn.lib().bntt_ntt_inverse_dev(good.handle, d.ptr, d.ptr, 1) == bn.OK
+    want = C.oracle_ntt_inverse(C.uniform_pairs(5, n, C.Q_NTT), t, logn)
+    assert np.array_equal(d.to_array(), want)
+    t[n - 1 if entry == "last" else entry] = 0
+    zero = bn.Plan(ctx, logn, C.Q_NTT, C.MU_NTT, t)
+    assert bn.lib().bntt_ntt_inverse_dev(zero.handle, d.ptr, d.ptr, 1) == bn.EINVAL
+    assert b"no inverse" in bn.lib().bntt_last_error()
+    q = (1 << 124) - 721                            # a multiple of 3
+    assert q % 3 == 0
+    comp = bn.Plan(ctx, logn, q, mu_of(q), C.uniform_pairs(7, n, q))
+    assert bn.lib().bntt_ntt_inverse_dev(comp.handle, d.ptr, d.ptr, 1) == bn.EINVAL
+    assert np.array_equal(d.to_array(), want)       # nothing was written
+    for o in (good, zero, comp):
+        o.close()
+    d.free()
+    ctx.close()
