@@ -82,9 +82,7 @@ struct MulB {
 //   TW_AHEAD    the entries of every pass are loaded into registers together
 //               with the input (launches that do not fill the SMs, where a
 //               table load per pass is latency nothing hides)
-//   NO_LOOK     passes do not look for zeros before they run (pass_lazy): a vote
-//               per pass, 0.4 us of a lone transform
-enum : int { SRC_GLOBAL = 0, SRC_STAGED = 1, TW_SHARED = 2, TW_CONST = 4, TW_AHEAD = 8, NO_LOOK = 16 };
+enum : int { SRC_GLOBAL = 0, SRC_STAGED = 1, TW_SHARED = 2, TW_CONST = 4, TW_AHEAD = 8 };
 
 // 16-byte asynchronous copy global -> shared (cp.async, L2 only), and the
 // group commit / wait that order them.
@@ -208,7 +206,8 @@ struct NttTile {
     if constexpr (Arith::kFast) {
       Table<SRC> tw;
       load_table<0, SRC>(tw, sr, lane);
-      pass_lazy<0, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw, false);
+      if constexpr (Table<SRC>::kAhead) pass_ahead<0, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw, false);
+      else pass_lazy<0, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw, false);
     } else {
       pass<0>(v, sr, sub, lane, smem, mp, layout, mb);
     }
@@ -306,34 +305,68 @@ struct NttTile {
     }
   }
 
-  // The second limbs by which a pass knows a multiplicand of its first stage
-  // that may be zero: 0 in the input, all ones in what an exact pass left.
+  // 0 where the first stage's sum of x and a product of y will be flagged because
+  // both are zero, as their second limbs tell: 0 in the input, all ones in what an
+  // exact pass left.
   template <int P>
-  __device__ __forceinline__ static void see_limb(uint32_t& limb, const U128& e) {
-    limb = P == 0 ? min(limb, e.w[1]) : max(limb, e.w[1]);
+  __device__ __forceinline__ static uint32_t zero_pair(const U128& x, const U128& y) {
+    return P == 0 ? x.w[1] | y.w[1] : ~(x.w[1] & y.w[1]);
   }
+  // Whether a lane of the warp holds such a pair among its elements of pass P.
   template <int P>
-  static constexpr uint32_t kNoLimb = P == 0 ? 0xFFFFFFFFu : 0u;
+  __device__ __forceinline__ static bool warp_sees_zeros(const U128 (&v)[R], bool valid) {
+    constexpr int G = 1 << bits(P);
+    uint32_t seen = ~0u;
+#pragma unroll
+    for (int i = 0; i < R / G; ++i)
+#pragma unroll
+      for (int j = 0; j < G / 2; ++j) seen = min(seen, zero_pair<P>(v[i * G + j], v[i * G + j + G / 2]));
+    return __any_sync(0xFFFFFFFFu, valid && seen == 0u);
+  }
+
+  // All of the thread's elements before pass P.
+  template <int P, int SRC>
+  __device__ __forceinline__ static void gather_pass(U128 (&v)[R], const SubRef& sr, int sub, int lane,
+                                                     const uint4* smem, int layout) {
+    constexpr int G = 1 << bits(P);
+#pragma unroll
+    for (int i = 0; i < R / G; ++i) {
+      const int base = base_of<P>(lane, i), sb = slot(sub, base);
+#pragma unroll
+      for (int j = 0; j < G; ++j) v[i * G + j] = gather<P, SRC>(sr, smem, layout, base, sb, j);
+    }
+  }
+
+  // The reference's butterflies on the exact values e of a group, tw(t, u) as in
+  // lazy_stages; a group of zeros stays one.
+  template <int r, class Tw>
+  __device__ __forceinline__ static void exact_group(U128 (&e)[1 << r], const Tw& tw, uint32_t k) {
+    uint32_t any = 0;
+#pragma unroll
+    for (int j = 0; j < (1 << r); ++j) any |= e[j].w[0] | e[j].w[1] | e[j].w[2] | e[j].w[3];
+    if (any != 0u) exact_stages<r>(e, tw, k);
+  }
 
   // The thread's part of pass P with the reference's butterflies, from its
-  // gather to its scatter; with `look`, only if its warp holds such a
-  // multiplicand.  Returns whether it ran.  A function of its own, without
-  // register results, so that the common path carries no registers for it
-  // (inlined in every pass it cost 3 % of a plan transform and 6 % of the
-  // persistent kernel).
+  // gather to its scatter; with `look`, only if its warp holds a zero pair.
+  // Returns whether it ran.  A function of its own, without register results, so
+  // that the common path carries no registers for it (inlined in every pass it
+  // cost 3 % of a plan transform and 6 % of the persistent kernel).
   template <int P, int SRC>
   __device__ __noinline__ static bool exact_pass(const SubRef sr, int sub, int lane, uint4* smem, uint32_t k, int layout,
                                                  const MulB mb, bool look) {
     constexpr int r = bits(P), G = 1 << r;
     if (look) {
-      uint32_t limb = kNoLimb<P>;
+      uint32_t seen = ~0u;
 #pragma unroll 1
       for (int i = 0; i < R / G; ++i) {
         const int base = base_of<P>(lane, i), sb = slot(sub, base);
 #pragma unroll
-        for (int j = G / 2; j < G; ++j) see_limb<P>(limb, gather<P, SRC>(sr, smem, layout, base, sb, j));
+        for (int j = 0; j < G / 2; ++j)
+          seen = min(seen, zero_pair<P>(gather<P, SRC>(sr, smem, layout, base, sb, j),
+                                        gather<P, SRC>(sr, smem, layout, base, sb, j + G / 2)));
       }
-      if (!__any_sync(0xFFFFFFFFu, sr.valid && limb == ~kNoLimb<P>)) return false;
+      if (!__any_sync(0xFFFFFFFFu, sr.valid && seen == 0u)) return false;
     }
 #pragma unroll 1
     for (int i = 0; i < R / G; ++i) {
@@ -345,7 +378,7 @@ struct NttTile {
         e[j] = gather<P, SRC>(sr, smem, layout, base, sb, j);
         if constexpr (P > 0) e[j] = lazy_value(e[j], k);
       }
-      exact_stages<r>(e, [&](int t, int u) {
+      exact_group<r>(e, [&](int t, int u) {
         const uint4 v = (tw_at(sr.tw, gt << t))[u];  // generic: the table may be in shared memory
         return U128{{v.x, v.y, v.z, v.w}};
       }, k);
@@ -356,17 +389,51 @@ struct NttTile {
     return true;
   }
 
-  // One pass on partly reduced values (fast moduli).  Only the elements that
-  // the first stage adds to need a base of 8q; the ones it multiplies are
-  // taken as they are.
+  // The stages of pass P on partly reduced values, in registers; whether the
+  // pass has to be rerun with the reference's butterflies.  Only the elements
+  // that the first stage adds to need a base of 8q; the ones it multiplies are
+  // taken as they are.  STOP as in lazy_stages.
+  template <int P, int SRC, bool STOP>
+  __device__ __forceinline__ static bool lazy_pass(U128 (&v)[R], const SubRef& sr, int lane, uint32_t k,
+                                                   const MulB& mb, const Table<SRC>& tw) {
+    constexpr int r = bits(P), G = 1 << r;
+    bool rerun = false;
+#pragma unroll
+    for (int i = 0; i < R / G; ++i) {
+#pragma unroll
+      for (int j = 0; j < G / 2; ++j) {
+        U128& x = v[i * G + j];
+        if constexpr (P == 0) x = add_8q(x, k);
+        else if constexpr (rebase(P)) x = add_8q(fold_top(x, k), k);
+      }
+      const uint32_t gt = table_row(sr, lane, i, start(P), low(P));
+      lazy_stages<r, STOP>(v, i * G, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, gt, i, t, u); }, k, rerun,
+                           sr.valid);
+    }
+    // the transform's outputs: below q unless the top limb says otherwise
+    if constexpr (P == NPASS - 1) {
+      if (!mb.b) {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          v[j] = fold_top(v[j], k);
+          rerun |= v[j].w[3] >= 0x0FFFFFFFu;
+        }
+      }
+    }
+    return rerun && sr.valid;
+  }
+
+  // One pass of a fast modulus: lazy_pass, or the exact pass in its place.
   //
-  // A zero among the latter makes its sum the element it is added to, and
-  // small values and zeros (sparse or short-coefficient polynomials) then look
-  // like the corner cases.  A warp that finds one takes the exact pass at once
-  // instead of running the stages twice; after the first pass it looks only if
-  // a thread it exchanges with ran an exact pass (`suspect`).  16,384 x 2^10,
-  // us: spread residues 282, ternary 343, all zero 454 (434 and 846 without
-  // looking; the exact arithmetic of every stage took 433 for any values).
+  // Where x and y of a butterfly are both zero, its sum looks like the corner
+  // cases (all-zero, sparse and short-coefficient polynomials).  A warp that
+  // finds such a pair takes the exact pass at once instead of running the stages
+  // twice; after the first pass it looks only if a thread it exchanges with ran
+  // an exact pass (`suspect`).  16,384 x 2^10, us: spread residues 282, their
+  // upper half zero 283, ternary 342, 31 of 32 values zero 408, all zero 157 (334,
+  // 343, 435 and 454 for the last four kinds when any zero multiplicand called for the
+  // exact pass and zeros were multiplied; 431 for any values with the exact
+  // butterflies throughout).
   template <int P, int SRC>
   __device__ __forceinline__ static void pass_lazy(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                                    uint4* smem, const ModParams& mp, int layout,
@@ -374,13 +441,12 @@ struct NttTile {
     constexpr int r = bits(P);
     constexpr int G = 1 << r;             // elements per group
     constexpr int GPT = R / G;            // groups per thread
-    constexpr bool last = P == NPASS - 1;
     static_assert(GPT >= 1, "pass wider than the register tile");
     static_assert(r <= kLazyStages, "pass wider than the partly reduced range");
     const uint32_t k = mp.k;
 
     bool ran = false;  // an exact pass
-    if constexpr (P > 0 && (SRC & NO_LOOK) == 0) {
+    if constexpr (P > 0) {
       if (__builtin_expect(suspect, 0)) ran = exact_pass<P, SRC>(sr, sub, lane, smem, k, layout, mb, true);
     }
     if (__builtin_expect(!ran, 1)) {
@@ -391,39 +457,8 @@ struct NttTile {
         for (int j = 0; j < G; ++j) v[i * G + j] = gather<P, SRC>(sr, smem, layout, base, sb, j);
       }
       bool exact = false;
-      if constexpr (P == 0 && (SRC & NO_LOOK) == 0) {
-        uint32_t limb = kNoLimb<P>;
-#pragma unroll
-        for (int i = 0; i < GPT; ++i)
-#pragma unroll
-          for (int j = G / 2; j < G; ++j) see_limb<P>(limb, v[i * G + j]);
-        exact = __any_sync(0xFFFFFFFFu, sr.valid && limb == ~kNoLimb<P>);
-      }
-      if (__builtin_expect(!exact, 1)) {
-        bool rerun = false;
-#pragma unroll
-        for (int i = 0; i < GPT; ++i) {
-#pragma unroll
-          for (int j = 0; j < G / 2; ++j) {
-            U128& x = v[i * G + j];
-            if constexpr (P == 0) x = add_8q(x, k);
-            else if constexpr (rebase(P)) x = add_8q(fold_top(x, k), k);
-          }
-          const uint32_t gt = table_row(sr, lane, i, start(P), low(P));
-          lazy_stages<r>(v, i * G, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, gt, i, t, u); }, k, rerun);
-        }
-        // the transform's outputs: below q unless the top limb says otherwise
-        if constexpr (last) {
-          if (!mb.b) {
-#pragma unroll
-            for (int j = 0; j < R; ++j) {
-              v[j] = fold_top(v[j], k);
-              rerun |= v[j].w[3] >= 0x0FFFFFFFu;
-            }
-          }
-        }
-        exact = rerun && sr.valid;
-      }
+      if constexpr (P == 0) exact = warp_sees_zeros<P>(v, sr.valid);
+      if (__builtin_expect(!exact, 1)) exact = lazy_pass<P, SRC, false>(v, sr, lane, k, mb, tw);
       if (__builtin_expect(exact, 0)) {
         // the pass's inputs are still where they were gathered from
         ran = exact_pass<P, SRC>(sr, sub, lane, smem, k, layout, mb, false);
@@ -436,11 +471,57 @@ struct NttTile {
         }
       }
     }
+    if constexpr (P + 1 < NPASS)
+      pass_lazy<P + 1, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw, any_between<P, P + 1>(ran));
+  }
+
+  // The same for launches with TW_AHEAD, which wait for every load and have
+  // registers to spare: the exact pass is inline, on the registers that hold the
+  // table's entries.  Zeros are found where spread values do not pay for it: in
+  // the first pass by the sums of its first stage (a look at the elements costs a
+  // lone 2^10 transform 0.25 us, as the first butterflies then wait for every
+  // load), later among the elements of a warp that ran an exact pass before.  One
+  // transform of 2^10, us: spread 4.5, ternary 5.2, 31 of 32 values zero 6.4, all
+  // zero 3.5 (4.4, 5.8, 8.6 and 10.6 when each pass was run twice, out of line;
+  // 5.9 for any values with the exact butterflies throughout, which mostly zero
+  // inputs do not quite reach: up to 1.13 of that for 4,096 x 2^5).
+  template <int P, int SRC>
+  __device__ __forceinline__ static void pass_ahead(U128 (&v)[R], const SubRef& sr, int sub, int lane,
+                                                    uint4* smem, const ModParams& mp, int layout,
+                                                    const MulB& mb, const Table<SRC>& tw, bool suspect) {
+    constexpr int G = 1 << bits(P);
+    static_assert(R >= G && bits(P) <= kLazyStages, "pass shape");
+    const uint32_t k = mp.k;
+    bool zeros = false, rerun = false;
+    gather_pass<P, SRC>(v, sr, sub, lane, smem, layout);
+    if constexpr (P > 0) zeros = suspect && warp_sees_zeros<P>(v, sr.valid);
+    if (__builtin_expect(!zeros, 1)) rerun = lazy_pass<P, SRC, P == 0>(v, sr, lane, k, mb, tw);
+    const bool ran = zeros || rerun;
+    if (__builtin_expect(!ran, 1)) {
+#pragma unroll
+      for (int i = 0; i < R / G; ++i) {
+        const int base = base_of<P>(lane, i), sb = slot(sub, base);
+#pragma unroll
+        for (int j = 0; j < G; ++j) scatter<P>(sr, smem, layout, mb, k, base, sb, j, v[i * G + j]);
+      }
+    } else {
+      if (rerun) gather_pass<P, SRC>(v, sr, sub, lane, smem, layout);  // the inputs are still there
+#pragma unroll
+      for (int i = 0; i < R / G; ++i) {
+        const int base = base_of<P>(lane, i), sb = slot(sub, base);
+        U128 e[G];
+#pragma unroll
+        for (int j = 0; j < G; ++j) e[j] = P > 0 ? lazy_value(v[i * G + j], k) : v[i * G + j];
+        exact_group<bits(P)>(e, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, 0u, i, t, u); }, k);
+#pragma unroll
+        for (int j = 0; j < G; ++j)
+          scatter<P>(sr, smem, layout, mb, k, base, sb, j, P == NPASS - 1 ? e[j] : add_8q(e[j], k));
+      }
+    }
     if constexpr (P + 1 < NPASS) {
-      bool next = false;
-      if constexpr ((SRC & NO_LOOK) != 0) sync_between<P, P + 1>();
-      else next = any_between<P, P + 1>(ran);
-      pass_lazy<P + 1, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw, next);
+      const bool next = __any_sync(0xFFFFFFFFu, ran);
+      sync_between<P, P + 1>();
+      pass_ahead<P + 1, SRC>(v, sr, sub, lane, smem, mp, layout, mb, tw, next);
     }
   }
 

@@ -106,31 +106,32 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP_CONTIG, Arith>::THRE
   X(1, 1, 256, MAP_CONTIG, 4, SRC_GLOBAL, USE_ALL)                   \
   X(2, 2, 256, MAP_CONTIG, 4, SRC_GLOBAL, USE_ALL)                   \
   X(3, 2, 32, MAP_CONTIG, 16, SRC_GLOBAL, USE_ALL)                   \
-  X(4, 2, 16, MAP_CONTIG, 16, SRC_GLOBAL, USE_ALL)                   \
-  X(5, 2, 8, MAP_CONTIG, 8, TW_AHEAD | NO_LOOK, USE_LONE)            \
+  X(4, 2, 16, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                     \
+  X(4, 2, 16, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW | USE_MANY)        \
+  X(5, 2, 8, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
   X(5, 2, 8, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
   X(5, 3, 16, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)                  \
-  X(6, 2, 4, MAP_CONTIG, 8, TW_AHEAD | NO_LOOK, USE_LONE)            \
+  X(6, 2, 4, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
   X(6, 2, 4, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
   X(6, 3, 8, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)                   \
-  X(7, 2, 2, MAP_CONTIG, 8, TW_AHEAD | NO_LOOK, USE_LONE)            \
+  X(7, 2, 2, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
   X(7, 2, 2, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
   X(7, 3, 4, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)                   \
-  X(8, 2, 1, MAP_CONTIG, 8, TW_AHEAD | NO_LOOK, USE_LONE)            \
+  X(8, 2, 1, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
   X(8, 2, 1, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
   X(8, 3, 2, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)                   \
-  X(9, 2, 1, MAP_CONTIG, 4, TW_AHEAD | NO_LOOK, USE_LONE)            \
+  X(9, 2, 1, MAP_CONTIG, 4, TW_AHEAD, USE_LONE)                      \
   X(9, 2, 1, MAP_CONTIG, 8, SRC_GLOBAL, USE_FEW)                     \
   X(9, 3, 1, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)                   \
-  X(10, 2, 1, MAP_CONTIG, 2, TW_AHEAD | NO_LOOK, USE_LONE)           \
+  X(10, 2, 1, MAP_CONTIG, 2, TW_AHEAD, USE_LONE)                     \
   X(10, 2, 1, MAP_CONTIG, 4, SRC_GLOBAL, USE_FEW)                    \
   X(10, 3, 1, MAP_CONTIG, 7, SRC_GLOBAL, USE_MANY)                   \
   X(5, 2, 16, MAP_INTERLEAVED, 8, SRC_GLOBAL, USE_LONE | USE_FEW)    \
   X(5, 3, 32, MAP_INTERLEAVED, 6, SRC_GLOBAL, USE_MANY)              \
-  X(6, 2, 8, MAP_INTERLEAVED, 4, TW_AHEAD | NO_LOOK, USE_LONE)       \
+  X(6, 2, 8, MAP_INTERLEAVED, 4, TW_AHEAD, USE_LONE)                 \
   X(6, 2, 8, MAP_INTERLEAVED, 8, SRC_GLOBAL, USE_FEW)                \
   X(6, 3, 16, MAP_INTERLEAVED, 5, SRC_GLOBAL, USE_MANY)              \
-  X(7, 2, 8, MAP_INTERLEAVED, 2, TW_AHEAD | NO_LOOK, USE_LONE)       \
+  X(7, 2, 8, MAP_INTERLEAVED, 2, TW_AHEAD, USE_LONE)                 \
   X(7, 2, 8, MAP_INTERLEAVED, 4, SRC_GLOBAL, USE_FEW)                \
   X(7, 3, 8, MAP_INTERLEAVED, 6, SRC_GLOBAL, USE_MANY)
 

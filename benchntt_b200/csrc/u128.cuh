@@ -706,21 +706,27 @@ __device__ __forceinline__ U128 fold_top(const U128& a, uint32_t k) {
 }
 // the reference's value of a u that a pass left
 __device__ __forceinline__ U128 lazy_value(const U128& u, uint32_t k) {
-  const U128 zero_based = add_8q(u, k);             // u + 8q = (u - 8q) + 16q, 16q = 2^128 - 16k
-  if (u.w[1] == 0xFFFFFFFFu) {                      // left by a rerun: u - 8q
-    const U128 c{{k << 4, 0u, 0u, 0u}};
-    return add_nc(zero_based, c);
+  if (u.w[1] == 0xFFFFFFFFu) {  // left by a rerun: u - 8q = u + 2^127 + 8k (mod 2^128)
+    const U128 c{{k << 3, 0u, 0u, 0x80000000u}};
+    return add_nc(u, c);
   }
   return reduce_once(fold_top(u, k), k);
 }
 
 // The r stages of a group of 2^r registers from e0 on partly reduced values;
 // tw(t, u) is the twiddle of block u of stage t.  Sets `rerun` when a value
-// has the limb described above.
-template <int r, int R, class Tw>
-__device__ __forceinline__ void lazy_stages(U128 (&v)[R], int e0, const Tw& tw, uint32_t k, bool& rerun) {
+// has the limb described above.  STOP (every lane of the warp takes part): the
+// warp's lanes end together after the first stage, all with `rerun` set, if one
+// of those with `counts` has it set by then.
+template <int r, bool STOP = false, int R, class Tw>
+__device__ __forceinline__ void lazy_stages(U128 (&v)[R], int e0, const Tw& tw, uint32_t k, bool& rerun,
+                                            bool counts = true) {
 #pragma unroll
   for (int t = 0; t < r; ++t) {
+    if (STOP && t == 1 && __builtin_expect(__any_sync(0xFFFFFFFFu, rerun && counts), 0)) {
+      rerun = true;
+      return;
+    }
     const int half = 1 << (r - 1 - t);
 #pragma unroll
     for (int u = 0; u < (1 << t); ++u) {

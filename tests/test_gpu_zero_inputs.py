@@ -1,0 +1,126 @@
+"""Zero and mostly zero inputs: every sum of two zeros looks like one of the
+reference's corner sums to the partly reduced butterflies, so these inputs take
+the exact butterflies.  Results are compared bit for bit with the oracle, and an
+all-zero input must not take longer than a spread one.
+"""
+import numpy as np
+import pytest
+
+import benchntt_b200 as bn
+import common as C
+
+pytestmark = pytest.mark.gpu
+
+
+def mostly_zero(kind: str, logn: int, batch: int):
+    """Transforms of zeros with single values among them."""
+    rng = np.random.default_rng(77 * logn + batch)
+    n = batch << logn
+    x = np.zeros((n, 2), dtype=np.uint64)
+    if kind == "one":                     # one value in all
+        at = rng.integers(0, n, size=1)
+    elif kind == "few":                   # about one value in 32
+        at = np.flatnonzero(rng.random(n) < 1 / 32)
+    elif kind == "upper":                 # zeros in the upper half, which the first stage multiplies
+        at = np.flatnonzero((np.arange(n) >> (logn - 1)) & 1 == 0)
+    else:                                 # alternate transforms: zeros and spread values
+        at = np.flatnonzero((np.arange(n) >> logn) & 1 == 1)
+    x[at] = C.uniform_pairs(5 + logn, len(at), C.Q_NTT)
+    if kind == "few":
+        edge = C.to_pairs([0, 1, C.Q_NTT - 1])
+        x[at[::2]] = edge[rng.integers(0, 3, size=len(at[::2]))]
+    return x
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    torch = pytest.importorskip("torch")
+    stream = torch.cuda.Stream()
+    c = bn.Context(0, stream=stream.cuda_stream)
+    c.torch_stream = stream
+    yield c
+    c.close()
+
+
+# every size of the launches that hold the table in registers (2^4..2^10 and the
+# strided passes above), one tile and a ragged last tile, and larger launches
+@pytest.mark.parametrize("kind", ["one", "few", "upper", "alternate"])
+@pytest.mark.parametrize("logn,batch", [(1, 5), (2, 3), (3, 33), (4, 1), (4, 67), (5, 19), (6, 9), (7, 5), (8, 3), (9, 3),
+                                        (10, 3), (11, 3), (12, 2), (13, 2), (16, 2), (4, 9001), (6, 4099), (10, 259)])
+def test_mostly_zero_inputs_match_oracle(ctx, kind, logn, batch):
+    import torch
+    x = mostly_zero(kind, logn, batch)
+    t = C.uniform_pairs(4 + logn, 1 << logn, C.Q_NTT)
+    plan = bn.Plan(ctx, logn, C.Q_NTT, C.MU_NTT, t)
+    dx = torch.from_numpy(x.view(np.int64)).cuda()
+    dy = torch.empty_like(dx)
+    plan.forward(dy, dx, batch)
+    torch.cuda.synchronize()
+    want = C.oracle_ntt(x, t, logn, C.Q_NTT, C.MU_NTT, form=1, threads=8)
+    assert np.array_equal(dy.cpu().numpy().view(np.uint64), want)
+    plan.close()
+
+
+def microseconds(ctx, call, reps):
+    """of one call, from the fastest of ten runs of `reps` in a row"""
+    import torch
+    best = float("inf")
+    with torch.cuda.stream(ctx.torch_stream):
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(reps):
+                call()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3 / reps)
+    return best
+
+
+# The exact butterfly is 1.5 times as long as the partly reduced one (87
+# instructions, 57), and a group of zeros needs none; running both, one after the
+# other, takes 2.5 times as long.
+LIMIT = 1.4
+
+
+# (short launches from a captured graph, so that the host does not set their pace)
+@pytest.mark.parametrize("logn,batch", [(5, 4096), (7, 1024), (8, 1), (10, 1), (10, 128), (16, 1), (10, 16384), (16, 256)])
+def test_zeros_take_no_longer_than_spread_values(ctx, logn, batch):
+    import torch
+    n = batch << logn
+    plan = bn.Plan(ctx, logn, C.Q_NTT, C.MU_NTT, C.uniform_pairs(4, 1 << logn, C.Q_NTT))
+    spread = torch.from_numpy(C.uniform_pairs(3, n, C.Q_NTT).view(np.int64)).cuda()
+    y = torch.empty_like(spread)
+    times = []
+    for x in (spread, torch.zeros_like(spread)):
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=ctx.torch_stream):
+            for _ in range(20):
+                plan.forward(y, x, batch)
+        times.append(microseconds(ctx, lambda: graph.replay(), 2))
+    assert times[1] < LIMIT * times[0], times
+    plan.close()
+
+
+def test_batch_of_zeros_takes_no_longer(ctx):
+    import torch
+    logns = np.array([n for n in range(4, 11)] * 4000 + [16] * 16)
+    sizes = sorted(set(logns.tolist()))
+    plans = [bn.Plan(ctx, n, C.Q_NTT, C.MU_NTT, C.uniform_pairs(n, 1 << n, C.Q_NTT)) for n in sizes]
+    lens = np.left_shift(1, logns)
+    offs = (np.cumsum(lens) - lens) * 16
+    spread = torch.from_numpy(C.uniform_pairs(3, int(lens.sum()), C.Q_NTT).view(np.int64)).cuda()
+    y = torch.empty_like(spread)
+    engine = bn.Batch(ctx, plans)
+    times = []
+    for x in (spread, torch.zeros_like(spread)):
+        torch.cuda.synchronize()
+        jobs = bn.Batch.jobs((x.data_ptr() + offs).tolist(), (y.data_ptr() + offs).tolist(),
+                             [sizes.index(int(n)) for n in logns])
+        times.append(microseconds(ctx, lambda: engine.run_dev(jobs), 5))
+    assert engine.status() == bn.OK
+    assert times[1] < LIMIT * times[0], times
+    engine.close()
+    for p in plans:
+        p.close()
