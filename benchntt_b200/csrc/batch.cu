@@ -12,15 +12,22 @@
 
 namespace bntt {
 
-const void* batch_kernel_fast(int layout);
+const void* batch_kernel_fast(int layout, int threads);
 const void* batch_kernel_ref();
+const void* batch_kernel_inverse(int layout, int threads);
 
 // Shared memory of an item: the exchange slots of the sub-transforms the
 // threads hold at a time (NttTile::SMEM_SLOTS; one pass needs none).
-size_t shape_smem(int s) {
+static size_t shape_smem(int s, int threads) {
   const BatchShape& b = kShapes[s];
-  if (b.m <= b.logr) return 0;
-  return ((size_t)kBatchThreads << b.logr) * 16;
+  const int logr = batch_logr(b.logr, threads);
+  if (b.m <= logr) return 0;
+  return ((size_t)threads << logr) * 16;
+}
+
+static const void* batch_kernel(const bntt_batch* b, bool inverse, int threads) {
+  return inverse ? batch_kernel_inverse(b->layout, threads)
+                 : b->fast ? batch_kernel_fast(b->layout, threads) : batch_kernel_ref();
 }
 
 // Resident CTAs per SM of a batch kernel (forward or inverse) at the largest
@@ -28,7 +35,7 @@ size_t shape_smem(int s) {
 // dynamic shared memory, so no launch raises the kernel's limit: a limit set
 // for one job list (and lowered for the next) would fail launches of others
 // that share the kernel, such as the serving loop's.
-int batch_kernel_bps(const void* fn, int* bps) {
+static int batch_kernel_bps(const void* fn, int threads, int* bps) {
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, int> cache;
   int dev = 0;
@@ -40,13 +47,38 @@ int batch_kernel_bps(const void* fn, int* bps) {
     return BNTT_OK;
   }
   size_t smem = 0;
-  for (int k = 0; k < kNumShapes; ++k) smem = std::max(smem, shape_smem(k));
+  for (int k = 0; k < kNumShapes; ++k) smem = std::max(smem, shape_smem(k, threads));
   BNTT_REQUIRE(smem <= 48 * 1024, "batch tile needs %zu bytes of shared memory", smem);
   int b = 0;
-  BNTT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kBatchThreads, smem));
+  BNTT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, smem));
   if (b < 1) return set_error(BNTT_ECUDA, "batch kernel does not fit on an SM (smem %zu)", smem);
   cache[{fn, dev}] = b;
   *bps = b;
+  return BNTT_OK;
+}
+
+// 256 threads for a list that the long lists' kernel would hold in one wave, and
+// with the general multiply (batch_dev.cuh).
+int batch_launch(const bntt_batch* b, const std::vector<WorkItem>& items, bool inverse, BatchLaunch* out) {
+  *out = BatchLaunch{};
+  if (items.empty()) return BNTT_OK;
+  const bool wave = items.size() <= (size_t)batch_ctas(kBatchThreads) * b->ctx->sms;
+  out->threads = b->fast && !wave ? kBatchThreads : kShortThreads;
+  out->fn = batch_kernel(b, inverse, out->threads);
+  int bps = 0;
+  if (int rc = batch_kernel_bps(out->fn, out->threads, &bps)) return rc;
+  bool used[kNumShapes] = {};
+  for (const WorkItem& w : items) used[w.shape] = true;
+  for (int s = 0; s < kNumShapes; ++s)
+    if (used[s]) out->smem = std::max(out->smem, shape_smem(s, out->threads));
+  out->grid = (unsigned)std::min<size_t>((size_t)bps * b->ctx->sms, items.size());
+  return BNTT_OK;
+}
+
+int batch_launch_prepare(const bntt_batch* b) {
+  int bps = 0;
+  for (int threads : {kBatchThreads, kShortThreads})
+    if (int rc = batch_kernel_bps(batch_kernel(b, false, threads), threads, &bps)) return rc;
   return BNTT_OK;
 }
 
@@ -99,10 +131,6 @@ void free_schedule(bntt_ctx* c, Schedule& s) {
   if (s.d_ctl) ctx_free(c, s.d_ctl);
   s.d_ctl = nullptr;
   s.d_ctl_cap = 0;
-}
-
-const void* batch_kernel(bool fast, int layout) {
-  return fast ? batch_kernel_fast(layout) : batch_kernel_ref();
 }
 
 constexpr int kMaxLog2n = 24;  // plans hold 2^1..2^24 points
@@ -435,18 +463,8 @@ static int upload(bntt_batch* b, Schedule& sc, cudaStream_t stream, bool inverse
   sc.stream = stream;
   sc.inverse = inverse;
   sc.sticky_err = sticky_err;
-  sc.grid = 0;
-  if (sc.items.empty()) return BNTT_OK;
-  const void* fn = inverse ? batch_kernel_inverse(b->layout) : batch_kernel(b->fast, b->layout);
-  size_t smem = 0;
-  bool used[kNumShapes] = {};
-  for (const WorkItem& w : sc.items) used[w.shape] = true;
-  for (int s = 0; s < kNumShapes; ++s)
-    if (used[s]) smem = std::max(smem, shape_smem(s));
-  int bps = 0;
-  if (int rc = batch_kernel_bps(fn, &bps)) return rc;
-  sc.grid = (int)std::min<size_t>((size_t)bps * c->sms, sc.items.size());
-  sc.smem = smem;
+  if (int rc = batch_launch(b, sc.items, inverse, &sc.run)) return rc;
+  if (sc.run.grid == 0) return BNTT_OK;
   BatchArgs& ba = sc.args;
   ba.items = reinterpret_cast<const WorkItem*>(d + o_ib);
   ba.nitems = (uint32_t)sc.items.size();
@@ -468,17 +486,16 @@ static cudaError_t enqueue_run(bntt_batch* b, Schedule& sc, cudaStream_t stream)
     if (e == cudaSuccess && cb > 8) e = cudaMemsetAsync(static_cast<char*>(sc.d_ctl) + 8, 0, cb - 8, stream);
   }
   if (e != cudaSuccess) return e;
-  const void* fn = sc.inverse ? batch_kernel_inverse(b->layout) : batch_kernel(b->fast, b->layout);
   BatchArgs ba = sc.args;
   ModParams mp = b->mp;
   int layout = b->layout;
   void* args[] = {&ba, &mp, &layout};
-  return cudaLaunchKernel(fn, dim3(sc.grid), dim3(kBatchThreads), args, sc.smem, stream);
+  return cudaLaunchKernel(sc.run.fn, dim3(sc.run.grid), dim3(sc.run.threads), args, sc.run.smem, stream);
 }
 
 // Captures the schedule's launch into a graph for later replays.
 static int capture(bntt_batch* b, Schedule& sc) {
-  if (sc.exec || sc.grid == 0) return BNTT_OK;
+  if (sc.exec || sc.run.grid == 0) return BNTT_OK;
   cudaGraph_t graph = nullptr;
   BNTT_CK(cudaStreamBeginCapture(sc.stream, cudaStreamCaptureModeThreadLocal));
   const cudaError_t e1 = enqueue_run(b, sc, sc.stream);
@@ -499,7 +516,7 @@ static int capture(bntt_batch* b, Schedule& sc) {
 
 // A replay of the captured graph, or the launch itself when there is none.
 static int launch_schedule(bntt_batch* b, Schedule& sc, cudaStream_t stream) {
-  if (sc.grid == 0) return BNTT_OK;
+  if (sc.run.grid == 0) return BNTT_OK;
   if (sc.exec) {
     BNTT_CK(cudaGraphLaunch(sc.exec, stream));
   } else {
@@ -961,15 +978,8 @@ extern "C" int bntt_batch_run_dev_noalloc(bntt_batch* b, const bntt_job* jobs, s
   if (ib) BNTT_CK(cudaMemcpyAsync(s + o_it, sc.items.data(), ib, cudaMemcpyHostToDevice, st));
   if (jb) BNTT_CK(cudaMemcpyAsync(s + o_jb, sc.djobs.data(), jb, cudaMemcpyHostToDevice, st));
   if (sc.items.empty()) return BNTT_OK;
-  const void* fn = batch_kernel(b->fast, b->layout);
-  size_t smem = 0;
-  bool used[kNumShapes] = {};
-  for (const WorkItem& w : sc.items) used[w.shape] = true;
-  for (int k = 0; k < kNumShapes; ++k)
-    if (used[k]) smem = std::max(smem, shape_smem(k));
-  int bps = 0;
-  if (int rc = batch_kernel_bps(fn, &bps)) return rc;
-  const unsigned grid = (unsigned)std::min<size_t>((size_t)bps * c->sms, sc.items.size());
+  BatchLaunch run;
+  if (int rc = batch_launch(b, sc.items, false, &run)) return rc;
   BatchArgs ba;
   ba.items = reinterpret_cast<const WorkItem*>(s + o_it);
   ba.nitems = (uint32_t)sc.items.size();
@@ -980,7 +990,7 @@ extern "C" int bntt_batch_run_dev_noalloc(bntt_batch* b, const bntt_job* jobs, s
   ModParams mp = b->mp;
   int layout = b->layout;
   void* args[] = {&ba, &mp, &layout};
-  BNTT_CK(cudaLaunchKernel(fn, dim3(grid), dim3(kBatchThreads), args, smem, st));
+  BNTT_CK(cudaLaunchKernel(run.fn, dim3(run.grid), dim3(run.threads), args, run.smem, st));
   c->launches++;
   b->last_launches = 1;
   return BNTT_OK;

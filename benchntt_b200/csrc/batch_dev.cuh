@@ -1,7 +1,7 @@
 // batch_dev.cuh -- device side of the batch engine: many independent transforms of uneven sizes in one persistent,
 // graph-launched work-queue kernel.
 //
-// Work items (16 bytes each) are tiles of kBatchThreads threads:
+// Work items (16 bytes each) are tiles:
 //   SMALL   TPC transforms of one size 2^n <= 1024, consecutive in the
 //           size-sorted job descriptors (one sub-transform per job)
 //   PASS p  TPC sub-transforms of HBM pass p of one large transform
@@ -25,15 +25,28 @@
 
 namespace bntt {
 
-// 128 threads, 7 resident CTAs per SM (72 registers; the general multiply 6 at
-// 80).  The rate of a tile does not change between 24 and 32 resident warps,
-// and small CTAs overlap more of each other's item fetches, loads and barriers
-// (818 us for the uneven batch with 4 CTAs of 256 threads, 804 with 6 of 128).
-// Uneven batch and ragged inverse batch, us, with 5, 6 and 7 CTAs: 813 and 533,
-// 793 and 520, 791 and 513.
-constexpr int kBatchThreads = 128;
-template <class Arith>
-constexpr int kBatchCtas = Arith::kFast ? 7 : 6;
+// Threads and resident CTAs per SM of the kernels.
+//
+// Long lists of a fast modulus: 128 threads, 7 CTAs (72 registers).  The rate of
+// a tile does not change between 24 and 32 resident warps, and small CTAs overlap
+// more of each other's item fetches, loads and barriers (818 us for the uneven
+// batch with 4 CTAs of 256 threads, 804 with 6 of 128).  Uneven batch and ragged
+// inverse batch, us, with 5, 6 and 7 CTAs: 813 and 533, 793 and 520, 791 and 513.
+//
+// Short lists: 256 threads, 4 CTAs (64 registers), 4 elements per thread
+// throughout.  Their tiles do not fill the SMs, so a tile's own time counts, and
+// with twice the threads it is shorter.  Lists of tiles, us, 128 and 256 threads:
+// 1 x 2^10 12.0 and 10.3, 1,036 x 2^10 28.7 and 26.8, 8 x 2^16 43.1 and 28.7, 143
+// of each of 2^4..2^10 16.3 and 12.3; but 8,288 x 2^10 166 and 170, 4 x 2^20 168
+// and 190.  Short is what the long lists' kernel would hold in one wave
+// (batch_launch): 1,500 x 2^10 are 37.0 and 37.5.
+//
+// The general multiply always takes 256 threads: 4,000 of each of 2^4..2^10 292
+// us, with 128 (6 CTAs of 80 registers) 336.
+constexpr int kBatchThreads = 128, kShortThreads = 256;
+constexpr int batch_ctas(int threads) { return threads == kBatchThreads ? 7 : 4; }
+// log2 of the elements per thread of a tile whose shape has 2^logr of them
+constexpr int batch_logr(int logr, int threads) { return threads == kBatchThreads || logr < 2 ? logr : 2; }
 
 struct alignas(16) DevJob {  // two 16-byte loads
   const uint4* x;
@@ -73,8 +86,9 @@ struct WorkItem {
 static_assert(sizeof(WorkItem) == 16, "work item layout");
 
 // Tile shapes of the persistent kernel: X(id, M, LOGR, TPC, map), TPC
-// sub-transforms per item, of which the CTA's threads hold kBatchThreads >>
-// (M - LOGR) at a time (4-element shapes take two turns).  Interleaved
+// sub-transforms per item, of which 128 threads hold 128 >> (M - LOGR) at a time
+// (4-element shapes take two turns); 256 threads hold all of them, 4 elements
+// each (batch_logr).  Interleaved
 // (strided) tiles keep at least 8 adjacent columns (128 bytes of each row).
 // 8 elements per thread run three stages per exchange, with about a fifth
 // fewer index and exchange instructions, but twice the code: the strided
@@ -205,13 +219,13 @@ __device__ __forceinline__ void item_publish(const WorkItem& it, const BatchArgs
 // kernel: as separate functions the items spilled around the call's fixed
 // registers (848 -> 826 us for the uneven batch).  L2-coherent loads: a later
 // pass reads what other CTAs wrote in this launch.
-template <int M, int LOGR, int TPC, int MAP, class Arith, int LY>
+template <int M, int LOGR, int TPC, int MAP, class Arith, int LY, int THREADS>
 __device__ __forceinline__ void run_item(const WorkItem& it, const BatchArgs& ba, uint4* smem,
                                       const ModParams& mp, int layout_arg, int* s_flag) {
   const int layout = LY >= 0 ? LY : layout_arg;
-  constexpr int HELD = kBatchThreads >> (M - LOGR);  // sub-transforms the threads hold at a time
+  constexpr int HELD = THREADS >> (M - LOGR);  // sub-transforms the threads hold at a time
   using T = NttTile<M, LOGR, HELD, MAP, Arith>;
-  static_assert(T::THREADS == kBatchThreads && TPC % HELD == 0, "tile shape");
+  static_assert(T::THREADS == THREADS && TPC % HELD == 0, "tile shape");
   if (!item_wait<false>(it, ba, s_flag)) return;
 #pragma unroll 1
   for (int turn = 0; turn < TPC / HELD; ++turn) {
@@ -226,22 +240,17 @@ __device__ __forceinline__ void run_item(const WorkItem& it, const BatchArgs& ba
 // LY: the element layout as a constant (LAYOUT_HILO or LAYOUT_U128), or -1
 // for the `layout` argument.  A constant layout removes the runtime word
 // select of every HBM load and store (measured +0.9 % on the uneven batch).
-template <class Arith, int LY>
-__global__ void __launch_bounds__(kBatchThreads, kBatchCtas<Arith>) k_batch(BatchArgs ba, ModParams mp, int layout) {
+template <class Arith, int LY, int THREADS>
+__global__ void __launch_bounds__(THREADS, batch_ctas(THREADS)) k_batch(BatchArgs ba, ModParams mp, int layout) {
   extern __shared__ uint4 smem[];
   __shared__ uint32_t s_item;
   __shared__ int s_flag;
-  // Thread 0 holds one item more than the CTA runs, so the counter's round
-  // trip overlaps the current item.  A held item waits at most for the
-  // current one, whose waits are for items earlier in the queue: the earliest
-  // unfinished item is always running and has nothing to wait for.
-  uint32_t next = 0;
-  if (threadIdx.x == 0) next = atomicAdd(&ba.ctl[0], 1u);
+  // (The next item is not taken while this one runs: with few items per CTA the
+  // early CTAs then hold what late ones could run -- 296 x 2^10 22.3 instead of
+  // 14.4 us, one 2^20 91 instead of 55 -- and long lists gain nothing, the uneven
+  // batch 789 instead of 784.)
   for (;;) {
-    if (threadIdx.x == 0) {
-      s_item = next;
-      next = atomicAdd(&ba.ctl[0], 1u);
-    }
+    if (threadIdx.x == 0) s_item = atomicAdd(&ba.ctl[0], 1u);
     __syncthreads();
     const uint32_t i = s_item;
     if (i >= ba.nitems) break;
@@ -249,7 +258,7 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtas<Arith>) k_batch(Batc
     switch (it.shape) {
 #define BNTT_RUN_SHAPE(id, M, LOGR, TPC, MAP)                                   \
   case id:                                                                      \
-    run_item<M, LOGR, TPC, MAP, Arith, LY>(it, ba, smem, mp, layout, &s_flag);  \
+    run_item<M, batch_logr(LOGR, THREADS), TPC, MAP, Arith, LY, THREADS>(it, ba, smem, mp, layout, &s_flag);  \
     break;
       BNTT_BATCH_SHAPES(BNTT_RUN_SHAPE)
 #undef BNTT_RUN_SHAPE

@@ -12,6 +12,14 @@ struct ShapeChoice {
   int pass_contig[11];
 };
 
+// The kernel that runs a list of work items, and its launch.
+struct BatchLaunch {
+  const void* fn = nullptr;
+  unsigned grid = 0;
+  int threads = 0;
+  size_t smem = 0;
+};
+
 // One job list turned into work items, with its device copies and graph.
 struct Schedule {
   std::vector<DevJob> djobs;  // small jobs by size (largest first), then the large jobs by slot
@@ -63,8 +71,7 @@ struct Schedule {
   bool inverse = false;               // k_batch_inv instead of k_batch
   bool sticky_err = false;            // launches leave the error word alone
   BatchArgs args{};
-  int grid = 0;
-  size_t smem = 0;
+  BatchLaunch run;  // grid 0: nothing to launch
 };
 
 }  // namespace bntt
@@ -107,11 +114,10 @@ namespace bntt {
 // device buffer of at least `bytes` (headroom: a quarter more when it grows)
 int grow(bntt_ctx* c, void** p, size_t* cap, size_t bytes, bool headroom = false);
 void free_schedule(bntt_ctx* c, Schedule& s);
-const void* batch_kernel(bool fast, int layout);
-const void* batch_kernel_inverse(int layout);
-// resident CTAs per SM of a batch kernel (cached per device)
-int batch_kernel_bps(const void* fn, int* bps);
-size_t shape_smem(int s);
+// the launch for a list of work items
+int batch_launch(const bntt_batch* b, const std::vector<WorkItem>& items, bool inverse, BatchLaunch* out);
+// what batch_launch asks the device, asked once ahead of the first launch
+int batch_launch_prepare(const bntt_batch* b);
 // inverse = true: the jobs' inverse transforms (plans' inverse tables, the
 // passes of a large job queued last to first)
 int build_schedule(const bntt_batch* b, Schedule& sc, const bntt_job* jobs, size_t count,

@@ -12,12 +12,12 @@ namespace bntt {
 
 namespace {
 
-template <int M, int LOGR, int TPC, int MAP, int LY>
+template <int M, int LOGR, int TPC, int MAP, int LY, int THREADS>
 __device__ __forceinline__ void run_item_inv(const WorkItem& it, const BatchArgs& ba, uint4* smem,
                                           const ModParams& mp, int* s_flag) {
-  constexpr int HELD = kBatchThreads >> (M - LOGR);
+  constexpr int HELD = THREADS >> (M - LOGR);
   using T = NttTile<M, LOGR, HELD, MAP, ArithFast>;
-  static_assert(T::THREADS == kBatchThreads && TPC % HELD == 0, "tile shape");
+  static_assert(T::THREADS == THREADS && TPC % HELD == 0, "tile shape");
   if (!item_wait<true>(it, ba, s_flag)) return;
   const bool finishes = it.kind == ITEM_SMALL || it.pass == 0;
 #pragma unroll 1
@@ -31,18 +31,13 @@ __device__ __forceinline__ void run_item_inv(const WorkItem& it, const BatchArgs
 }
 
 // LY: the element layout as a constant, as in k_batch.
-template <int LY>
-__global__ void __launch_bounds__(kBatchThreads, kBatchCtas<ArithFast>) k_batch_inv(BatchArgs ba, ModParams mp, int) {
+template <int LY, int THREADS>
+__global__ void __launch_bounds__(THREADS, batch_ctas(THREADS)) k_batch_inv(BatchArgs ba, ModParams mp, int) {
   extern __shared__ uint4 smem[];
   __shared__ uint32_t s_item;
   __shared__ int s_flag;
-  uint32_t next = 0;  // one item ahead, as in k_batch
-  if (threadIdx.x == 0) next = atomicAdd(&ba.ctl[0], 1u);
   for (;;) {
-    if (threadIdx.x == 0) {
-      s_item = next;
-      next = atomicAdd(&ba.ctl[0], 1u);
-    }
+    if (threadIdx.x == 0) s_item = atomicAdd(&ba.ctl[0], 1u);
     __syncthreads();
     const uint32_t i = s_item;
     if (i >= ba.nitems) break;
@@ -50,7 +45,7 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtas<ArithFast>) k_batch_
     switch (it.shape) {
 #define BNTT_RUN_SHAPE(id, M, LOGR, TPC, MAP)                     \
   case id:                                                        \
-    run_item_inv<M, LOGR, TPC, MAP, LY>(it, ba, smem, mp, &s_flag); \
+    run_item_inv<M, batch_logr(LOGR, THREADS), TPC, MAP, LY, THREADS>(it, ba, smem, mp, &s_flag); \
     break;
       BNTT_BATCH_SHAPES(BNTT_RUN_SHAPE)
 #undef BNTT_RUN_SHAPE
@@ -60,10 +55,16 @@ __global__ void __launch_bounds__(kBatchThreads, kBatchCtas<ArithFast>) k_batch_
   }
 }
 
+template <int THREADS>
+const void* kernel_of(int layout) {
+  return layout == LAYOUT_HILO ? (const void*)&k_batch_inv<LAYOUT_HILO, THREADS>
+                               : (const void*)&k_batch_inv<LAYOUT_U128, THREADS>;
+}
+
 }  // namespace
 
-const void* batch_kernel_inverse(int layout) {
-  return layout == LAYOUT_HILO ? (const void*)&k_batch_inv<LAYOUT_HILO> : (const void*)&k_batch_inv<LAYOUT_U128>;
+const void* batch_kernel_inverse(int layout, int threads) {
+  return threads == kBatchThreads ? kernel_of<kBatchThreads>(layout) : kernel_of<kShortThreads>(layout);
 }
 
 }  // namespace bntt

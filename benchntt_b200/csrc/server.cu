@@ -140,7 +140,6 @@ struct bntt_server {
   std::atomic<bool> stop{false};
   std::atomic<uint64_t> submitted{0}, completed{0}, launches{0}, admission_waits{0};
   int worker_error = BNTT_OK;
-  int batch_bps = 0;  // resident batch-kernel CTAs per SM
 
   double now() const {
     return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -187,12 +186,8 @@ static int launch_slot(bntt_server* s, Slot& slot) {
     memcpy(h + o_jb, sc.djobs.data(), jb);
     char* d = static_cast<char*>(slot.dev);
     BNTT_CK(cudaMemcpyAsync(d, h, need, cudaMemcpyHostToDevice, slot.stream));
-    const void* fn = batch_kernel(s->engine->fast, s->engine->layout);
-    size_t smem = 0;
-    for (const WorkItem& w : sc.items) smem = std::max(smem, shape_smem(w.shape));
-    // occupancy queried once at creation
-    const unsigned grid =
-        (unsigned)std::max<size_t>(1, std::min<size_t>((size_t)s->batch_bps * c->sms, sc.items.size()));
+    BatchLaunch run;  // what it asks the device is known since the server was created
+    if (int rc = batch_launch(s->engine, sc.items, false, &run)) return rc;
     BatchArgs ba;
     ba.items = reinterpret_cast<const WorkItem*>(d + o_it);
     ba.nitems = (uint32_t)sc.items.size();
@@ -203,7 +198,7 @@ static int launch_slot(bntt_server* s, Slot& slot) {
     ModParams mp = s->engine->mp;
     int layout = s->engine->layout;
     void* args[] = {&ba, &mp, &layout};
-    BNTT_CK(cudaLaunchKernel(fn, dim3(grid), dim3(kBatchThreads), args, smem, slot.stream));
+    BNTT_CK(cudaLaunchKernel(run.fn, dim3(run.grid), dim3(run.threads), args, run.smem, slot.stream));
     c->launches++;
   }
   for (const PendingReq& p : slot.reqs) {
@@ -325,7 +320,7 @@ int bntt_server_create(bntt_ctx* c, bntt_server** out, bntt_plan* const* plans, 
     return rc;
   }
   s->arena.init(static_cast<char*>(s->arena_mem), s->cfg.hbm_budget);
-  if ((rc = batch_kernel_bps(batch_kernel(s->engine->fast, s->engine->layout), &s->batch_bps))) {
+  if ((rc = batch_launch_prepare(s->engine))) {
     ctx_free(c, s->arena_mem);
     bntt_batch_destroy(s->engine);
     delete s;
