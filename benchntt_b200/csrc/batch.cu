@@ -12,9 +12,15 @@
 
 namespace bntt {
 
-const void* batch_kernel_fast(int layout, int threads);
 const void* batch_kernel_ref();
-const void* batch_kernel_inverse(int layout, int threads);
+template <> const void* batch_kernel_fast<0>();
+template <> const void* batch_kernel_fast<1>();
+template <> const void* batch_kernel_fast<2>();
+template <> const void* batch_kernel_fast<3>();
+template <> const void* batch_kernel_inverse<0>();
+template <> const void* batch_kernel_inverse<1>();
+template <> const void* batch_kernel_inverse<2>();
+template <> const void* batch_kernel_inverse<3>();
 
 // Shared memory of an item: the exchange slots of the sub-transforms the
 // threads hold at a time (NttTile::SMEM_SLOTS; one pass needs none).
@@ -26,8 +32,13 @@ static size_t shape_smem(int s, int threads) {
 }
 
 static const void* batch_kernel(const bntt_batch* b, bool inverse, int threads) {
-  return inverse ? batch_kernel_inverse(b->layout, threads)
-                 : b->fast ? batch_kernel_fast(b->layout, threads) : batch_kernel_ref();
+  if (!inverse && !b->fast) return batch_kernel_ref();
+  switch (batch_part(b->layout, threads)) {
+    case 0: return inverse ? batch_kernel_inverse<0>() : batch_kernel_fast<0>();
+    case 1: return inverse ? batch_kernel_inverse<1>() : batch_kernel_fast<1>();
+    case 2: return inverse ? batch_kernel_inverse<2>() : batch_kernel_fast<2>();
+    default: return inverse ? batch_kernel_inverse<3>() : batch_kernel_fast<3>();
+  }
 }
 
 // Resident CTAs per SM of a batch kernel (forward or inverse) at the largest

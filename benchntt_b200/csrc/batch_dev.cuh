@@ -48,6 +48,20 @@ constexpr int batch_ctas(int threads) { return threads == kBatchThreads ? 7 : 4;
 // log2 of the elements per thread of a tile whose shape has 2^logr of them
 constexpr int batch_logr(int logr, int threads) { return threads == kBatchThreads || logr < 2 ? logr : 2; }
 
+// Object files of the fast kernels, forward and inverse: one layout and one number
+// of threads each, so that a program loads what it runs (ntt_kernels.cuh; the
+// first batch of a process took 12.4 ms forward and 6.1 to 8.2 inverse with all
+// four in one module, 3.5 to 4.8 and 1.1 to 3.7 now).
+constexpr int batch_part(int layout, int threads) {
+  return (layout == LAYOUT_HILO ? 0 : 1) + (threads == kBatchThreads ? 0 : 2);
+}
+constexpr int part_layout(int part) { return part & 1 ? LAYOUT_U128 : LAYOUT_HILO; }
+constexpr int part_threads(int part) { return part < 2 ? kBatchThreads : kShortThreads; }
+template <int PART>
+const void* batch_kernel_fast();
+template <int PART>
+const void* batch_kernel_inverse();
+
 struct alignas(16) DevJob {  // two 16-byte loads
   const uint4* x;
   uint4* y;

@@ -5,7 +5,8 @@
 // to the first, and whatever finishes a transform -- a small tile, or pass 0
 // of a large job -- multiplies by N^-1 as it stores, read from entry 0 of the
 // job's inverse table (no stage uses that entry).
-// Fast moduli only, like the plans' inverse.
+// Fast moduli only, like the plans' inverse.  Compiled once per part (BNTT_PART,
+// batch_part).
 #include "batch_dev.cuh"
 
 namespace bntt {
@@ -55,16 +56,11 @@ __global__ void __launch_bounds__(THREADS, batch_ctas(THREADS)) k_batch_inv(Batc
   }
 }
 
-template <int THREADS>
-const void* kernel_of(int layout) {
-  return layout == LAYOUT_HILO ? (const void*)&k_batch_inv<LAYOUT_HILO, THREADS>
-                               : (const void*)&k_batch_inv<LAYOUT_U128, THREADS>;
-}
-
 }  // namespace
 
-const void* batch_kernel_inverse(int layout, int threads) {
-  return threads == kBatchThreads ? kernel_of<kBatchThreads>(layout) : kernel_of<kShortThreads>(layout);
+template <>
+const void* batch_kernel_inverse<BNTT_PART>() {
+  return (const void*)&k_batch_inv<part_layout(BNTT_PART), part_threads(BNTT_PART)>;
 }
 
 }  // namespace bntt

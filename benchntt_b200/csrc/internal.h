@@ -84,6 +84,11 @@ constexpr uint64_t kManyElems = 1ull << 21;
 constexpr uint64_t kLoneElems = 1ull << 17;
 inline int use_of(uint64_t elems) { return elems <= kLoneElems ? USE_LONE : elems < kManyElems ? USE_FEW : USE_MANY; }
 
+// The object files that the plans' kernels are in (ntt_kernels.cuh): the fast
+// defaults, forward and inverse, and those with the general multiply.
+#define BNTT_PLAN_PARTS(P) P(0) P(1) P(2) P(3) P(4) P(5) P(6)
+#define BNTT_REF_PARTS(P) P(0) P(1) P(2) P(3) P(4)
+
 const std::vector<SubKernel>& sub_kernels();
 // Default shape of a pass of m stages over `elems` elements; nullptr if none
 // is compiled.

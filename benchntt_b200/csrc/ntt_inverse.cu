@@ -15,7 +15,7 @@
 // no such code); results are canonical residues in [0, q).  The fast
 // pseudo-Mersenne multiply is required (q = 2^124 - k, k < 2^28).
 //
-// Kernels: the compile-time tile in inverse mode (k_ntt_tile_inv), one
+// Kernels: the compile-time tile in inverse mode (k_ntt_tile_inv, ntt_inst_inverse.cu), one
 // launch for N up to 2^10 and above that one launch per HBM pass of the
 // persistent kernel's split (tile_split), in reverse pass order (the pass
 // over the low index bits first).
@@ -24,36 +24,22 @@
 #include "ntt_kernels.cuh"
 
 namespace bntt {
-namespace {
 
-// One HBM pass of the inverse on the compile-time tile (NttTile::run_inv), one
-// CTA per tile, in the shapes of the forward transform (BNTT_PLAN_SHAPES):
-// whole transforms of up to 2^10 points (contiguous), or one pass of a larger
-// transform (interleaved for the strided passes).  `finishing` marks the
-// pass that ends the transform (stage 0 inside it), which applies N^-1 from
-// entry 0 of the inverse table.
-template <int M, int LOGR, int TPC, int MAP, int MINB, int SRC>
-__global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP, ArithFast>::THREADS, MINB)
-    k_ntt_tile_inv(SubGeom g, ModParams mp, int layout, int finishing) {
-  using T = NttTile<M, LOGR, TPC, MAP, ArithFast>;
-  extern __shared__ uint4 smem[];
-  const int sub = T::sub_of(threadIdx.x), lane = T::lane_of(threadIdx.x);
-  const uint4* scale_at = finishing ? g.tw : nullptr;
-  stream_wait();
-  const uint64_t sid = (uint64_t)blockIdx.x * TPC + (uint64_t)sub;
-  const SubRef sr = MAP == MAP_CONTIG ? make_subref_contig<M>(g, sid) : make_subref(g, sid);
-  if (layout == LAYOUT_HILO) T::template run_inv<SRC>(sr, sub, lane, smem, mp, LAYOUT_HILO, scale_at);
-  else T::template run_inv<SRC>(sr, sub, lane, smem, mp, LAYOUT_U128, scale_at);
-}
+#define BNTT_DECLARE(p) void append_inverse_##p(std::vector<SubKernel>& v);  // ntt_inst_inverse.cu
+BNTT_PLAN_PARTS(BNTT_DECLARE)
+#undef BNTT_DECLARE
+
+namespace {
 
 // The shape for a pass of m stages over `elems` elements.
 const SubKernel* inverse_kernel(int m, int map, uint64_t elems) {
-  static const SubKernel kernels[] = {
-#define BNTT_ADD(M, LOGR, TPC, MAP, MINB, SRC, USE) \
-  BNTT_SUBK_FN(M, LOGR, TPC, MAP, ArithFast, MINB, (k_ntt_tile_inv<M, LOGR, TPC, MAP, MINB, SRC>), USE),
-      BNTT_PLAN_SHAPES(BNTT_ADD)
+  static const std::vector<SubKernel> kernels = [] {
+    std::vector<SubKernel> v;
+#define BNTT_ADD(p) append_inverse_##p(v);
+    BNTT_PLAN_PARTS(BNTT_ADD)
 #undef BNTT_ADD
-  };
+    return v;
+  }();
   for (const SubKernel& k : kernels)
     if (k.m == m && k.map == map && (k.use & use_of(elems))) return &k;
   return nullptr;

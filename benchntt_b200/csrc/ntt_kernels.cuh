@@ -102,37 +102,49 @@ __global__ void __launch_bounds__(NttTile<M, LOGR, TPC, MAP_CONTIG, Arith>::THRE
 // 128 threads: with one CTA per tile, smaller ones keep an SM's warps in more
 // different phases (2^24 elements of 2^8: 256 threads 250 us, 64 threads 234).
 // Interleaved tiles keep at least 8 columns (128 bytes of a row).
-#define BNTT_PLAN_SHAPES(X)                                          \
-  X(1, 1, 256, MAP_CONTIG, 4, SRC_GLOBAL, USE_ALL)                   \
-  X(2, 2, 256, MAP_CONTIG, 4, SRC_GLOBAL, USE_ALL)                   \
-  X(3, 2, 32, MAP_CONTIG, 16, SRC_GLOBAL, USE_ALL)                   \
-  X(4, 2, 16, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                     \
-  X(4, 2, 16, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW | USE_MANY)        \
-  X(5, 2, 8, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
-  X(5, 2, 8, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
-  X(5, 3, 16, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)                  \
-  X(6, 2, 4, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
-  X(6, 2, 4, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
-  X(6, 3, 8, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)                   \
-  X(7, 2, 2, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
-  X(7, 2, 2, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
-  X(7, 3, 4, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)                   \
-  X(8, 2, 1, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
-  X(8, 2, 1, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                    \
-  X(8, 3, 2, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)                   \
-  X(9, 2, 1, MAP_CONTIG, 4, TW_AHEAD, USE_LONE)                      \
-  X(9, 2, 1, MAP_CONTIG, 8, SRC_GLOBAL, USE_FEW)                     \
-  X(9, 3, 1, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)                   \
-  X(10, 2, 1, MAP_CONTIG, 2, TW_AHEAD, USE_LONE)                     \
-  X(10, 2, 1, MAP_CONTIG, 4, SRC_GLOBAL, USE_FEW)                    \
-  X(10, 3, 1, MAP_CONTIG, 7, SRC_GLOBAL, USE_MANY)                   \
-  X(5, 2, 16, MAP_INTERLEAVED, 8, SRC_GLOBAL, USE_LONE | USE_FEW)    \
-  X(5, 3, 32, MAP_INTERLEAVED, 6, SRC_GLOBAL, USE_MANY)              \
-  X(6, 2, 8, MAP_INTERLEAVED, 4, TW_AHEAD, USE_LONE)                 \
-  X(6, 2, 8, MAP_INTERLEAVED, 8, SRC_GLOBAL, USE_FEW)                \
-  X(6, 3, 16, MAP_INTERLEAVED, 5, SRC_GLOBAL, USE_MANY)              \
-  X(7, 2, 8, MAP_INTERLEAVED, 2, TW_AHEAD, USE_LONE)                 \
-  X(7, 2, 8, MAP_INTERLEAVED, 4, SRC_GLOBAL, USE_FEW)                \
+//
+// In parts, one object file each (forward and inverse): an object file's module is
+// loaded by the first launch of one of its kernels, and that takes the longer the
+// more kernels and line tables it holds.  First transform of a process, all shapes
+// in one module and in parts, ms: one 2^10 forward 14.3 and 1.3, inverse 4.0 and
+// 0.7; 64 x 2^16 forward 13.7 and 3.2.  Three to eight kernels to a part.
+#define BNTT_PLAN_SHAPES_0(X)                                         \
+  X(1, 1, 256, MAP_CONTIG, 4, SRC_GLOBAL, USE_ALL)                    \
+  X(2, 2, 256, MAP_CONTIG, 4, SRC_GLOBAL, USE_ALL)                    \
+  X(3, 2, 32, MAP_CONTIG, 16, SRC_GLOBAL, USE_ALL)                    \
+  X(4, 2, 16, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                      \
+  X(4, 2, 16, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW | USE_MANY)
+#define BNTT_PLAN_SHAPES_1(X)                                         \
+  X(5, 2, 8, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                       \
+  X(5, 2, 8, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                     \
+  X(5, 3, 16, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)                   \
+  X(6, 2, 4, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                       \
+  X(6, 2, 4, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                     \
+  X(6, 3, 8, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)
+#define BNTT_PLAN_SHAPES_2(X)                                         \
+  X(7, 2, 2, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                       \
+  X(7, 2, 2, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                     \
+  X(7, 3, 4, MAP_CONTIG, 12, SRC_GLOBAL, USE_MANY)
+#define BNTT_PLAN_SHAPES_3(X)                                         \
+  X(8, 2, 1, MAP_CONTIG, 8, TW_AHEAD, USE_LONE)                       \
+  X(8, 2, 1, MAP_CONTIG, 16, SRC_GLOBAL, USE_FEW)                     \
+  X(8, 3, 2, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)
+#define BNTT_PLAN_SHAPES_4(X)                                         \
+  X(9, 2, 1, MAP_CONTIG, 4, TW_AHEAD, USE_LONE)                       \
+  X(9, 2, 1, MAP_CONTIG, 8, SRC_GLOBAL, USE_FEW)                      \
+  X(9, 3, 1, MAP_CONTIG, 10, SRC_GLOBAL, USE_MANY)
+#define BNTT_PLAN_SHAPES_5(X)                                         \
+  X(10, 2, 1, MAP_CONTIG, 2, TW_AHEAD, USE_LONE)                      \
+  X(10, 2, 1, MAP_CONTIG, 4, SRC_GLOBAL, USE_FEW)                     \
+  X(10, 3, 1, MAP_CONTIG, 7, SRC_GLOBAL, USE_MANY)
+#define BNTT_PLAN_SHAPES_6(X)                                         \
+  X(5, 2, 16, MAP_INTERLEAVED, 8, SRC_GLOBAL, USE_LONE | USE_FEW)     \
+  X(5, 3, 32, MAP_INTERLEAVED, 6, SRC_GLOBAL, USE_MANY)               \
+  X(6, 2, 8, MAP_INTERLEAVED, 4, TW_AHEAD, USE_LONE)                  \
+  X(6, 2, 8, MAP_INTERLEAVED, 8, SRC_GLOBAL, USE_FEW)                 \
+  X(6, 3, 16, MAP_INTERLEAVED, 5, SRC_GLOBAL, USE_MANY)               \
+  X(7, 2, 8, MAP_INTERLEAVED, 2, TW_AHEAD, USE_LONE)                  \
+  X(7, 2, 8, MAP_INTERLEAVED, 4, SRC_GLOBAL, USE_FEW)                 \
   X(7, 3, 8, MAP_INTERLEAVED, 6, SRC_GLOBAL, USE_MANY)
 
 #define BNTT_SUBK_FN(M, LOGR, TPC, MAP, ARITH, MINB, FN, USE)                             \

@@ -8,11 +8,15 @@
 
 namespace bntt {
 
-void append_fast_plan(std::vector<SubKernel>& v);
+#define BNTT_DECLARE(p) void append_fast_plan_##p(std::vector<SubKernel>& v);
+BNTT_PLAN_PARTS(BNTT_DECLARE)
+#undef BNTT_DECLARE
+#define BNTT_DECLARE(p) void append_ref_##p(std::vector<SubKernel>& v);
+BNTT_REF_PARTS(BNTT_DECLARE)
+#undef BNTT_DECLARE
 void append_fast_contig(std::vector<SubKernel>& v);
 void append_fast_contig_r4(std::vector<SubKernel>& v);
 void append_fast_il(std::vector<SubKernel>& v);
-void append_ref(std::vector<SubKernel>& v);
 void append_fast_occ(std::vector<SubKernel>& v);
 void append_fast_small(std::vector<SubKernel>& v);
 void append_fast_staged(std::vector<SubKernel>& v);
@@ -24,12 +28,16 @@ const std::vector<SubKernel>& sub_kernels() {
     append_fast_contig(r);
     append_fast_contig_r4(r);
     append_fast_il(r);
-    append_ref(r);
+#define BNTT_ADD(p) append_ref_##p(r);
+    BNTT_REF_PARTS(BNTT_ADD)
+#undef BNTT_ADD
     append_fast_occ(r);
     append_fast_small(r);
     append_fast_staged(r);
     append_fast_occ5(r);
-    append_fast_plan(r);
+#define BNTT_ADD(p) append_fast_plan_##p(r);
+    BNTT_PLAN_PARTS(BNTT_ADD)
+#undef BNTT_ADD
     return r;
   }();
   return v;
