@@ -54,6 +54,14 @@ static std::string device_key(bntt_ctx* c) {
   return buf;
 }
 
+// Shapes that files of earlier versions may name: strided passes of 8 to 10 stages,
+// which no transform has any more.
+static bool former_shape(int m, int map, int fast, int logr, int tpc, int minb, int src) {
+  if (map != MAP_INTERLEAVED || logr != 4 || src != 0) return false;
+  if (minb == 3) return m == 9 && tpc == 4 && fast == 1;
+  return minb == 1 && ((m == 8 && tpc == 8) || ((m == 9 || m == 10) && (tpc == 4 || (tpc == 8 && fast == 1))));
+}
+
 // time one kernel over a geometry: median of `reps` launches; with `flush`
 // (a buffer larger than L2) the L2 is overwritten before each timed launch,
 // so inputs that would fit in it come from HBM as in a first use
@@ -92,7 +100,7 @@ using namespace bntt;
 extern "C" {
 
 // Measures every compiled shape for transform sizes 2^1..2^10 (contiguous
-// tiles and, for 2^5..2^10, the strided first HBM pass of large transforms),
+// tiles) and for the strided HBM passes of 5 to 7 stages of larger transforms,
 // and the persistent kernel's tile shape per size; installs the fastest as
 // defaults.  If `path` is non-NULL the choices are also written there.
 // Contiguous shapes are timed on batches of 65,536 transforms (at most 2^24
@@ -120,7 +128,7 @@ int bntt_autotune(bntt_ctx* c, const char* path) {
   std::string report = "bntt-autotune 1 " + device_key(c) + "\n";
   for (int m = 1; m <= 10 && !rc; ++m) {
     for (int map = 0; map < 2 && !rc; ++map) {
-      if (map == MAP_INTERLEAVED && m < 5) continue;
+      if (map == MAP_INTERLEAVED && (m < 5 || m > 7)) continue;
       for (int fast = 0; fast < 2 && !rc; ++fast) {
         const SubKernel* best = nullptr;
         float best_ms = 1e30f;
@@ -140,10 +148,9 @@ int bntt_autotune(bntt_ctx* c, const char* path) {
             g.l = (uint32_t)m;
           }
           g.m = (uint32_t)m;
-          g.nsub = elems >> m;
+          g.nsub = tuner_elems(m, map) >> m;
           float ms = 0;
           if (map == MAP_CONTIG) {
-            g.nsub = std::min<uint64_t>(g.nsub, 65536);
             rc = time_sub(c, &k, g, mp, 5, &ms, flush, elems * 16);
           } else {
             rc = time_sub(c, &k, g, mp, 5, &ms);
@@ -244,7 +251,7 @@ int bntt_autotune_load(bntt_ctx* c, const char* path) {
           g_sub_choice[m][map][fast] = &k;
           found = true;
         }
-      if (!found)
+      if (!found && !former_shape(m, map, fast, logr, tpc, minb, src))
         rc = set_error(BNTT_EINVAL, "%s names a kernel shape this library does not have: %s", path, line);
     } else if (sscanf(line, "batch %d %d %d", &m, &logr, &tpc) == 3) {
       for (int s = 0; s < batch_shape_count(); ++s) {

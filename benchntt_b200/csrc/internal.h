@@ -105,6 +105,11 @@ int launch_overlapped(bntt_ctx* ctx, const void* fn, unsigned grid, unsigned thr
 
 // Autotuner choices (nullptr / -1 when not tuned).
 const SubKernel* tuned_sub_kernel(int m, int map, int fast, int l);
+// Elements of the launches that the tuner times a shape on.
+inline uint64_t tuner_elems(int m, int map) {
+  const uint64_t most = 1ull << 24;  // 256 MiB: larger than L2
+  return map == 0 /* contiguous */ && m <= 8 ? 65536ull << m : most;
+}
 int tuned_batch_small_shape(int m);
 
 // HBM passes of a 2^n transform (11 <= n <= 24), as the persistent kernel
@@ -159,7 +164,7 @@ struct bntt_plan {
   void* tw_inv = nullptr;
   std::vector<int> passes;                   // stages of each HBM pass
   bool created_fast = false;                 // arithmetic chosen when the plan was created
-  const bntt::SubKernel* tuned = nullptr;    // one pass: the autotuner's shape, if it ran
+  std::vector<const bntt::SubKernel*> tuned;  // of each pass: the autotuner's shape, or nullptr
 };
 
 namespace bntt {

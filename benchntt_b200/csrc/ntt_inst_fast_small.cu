@@ -15,6 +15,6 @@ void append_fast_small(std::vector<SubKernel>& v) {
   v.push_back(BNTT_SUBK_B(7, 2, 8, MAP_CONTIG, A, 4));
   v.push_back(BNTT_SUBK_B(8, 2, 4, MAP_CONTIG, A, 4));
   v.push_back(BNTT_SUBK_B(9, 2, 2, MAP_CONTIG, A, 4));
-  v.push_back(BNTT_SUBK_B(10, 2, 1, MAP_CONTIG, A, 4));
+  // (that of 2^10 is a default shape)
 }
 }  // namespace bntt

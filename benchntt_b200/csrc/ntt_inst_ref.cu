@@ -42,9 +42,6 @@ void append(std::vector<SubKernel>& v) {
     v.push_back(BNTT_SUBK(5, 4, 8, MAP_INTERLEAVED, A));
     v.push_back(BNTT_SUBK(6, 4, 8, MAP_INTERLEAVED, A));
     v.push_back(BNTT_SUBK(7, 4, 8, MAP_INTERLEAVED, A));
-    v.push_back(BNTT_SUBK(8, 4, 8, MAP_INTERLEAVED, A));
-    v.push_back(BNTT_SUBK(9, 4, 4, MAP_INTERLEAVED, A));
-    v.push_back(BNTT_SUBK(10, 4, 4, MAP_INTERLEAVED, A));
   }
 }
 }  // namespace

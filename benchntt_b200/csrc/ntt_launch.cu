@@ -116,7 +116,17 @@ int plan_choose_kernels(bntt_plan* p) {
   const int n = (int)p->log2n;
   p->passes = n <= 10 ? std::vector<int>{n} : tile_split(n);
   p->created_fast = arith_fast(p->ctx, p->fast);
-  if (n <= 10) p->tuned = tuned_sub_kernel(n, MAP_CONTIG, p->created_fast ? 1 : 0, 0);
+  p->tuned.clear();
+  int s0 = 0;
+  for (int m : p->passes) {
+    const int l = n - s0 - m;
+    const SubKernel* k = tuned_sub_kernel(m, l > 0 ? MAP_INTERLEAVED : MAP_CONTIG, p->created_fast ? 1 : 0, l);
+    // a table copied into shared memory holds entries below 2^m only: whole
+    // transforms
+    if (k && (k->src & TW_SHARED) && s0 != 0) k = nullptr;
+    p->tuned.push_back(k);
+    s0 += m;
+  }
   return BNTT_OK;
 }
 
@@ -135,7 +145,9 @@ int ntt_forward_on(bntt_plan* plan, void* y, const void* x, size_t batch, cudaSt
   for (size_t i = 0; i < plan->passes.size(); ++i) {
     const int m = plan->passes[i];
     const int map = n - s0 - m > 0 ? MAP_INTERLEAVED : MAP_CONTIG;
-    const SubKernel* k = plan->tuned ? plan->tuned : default_sub_kernel(m, map, fast ? 1 : 0, (uint64_t)batch << n);
+    const uint64_t elems = (uint64_t)batch << n;
+    const SubKernel* k = plan->tuned[i];
+    if (!k || k->fast != (fast ? 1 : 0)) k = default_sub_kernel(m, map, fast ? 1 : 0, elems);
     if (!k) return set_error(BNTT_EINVAL, "no kernel compiled for pass m=%d map=%d", m, map);
     SubGeom g;
     g.x = static_cast<const uint4*>(i == 0 ? x : y);

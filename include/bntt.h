@@ -410,7 +410,7 @@ int bntt_server_replay_ex(bntt_server *srv, const bntt_request *reqs, size_t n, 
  * passes, transforms per CTA, two to four resident CTAs per SM, inputs read
  * by the first pass or staged into shared memory a tile ahead, twiddles read
  * through L1 or from a copy of the table in shared memory), the strided
- * first pass of large transforms, and the persistent kernel's tile shape per
+ * passes of large transforms, and the persistent kernel's tile shape per
  * size, on this device; the fastest become the defaults of plans and batches
  * created afterwards in this process.  Writes the choices to `path` if it is
  * not NULL.  Contiguous shapes are timed on 65,536 transforms (at most 2^24
