@@ -7,7 +7,8 @@
 // twiddle table read through L1 or copied into shared memory per CTA (twiddle
 // placement).  The tuner times each candidate on this device with
 // seeded data larger than L2 and makes the fastest the default for plans and
-// batches created afterwards in the process.  Choices can be written to and
+// batches created afterwards in the process, in launches that are not much smaller
+// (tuned_from).  Choices can be written to and
 // read from a small text file (keyed by device name and SM count).
 #include <algorithm>
 #include <cstdio>

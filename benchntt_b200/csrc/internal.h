@@ -110,6 +110,15 @@ inline uint64_t tuner_elems(int m, int map) {
   const uint64_t most = 1ull << 24;  // 256 MiB: larger than L2
   return map == 0 /* contiguous */ && m <= 8 ? 65536ull << m : most;
 }
+// Smallest launch that takes the tuner's shape: the tuner times launches that fill
+// the device, and what is fastest there keeps a smaller one waiting.  Default and
+// tuned shape, us: one transform of 2^8 2.7 and 4.5, 4,100 of 2^7 9.4 and 12.8, 600
+// of 2^10 15.8 and 20.1, 9 of 2^16 21.6 and 30.6; at 2^20 elements, 8,192 of 2^7
+// 15.1 and 15.9, 1,024 of 2^10 21.2 and 21.6, 16 of 2^16 34.4 and 34.9.
+inline uint64_t tuned_from(int m, int map) {
+  const uint64_t timed = tuner_elems(m, map);
+  return timed < 1ull << 20 ? timed : 1ull << 20;
+}
 int tuned_batch_small_shape(int m);
 
 // HBM passes of a 2^n transform (11 <= n <= 24), as the persistent kernel

@@ -147,7 +147,7 @@ int ntt_forward_on(bntt_plan* plan, void* y, const void* x, size_t batch, cudaSt
     const int map = n - s0 - m > 0 ? MAP_INTERLEAVED : MAP_CONTIG;
     const uint64_t elems = (uint64_t)batch << n;
     const SubKernel* k = plan->tuned[i];
-    if (!k || k->fast != (fast ? 1 : 0)) k = default_sub_kernel(m, map, fast ? 1 : 0, elems);
+    if (!k || k->fast != (fast ? 1 : 0) || elems < tuned_from(m, map)) k = default_sub_kernel(m, map, fast ? 1 : 0, elems);
     if (!k) return set_error(BNTT_EINVAL, "no kernel compiled for pass m=%d map=%d", m, map);
     SubGeom g;
     g.x = static_cast<const uint4*>(i == 0 ? x : y);

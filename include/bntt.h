@@ -412,7 +412,8 @@ int bntt_server_replay_ex(bntt_server *srv, const bntt_request *reqs, size_t n, 
  * through L1 or from a copy of the table in shared memory), the strided
  * passes of large transforms, and the persistent kernel's tile shape per
  * size, on this device; the fastest become the defaults of plans and batches
- * created afterwards in this process.  Writes the choices to `path` if it is
+ * created afterwards in this process, for launches of at least 2^20 elements (or
+ * as many as they are timed on, where that is less).  Writes the choices to `path` if it is
  * not NULL.  Contiguous shapes are timed on 65,536 transforms (at most 2^24
  * elements) with the L2 flushed before each launch.  A few seconds; about
  * 1 GiB of device memory while it runs.

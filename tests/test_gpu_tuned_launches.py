@@ -1,5 +1,7 @@
-"""Launches take the autotuner's choices, for whole transforms and for the strided
-passes of large ones."""
+"""Which launches take the autotuner's choices: those that are not much smaller
+than the launches it times, for whole transforms and for the strided passes of
+large ones.  A small launch keeps its own default.
+"""
 import numpy as np
 import pytest
 
@@ -78,6 +80,14 @@ def pair(ctx, force, logn, q, batch, *lines):
     return times
 
 
+# The same kernel in both cases, or one that the tuner would not choose here: one
+# transform of 2^8 with the shape of large launches takes 1.6 times as long.
+@pytest.mark.parametrize("logn,line", [(8, "sub 8 0 1 3 2 10 0"), (10, "sub 10 0 1 3 1 7 0"), (9, "sub 9 0 1 3 4 3 0")])
+def test_one_transform_keeps_its_shape(ctx, force, logn, line):
+    plain, tuned = pair(ctx, force, logn, C.Q_NTT, 1, line)
+    assert tuned < 1.2 * plain, (plain, tuned)
+
+
 # 16 elements per thread and one resident CTA with the general multiply: slower than
 # the default by more than a tenth, which shows that the choice is taken
 def test_large_launches_take_the_strided_choice(ctx, force):
@@ -112,6 +122,27 @@ def test_strided_choices_match_oracle(ctx, force, m, fast, logr, tpc, minb):
     torch.cuda.synchronize()
     want = C.oracle_ntt(x, t, logn, q, mu, form=1, threads=8)
     assert np.array_equal(dy.cpu().numpy().view(np.uint64), want[at])
+    plan.close()
+
+
+@pytest.mark.parametrize("src", [1, 3])
+@pytest.mark.parametrize("layout", [bn.LAYOUT_HILO, bn.LAYOUT_U128])
+def test_staged_kernels_with_a_fused_product(ctx, force, src, layout):
+    """The staged kernels in a launch that takes them, with the pointwise product of
+    the last pass, in both layouts."""
+    import torch
+    force(f"sub 7 0 1 2 8 4 {src}")
+    logn, n, rows, batch = 7, 128, 3, (1 << 13) + 3
+    order = (lambda a: a) if layout == bn.LAYOUT_HILO else (lambda a: np.ascontiguousarray(a[:, ::-1]))
+    x, b, t = (C.uniform_pairs(seed, count, C.Q_NTT) for seed, count in ((51, rows * n), (52, rows * n), (53, n)))
+    at = ((np.arange(batch) % rows)[:, None] * n + np.arange(n)).reshape(-1)
+    plan = bn.Plan(ctx, logn, C.Q_NTT, C.MU_NTT, order(t), layout)
+    dx, db = (torch.from_numpy(order(a)[at].view(np.int64)).cuda() for a in (x, b))
+    dy = torch.empty_like(dx)
+    plan.forward_mul(dy, dx, db, True, batch)
+    torch.cuda.synchronize()
+    want = C.oracle_blas("vvmul", C.oracle_ntt(x, t, logn, threads=8), b, C.Q_NTT, C.MU_NTT)
+    assert np.array_equal(dy.cpu().numpy().view(np.uint64), order(want)[at])
     plan.close()
 
 
