@@ -574,14 +574,15 @@ class Server:
 # ------------------------------------------------------------- BLAS helpers
 @functools.lru_cache(maxsize=64)
 def _modulus_arg(q: int, mu: int):
-    """The C argument for a modulus, by value: building the structure anew
-    took a third of a short vector call."""
+    """The C argument for a modulus, by value (plain integers only, so that what
+    is taken does not depend on earlier calls): building the structure anew took a
+    third of a short vector call."""
     return ctypes.byref(modulus(q, mu))
 
 
 def blas(ctx: Context, op: str, c, a, b, q: int, mu: int, x: int = 0,
          layout: int = LAYOUT_HILO) -> None:
-    m = _modulus_arg(q, mu)
+    m = _modulus_arg(q, mu) if type(q) is int and type(mu) is int else ctypes.byref(modulus(q, mu))
     L = lib()
     if _is_cuda_tensor(a):
         n = a.numel() // 2
