@@ -138,6 +138,10 @@ class ClockSampler:
 
 
 # ---------------------------------------------------------------- CPU side
+class NoReference(Exception):
+    """The reference's CPU code cannot be run here."""
+
+
 def ref_cpu():
     """oracle/ref_cpu.py: the reference's own CPU code (built into
     oracle/_ref from the benchNTT sources), timed on this host.  It never
@@ -167,6 +171,8 @@ def cpu_uneven(logns, steps: int, warmup: int, full_steps: int) -> dict:
     chosen in the warm-up."""
     R = ref_cpu()
     from benchntt_b200 import workloads as W
+    if R.best_impl() is None:
+        raise NoReference("oracle/_ref is not built: the benchNTT sources were not there (make -C oracle ref)")
     topo = R.host_topology()
     rb = R.RefNttBatch(logns, Q_NTT, MU_NTT, W.SEED_TWIDDLE_BASE, W.SEED_INPUT)
     trial = {th: rb.run("ntt_only", th) for th in R.thread_choices(topo)}
@@ -1067,7 +1073,10 @@ def run_reference(args, dist: Dist):
     if dist.rank != 0:
         return None
     batch = W.uneven_batch()
-    cpu = cpu_uneven(batch.logns, args.steps, args.warmup, max(1, min(args.steps, 10)))
+    try:
+        cpu = cpu_uneven(batch.logns, args.steps, args.warmup, max(1, min(args.steps, 10)))
+    except NoReference as why:
+        return {"impl": "reference", "unavailable": str(why)}
     value = cpu["value"]
     return {
         "impl": "reference", "metric": METRIC, "value": value, "unit": UNIT,
@@ -1119,12 +1128,41 @@ def summary(res: dict) -> dict:
                                      r(v["continuous_batching"]["service_p99_ms"], 3),
                                      r(v["one_call_at_a_time"]["service_p99_ms"], 3)]
     cb = res.get("cpu_baseline")
-    if cb:
+    if cb and "value" in cb:
         out["cpu"] = {"ntt_only": round(cb["value"]), "full_sequence": round(cb["full_sequence"]["value"]),
                       "threads": cb["threads"], "physical_cores": cb["physical_cores"], "smt": cb["smt"],
                       "gpu_over_cpu": r(res["value"] / cb["value"]),
                       "e2e_over_cpu": r(res["e2e"]["value"] / cb["value"], 2) if "e2e" in res else None}
     return out
+
+
+def add_cpu_rows(res: dict) -> None:
+    """The reference's CPU figures beside those of the GPU."""
+    from benchntt_b200 import workloads as W
+    cpu = cpu_uneven(W.uneven_batch().logns, steps=3, warmup=1, full_steps=2)
+    res["cpu_baseline"] = cpu
+    res["gpu_over_cpu"] = res["value"] / cpu["value"]
+    res["gpu_over_cpu_full_sequence"] = res["value"] / cpu["full_sequence"]["value"]
+    res["e2e_over_cpu"] = res["e2e"]["value"] / cpu["value"]
+    res["e2e_over_cpu_full_sequence"] = res["e2e"]["value"] / cpu["full_sequence"]["value"]
+    ex = cpu_extras(cpu["threads"])
+    for n, row in ex["uniform"].items():
+        u = res.get("uniform", {}).get(n)
+        if u:
+            u["cpu_reference_ntt_per_s"] = row["ntt_per_s"]
+            u["cpu_sample_transforms"] = row["sample_transforms"]
+            u["gpu_over_cpu"] = u["ntt_per_s"] / row["ntt_per_s"]
+    one = res.get("single_ntt_1024")
+    if one:   # one core per transform, as the reference programs run
+        one["cpu_reference_us_per_transform"] = ex["single_ntt_1024_us"]
+    for op, row in ex["blas"].items():
+        b = res.get("blas", {}).get(op)
+        if isinstance(row, dict) and b:
+            b["cpu_reference_gbs"] = row["gbs"]
+            b["gpu_over_cpu"] = b["gbs"] / row["gbs"]
+    if "blas" in res:
+        res["blas"]["cpu_reference"] = {"impl": ex["blas"]["impl"], "threads": cpu["threads"],
+                                        "physical_cores": cpu["physical_cores"], "smt": cpu["smt"]}
 
 
 def main():
@@ -1145,31 +1183,10 @@ def main():
             return
         res, ctx = run_ours(args, dist)
         if dist.rank == 0 and dist.world == 1 and not args.no_cpu and not args.headline_only:
-            from benchntt_b200 import workloads as W
-            cpu = cpu_uneven(W.uneven_batch().logns, steps=3, warmup=1, full_steps=2)
-            res["cpu_baseline"] = cpu
-            res["gpu_over_cpu"] = res["value"] / cpu["value"]
-            res["gpu_over_cpu_full_sequence"] = res["value"] / cpu["full_sequence"]["value"]
-            res["e2e_over_cpu"] = res["e2e"]["value"] / cpu["value"]
-            res["e2e_over_cpu_full_sequence"] = res["e2e"]["value"] / cpu["full_sequence"]["value"]
-            ex = cpu_extras(cpu["threads"])
-            for n, row in ex["uniform"].items():
-                u = res.get("uniform", {}).get(n)
-                if u:
-                    u["cpu_reference_ntt_per_s"] = row["ntt_per_s"]
-                    u["cpu_sample_transforms"] = row["sample_transforms"]
-                    u["gpu_over_cpu"] = u["ntt_per_s"] / row["ntt_per_s"]
-            one = res.get("single_ntt_1024")
-            if one:   # one core per transform, as the reference programs run
-                one["cpu_reference_us_per_transform"] = ex["single_ntt_1024_us"]
-            for op, row in ex["blas"].items():
-                b = res.get("blas", {}).get(op)
-                if isinstance(row, dict) and b:
-                    b["cpu_reference_gbs"] = row["gbs"]
-                    b["gpu_over_cpu"] = b["gbs"] / row["gbs"]
-            if "blas" in res:
-                res["blas"]["cpu_reference"] = {"impl": ex["blas"]["impl"], "threads": cpu["threads"],
-                                                "physical_cores": cpu["physical_cores"], "smt": cpu["smt"]}
+            try:
+                add_cpu_rows(res)
+            except NoReference as why:   # the GPU's figures stand without it
+                res["cpu_baseline"] = {"unavailable": str(why)}
         if dist.rank == 0:
             res["summary"] = summary(res)
             print(json.dumps(res), flush=True)
