@@ -337,16 +337,6 @@ struct NttTile {
     }
   }
 
-  // The reference's butterflies on the exact values e of a group, tw(t, u) as in
-  // lazy_stages; a group of zeros stays one.
-  template <int r, class Tw>
-  __device__ __forceinline__ static void exact_group(U128 (&e)[1 << r], const Tw& tw, uint32_t k) {
-    uint32_t any = 0;
-#pragma unroll
-    for (int j = 0; j < (1 << r); ++j) any |= e[j].w[0] | e[j].w[1] | e[j].w[2] | e[j].w[3];
-    if (any != 0u) exact_stages<r>(e, tw, k);
-  }
-
   // The thread's part of pass P with the reference's butterflies, from its
   // gather to its scatter; with `look`, only if its warp holds a zero pair.
   // Returns whether it ran.  A function of its own, without register results, so
@@ -378,7 +368,7 @@ struct NttTile {
         e[j] = gather<P, SRC>(sr, smem, layout, base, sb, j);
         if constexpr (P > 0) e[j] = lazy_value(e[j], k);
       }
-      exact_group<r>(e, [&](int t, int u) {
+      exact_stages<r, true>(e, [&](int t, int u) {
         const uint4 v = (tw_at(sr.tw, gt << t))[u];  // generic: the table may be in shared memory
         return U128{{v.x, v.y, v.z, v.w}};
       }, k);
@@ -429,11 +419,12 @@ struct NttTile {
   // cases (all-zero, sparse and short-coefficient polynomials).  A warp that
   // finds such a pair takes the exact pass at once instead of running the stages
   // twice; after the first pass it looks only if a thread it exchanges with ran
-  // an exact pass (`suspect`).  16,384 x 2^10, us: spread residues 282, their
-  // upper half zero 283, ternary 342, 31 of 32 values zero 408, all zero 157 (334,
-  // 343, 435 and 454 for the last four kinds when any zero multiplicand called for the
-  // exact pass and zeros were multiplied; 431 for any values with the exact
-  // butterflies throughout).
+  // an exact pass (`suspect`).  16,384 x 2^10, us: spread residues 281, their
+  // upper half zero 281, ternary 338, 31 of 32 values zero 403, all zero 373 (334,
+  // 343, 435 and 454 for the last four kinds when any zero multiplicand called for
+  // the exact pass and zeros were multiplied; 431 for any values with the exact
+  // butterflies throughout).  Testing whole groups for zeros takes all-zero inputs
+  // to 157, and spread ones to 283.
   template <int P, int SRC>
   __device__ __forceinline__ static void pass_lazy(U128 (&v)[R], const SubRef& sr, int sub, int lane,
                                                    uint4* smem, const ModParams& mp, int layout,
@@ -512,7 +503,11 @@ struct NttTile {
         U128 e[G];
 #pragma unroll
         for (int j = 0; j < G; ++j) e[j] = P > 0 ? lazy_value(v[i * G + j], k) : v[i * G + j];
-        exact_group<bits(P)>(e, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, 0u, i, t, u); }, k);
+        uint32_t any = 0;
+#pragma unroll
+        for (int j = 0; j < G; ++j) any |= e[j].w[0] | e[j].w[1] | e[j].w[2] | e[j].w[3];
+        if (any != 0u)  // a group of zeros stays one
+          exact_stages<bits(P)>(e, [&](int t, int u) { return table_entry<P, SRC>(tw, sr, 0u, i, t, u); }, k);
 #pragma unroll
         for (int j = 0; j < G; ++j)
           scatter<P>(sr, smem, layout, mb, k, base, sb, j, P == NPASS - 1 ? e[j] : add_8q(e[j], k));

@@ -706,9 +706,10 @@ __device__ __forceinline__ U128 fold_top(const U128& a, uint32_t k) {
 }
 // the reference's value of a u that a pass left
 __device__ __forceinline__ U128 lazy_value(const U128& u, uint32_t k) {
-  if (u.w[1] == 0xFFFFFFFFu) {  // left by a rerun: u - 8q = u + 2^127 + 8k (mod 2^128)
-    const U128 c{{k << 3, 0u, 0u, 0x80000000u}};
-    return add_nc(u, c);
+  const U128 zero_based = add_8q(u, k);             // u + 8q = (u - 8q) + 16q, 16q = 2^128 - 16k
+  if (u.w[1] == 0xFFFFFFFFu) {                      // left by a rerun: u - 8q
+    const U128 c{{k << 4, 0u, 0u, 0u}};
+    return add_nc(zero_based, c);
   }
   return reduce_once(fold_top(u, k), k);
 }
@@ -744,8 +745,9 @@ __device__ __forceinline__ void lazy_stages(U128 (&v)[R], int e0, const Tw& tw, 
   }
 }
 
-// The same stages with the reference's butterflies, on exact values.
-template <int r, int R, class Tw>
+// The same stages with the reference's butterflies, on exact values.  ZEROS: the
+// first stage multiplies no zeros.
+template <int r, bool ZEROS = false, int R, class Tw>
 __device__ __forceinline__ void exact_stages(U128 (&v)[R], const Tw& tw, uint32_t k) {
 #pragma unroll
   for (int t = 0; t < r; ++t) {
@@ -756,7 +758,8 @@ __device__ __forceinline__ void exact_stages(U128 (&v)[R], const Tw& tw, uint32_
 #pragma unroll
       for (int i = 0; i < half; ++i) {
         U128 &x = v[(u << (r - t)) | i], &y = v[((u << (r - t)) | i) + half];
-        const U128 p = reduce_once(mul_lazy(w, y, k), k);
+        U128 p = y;
+        if (!ZEROS || t > 0 || (y.w[0] | y.w[1] | y.w[2] | y.w[3])) p = reduce_once(mul_lazy(w, y, k), k);
         y = submod_pm(x, p, 0u - k);
         x = addmod_pm(x, p, 0u - k);
       }
