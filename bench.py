@@ -422,8 +422,9 @@ def run_ours(args, dist: Dist):
 
 
 def butterfly_ceiling(ctx, bfly: int, ms: float) -> dict:
-    """The kernel's butterfly rate against the same butterfly on registers
-    (no memory, no index arithmetic) at the same occupancy."""
+    """The kernel's butterfly rate against its forward stages alone on registers
+    (no memory, no index arithmetic, no reductions between passes; 4 CTAs of 256
+    threads per SM)."""
     peak = ctx.butterfly_peak()
     achieved = bfly / (ms * 1e-3)
     return {"achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "G butterflies/s",

@@ -13,7 +13,8 @@ namespace bntt {
 // tiles) the CTAs drifted apart and the SM ran its last third with fewer of
 // them (39 % of the warp slots active on average, of the 50 % the registers
 // allow).  65,536 x 1024: 1331 -> 1219 us; a grid of 2, 4 and 8 times the
-// resident CTAs lies between (1282, 1247, 1229).
+// resident CTAs lies between (1282, 1247, 1229).  Without the walk's loop and its
+// registers 1183 us.
 // MINB > 0 asks for at least MINB resident CTAs per SM (fewer registers per
 // thread, more warps to hide the latency of the carry chains).
 template <int M, int LOGR, int TPC, int MAP, class Arith, int MINB, int SRC = SRC_GLOBAL>

@@ -62,12 +62,13 @@ extern "C" int bntt_probe_imad_peak(bntt_ctx* c, double* ops_per_second) {
   return BNTT_OK;
 }
 
-// Butterfly ceiling: the kernels' own butterfly (lazy_stages: pseudo-Mersenne
+// Butterfly ceiling: the forward stages alone (lazy_stages: pseudo-Mersenne
 // multiply, sums on partly reduced values) on register-resident data, in radix-4
-// groups of 4 butterflies (the persistent kernel's 4 elements per thread), at
-// the persistent kernel's occupancy (4 CTAs of 256 threads per SM).  No
-// memory traffic, no index arithmetic: the rate any NTT kernel of this
-// arithmetic can approach.
+// groups of 4 butterflies, 4 CTAs of 256 threads per SM (the occupancy of the
+// persistent kernel's short lists; its long lists' kernel has 7 of 128).  No memory
+// traffic, no index arithmetic, and none of what a pass adds around its stages: the
+// base of 8q, the fold and the check of its results, the look for zeros.  No kernel
+// of this arithmetic can be faster, and none reaches it.
 namespace bntt {
 
 constexpr int kProbeCtasPerSm = 4;
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(256, kProbeCtasPerSm) k_butterfly_probe(uint4*
     if (e < 4) v[e] = t;
     else w[e - 4] = t;
   }
-  bool rerun = false;  // as the kernels: noted, and acted on outside the stages
+  bool rerun = false;  // noted, as in the kernels
   for (uint32_t it = 0; it < iters; ++it)
     lazy_stages<2>(v, 0, [&](int t, int u) { return w[t + u]; }, mp.k, rerun);
   uint32_t s = rerun ? 1u : 0u;

@@ -432,10 +432,10 @@ int bntt_autotune_reset(void);
  * roofline the NTT kernels are reported against.  No reference counterpart
  * (the reference times CPU code only, src/ntt_scalar.c:670-683). */
 int bntt_probe_imad_peak(bntt_ctx *ctx, double *ops_per_second);
-/* Butterflies per second of the kernels' own butterfly (fast multiply,
- * reference add/sub) on register-resident data at the persistent kernel's
- * occupancy: the compute ceiling of the NTT kernels, with no memory traffic
- * or index arithmetic. */
+/* Butterflies per second of the forward stages alone (fast multiply, sums on
+ * partly reduced values) on register-resident data, 4 CTAs of 256 threads per
+ * SM: a ceiling of the NTT kernels, with no memory traffic, index arithmetic or
+ * reductions between passes. */
 int bntt_probe_butterfly_peak(bntt_ctx *ctx, double *butterflies_per_second);
 
 #ifdef __cplusplus
