@@ -6,6 +6,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <tuple>
 #include <mutex>
 
 #include "batch_host.h"
@@ -48,11 +49,11 @@ static const void* batch_kernel(const bntt_batch* b, bool inverse, int threads) 
 // that share the kernel, such as the serving loop's.
 static int batch_kernel_bps(const void* fn, int threads, int* bps) {
   static std::mutex mu;
-  static std::map<std::pair<const void*, int>, int> cache;
+  static std::map<std::tuple<const void*, int, int>, int> cache;  // kernel, threads, device
   int dev = 0;
   BNTT_CK(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> g(mu);
-  auto it = cache.find({fn, dev});
+  auto it = cache.find({fn, threads, dev});
   if (it != cache.end()) {
     *bps = it->second;
     return BNTT_OK;
@@ -63,7 +64,7 @@ static int batch_kernel_bps(const void* fn, int threads, int* bps) {
   int b = 0;
   BNTT_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, smem));
   if (b < 1) return set_error(BNTT_ECUDA, "batch kernel does not fit on an SM (smem %zu)", smem);
-  cache[{fn, dev}] = b;
+  cache[{fn, threads, dev}] = b;
   *bps = b;
   return BNTT_OK;
 }
@@ -88,9 +89,9 @@ int batch_launch(const bntt_batch* b, const std::vector<WorkItem>& items, bool i
 
 int batch_launch_prepare(const bntt_batch* b) {
   int bps = 0;
-  for (int threads : {kBatchThreads, kShortThreads})
-    if (int rc = batch_kernel_bps(batch_kernel(b, false, threads), threads, &bps)) return rc;
-  return BNTT_OK;
+  if (b->fast)
+    if (int rc = batch_kernel_bps(batch_kernel(b, false, kBatchThreads), kBatchThreads, &bps)) return rc;
+  return batch_kernel_bps(batch_kernel(b, false, kShortThreads), kShortThreads, &bps);
 }
 
 // First shape for (m, map) with the preferred radix (0 = any).
