@@ -1,13 +1,13 @@
 // batch.cu -- host side of the batch engine (schedules, uploads, CUDA graphs)
 // and the bntt_batch_* entry points.  Device code: batch_dev.cuh,
-// instantiated in batch_kfast.cu / batch_kref.cu.
+// instantiated in batch_kfast.cu / batch_kinv.cu / batch_kref.cu.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <functional>
 #include <map>
-#include <tuple>
 #include <mutex>
+#include <tuple>
 
 #include "batch_host.h"
 
@@ -967,6 +967,9 @@ extern "C" int bntt_batch_run_dev_noalloc(bntt_batch* b, const bntt_job* jobs, s
     }
     base = c->noalloc_base;
   }
+  // both kernels that lists of this engine take are loaded by its first call, so
+  // that a later one need not load a module into memory that may be taken
+  if (int rc = batch_launch_prepare(b)) return rc;
   Schedule sc;  // host-side vectors only
   if (int rc = build_schedule(b, sc, jobs, count)) return rc;
   const size_t cb = (kCtlHeader + sc.nslots * kMaxPasses) * 4, pb = sc.pass_tiles.size() * 4,
